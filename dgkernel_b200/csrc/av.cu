@@ -11,8 +11,8 @@
 // rhs += eps_e sum_d D_d q_d + LIFT (Fscale 1/2 sum_d n_d (epsP qP_d - epsM qM_d)), added to the
 // Lax-Friedrichs right-hand side of the plain stage; the LSERK4 update follows in the same kernel.
 //
-// Two kernels per stage: av_prep (sensor, eps per node, q) and av_rhs (LF + viscous RHS + update).  Both
-// stage TE elements per block with one thread per node; the FP64 reference matrices sit in shared memory.
+// Three kernels per stage: av_sensor (eps per node), av_flux<GRAD> (q) and av_flux<RHS> (LF + viscous RHS + update).
+// All products run on the FP64 tensor path (mma.sync m8n8k4) in groups of 8 elements.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -21,6 +21,7 @@
 #include "dg_kernels.cuh"
 #include "kernels.hpp"
 #include "runner.hpp"
+#include "tma.cuh"
 
 namespace dgk {
 
@@ -33,10 +34,16 @@ __host__ __device__ constexpr int mlp_params(int nin) { return kHid * nin + kHid
 template <int N>
 struct AvCfg {
   using O = Order<N>;
-  static constexpr int NP = O::NP, NFP = O::NFP, NF = O::NF;
-  static constexpr int TE = (N <= 2) ? 16 : 8;
-  static constexpr int THREADS = ((TE * NP + 31) / 32) * 32;
+  static constexpr int NP = O::NP, NFP = O::NFP, NF = O::NF, NFS = O::NFS;
+  static constexpr int TE = N == 1 ? 32 : N == 2 ? 16 : 8;  // elements per tile: about 100 KB of ring for two CTAs per SM
+  static constexpr int MT = (NP + 7) / 8, KT = (NP + 3) / 4, KL = NF / 4, NT = TE / 8;
 };
+
+__device__ __forceinline__ void av_dmma(double &c0, double &c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
 
 __device__ __forceinline__ double pp_sigma(double S, double s0, double kappa) {
   if (!(S >= s0 - kappa)) return 0.0;
@@ -44,287 +51,483 @@ __device__ __forceinline__ double pp_sigma(double S, double s0, double kappa) {
   return 0.5 * (1.0 + sin(3.141592653589793 * (S - s0) / (2.0 * kappa)));
 }
 
+// ---- sensor pass: eps per node from the modal coefficients ----
+//
+// A warp takes 8 elements at a time: Vinv u as 8-row m-tiles on the FP64 tensor path, the energies by 4 lanes per
+// element, the network (mode 2) with a hidden unit per lane and the 8 elements as independent sums.  The state of the
+// warp's next group is loaded while the current one is computed.  24 us at order 4 and
+// 82,944 elements with the Persson-Peraire sensor (0.93 TB/s of eps and u; bound by the FP64 chains of a warp).
+constexpr int kSensorWarps = 8;
+
 template <int N>
-__global__ void __launch_bounds__(AvCfg<N>::THREADS) av_prep_kernel(const AvArgs A) {
+struct SensorSmem {
+  static constexpr int NP = Order<N>::NP, NPS = Order<N>::NPS;
+  double vinv[NP * NP];
+  double uh[kSensorWarps][8 * NPS];
+  float x[kSensorWarps][8 * NP], h1[kSensorWarps][8 * kHid], h2[kSensorWarps][8 * kHid];
+  __half w[(mlp_params(NP) + 7) & ~7];
+  int top[NP];
+};
+
+template <int N>
+__global__ void __launch_bounds__(32 * kSensorWarps) av_sensor_kernel(const AvArgs A) {
   using C = AvCfg<N>;
-  constexpr int NP = C::NP, NFP = C::NFP, NF = C::NF, TE = C::TE;
+  using S = SensorSmem<N>;
+  constexpr int NP = C::NP, NPS = S::NPS, MT = C::MT, KT = C::KT, GPT = C::TE / 8;  // groups per tile
+  constexpr int FILL = (8 * NP + 31) / 32;
   extern __shared__ __align__(16) unsigned char sm[];
-  double *sDr = reinterpret_cast<double *>(sm);
-  double *sDs = sDr + NP * NP, *sDt = sDs + NP * NP, *sVi = sDt + NP * NP, *sL = sVi + NP * NP;
-  double *su = sL + NP * NF;          // [TE][NP]
-  double *suh = su + TE * NP;         // [TE][NP] modal coefficients, then features
-  double *sfl = suh + TE * NP;        // [3][TE][NF]
-  double *sfmax = sfl + 3 * TE * NF;  // [TE] feature scale
-  double *ssig = sfmax + TE;          // [TE]
-  float *sh1 = reinterpret_cast<float *>(ssig + TE);  // [TE][32]
-  float *sh2 = sh1 + TE * kHid;                       // [TE][32]
-  __half *sW = reinterpret_cast<__half *>(sh2 + TE * kHid);
-  int *sfm = reinterpret_cast<int *>(sW + ((mlp_params(NP) + 7) & ~7));
-  const int tid = threadIdx.x;
-  for (int x = tid; x < NP * NP; x += blockDim.x) {
-    sDr[x] = A.Dr[x];
-    sDs[x] = A.Ds[x];
-    sDt[x] = A.Dt[x];
-    sVi[x] = A.Vinv[x];
-  }
-  for (int x = tid; x < NP * NF; x += blockDim.x) sL[x] = A.LIFT[x];
-  for (int x = tid; x < NF; x += blockDim.x) sfm[x] = A.fmask[x];
+  S &m = *reinterpret_cast<S *>(sm);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int x = tid; x < NP * NP; x += blockDim.x) m.vinv[x] = A.Vinv[x];
+  for (int x = tid; x < NP; x += blockDim.x) m.top[x] = A.top[x];
   if (A.mode == 2)
-    for (int x = tid; x < mlp_params(NP); x += blockDim.x) sW[x] = __ushort_as_half(A.mlp16[x]);
+    for (int x = tid; x < mlp_params(NP); x += blockDim.x) m.w[x] = __ushort_as_half(A.mlp16[x]);
   __syncthreads();
-  const int e = tid / NP, i = tid - e * NP;
-  for (int t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
-    const AvTile tl = A.tiles[t];
-    const bool act = tid < TE * NP && e < tl.nelem;
-    const int64_t nb = tl.node_base + (int64_t)e * NP, fb = tl.face_base + (int64_t)e * NF;
-    if (act) su[e * NP + i] = A.u[nb + i];
-    __syncthreads();
-    if (act) {
-      for (int m = i; m < NF; m += NP) {
-        const int32_t g = A.gmap[fb + m];
-        double uP;
-        if ((uint64_t)g < (uint64_t)A.n_u_values) {
-          uP = A.u[g];
-        } else {
-          uP = su[e * NP + sfm[m]];
-          atomicExch(A.status, kStatusBadGather);
+  double *uh = m.uh[warp];
+  float *x = m.x[warp], *h1 = m.h1[warp], *h2 = m.h2[warp];
+  const int ngroups = A.ntiles * GPT, gstep = gridDim.x * kSensorWarps;
+  double v[FILL];
+  AvTile tl{};
+  int ne = 0;
+  auto load = [&](int g) {
+    tl = A.tiles[g / GPT];
+    const int e0 = 8 * (g % GPT);
+    ne = max(0, min(8, tl.nelem - e0));
+    tl.node_base += (int64_t)e0 * NP;
+    tl.elem_base += e0;
+    tl.e1_base += e0;
+    tl.feat_base += (int64_t)e0 * NP;
+#pragma unroll
+    for (int q = 0; q < FILL; ++q) v[q] = lane + 32 * q < ne * NP ? A.u[tl.node_base + lane + 32 * q] : 0.0;
+  };
+  const int g0 = blockIdx.x * kSensorWarps + warp;
+  if (g0 < ngroups) load(g0);
+  for (int g = g0; g < ngroups; g += gstep) {
+    const AvTile cur = tl;
+    const int cne = ne;
+#pragma unroll
+    for (int q = 0; q < FILL; ++q) {
+      const int i = lane + 32 * q, e = i / NP;
+      if (i < 8 * NP) uh[e * NPS + i - e * NP] = v[q];
+    }
+    __syncwarp();
+    if (g + gstep < ngroups) load(g + gstep);
+    if (cne == 0) {
+      __syncwarp();
+      continue;  // past the tile's last element (warp-uniform)
+    }
+    {
+      const int ar = lane >> 2, ac = lane & 3;
+      double c[MT][2];
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) c[mt][0] = c[mt][1] = 0.0;
+#pragma unroll
+      for (int kk = 0; kk < KT; ++kk) {
+        const int j = 4 * kk + ac;
+        const double bv = j < NP ? uh[ar * NPS + j] : 0.0;
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          const int r = 8 * mt + ar;
+          av_dmma(c[mt][0], c[mt][1], (r < NP && j < NP) ? m.vinv[r * NP + j] : 0.0, bv);
         }
-        const double fs = A.face[3][fb + m];
-        const double jump = 0.5 * (uP - su[e * NP + sfm[m]]) * fs;
-        for (int d = 0; d < 3; ++d) sfl[(d * TE + e) * NF + m] = A.face[d][fb + m] * jump;
       }
+      __syncwarp();  // every lane's reads of the nodal values are done
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (8 * mt + ar < NP) uh[(2 * ac + h) * NPS + 8 * mt + ar] = c[mt][h];
+      __syncwarp();
     }
-    __syncthreads();
-    if (act) {
-      const double *ue = su + e * NP;
-      double uh = 0.0, ur = 0.0, us = 0.0, ut = 0.0;
-#pragma unroll 5
-      for (int j = 0; j < NP; ++j) {
-        const double v = ue[j];
-        uh = fma(sVi[i * NP + j], v, uh);
-        ur = fma(sDr[i * NP + j], v, ur);
-        us = fma(sDs[i * NP + j], v, us);
-        ut = fma(sDt[i * NP + j], v, ut);
+    const int e = lane >> 2, t = lane & 3;  // 4 lanes per element
+    const bool mine = e < cne;
+    double tot = 0.0, hi = 0.0;
+    for (int j = t; j < NP; j += 4) {
+      const double w = uh[e * NPS + j];
+      tot = fma(w, w, tot);
+      if (m.top[j]) hi = fma(w, w, hi);
+    }
+    tot += __shfl_xor_sync(0xffffffffu, tot, 1);
+    tot += __shfl_xor_sync(0xffffffffu, tot, 2);
+    hi += __shfl_xor_sync(0xffffffffu, hi, 1);
+    hi += __shfl_xor_sync(0xffffffffu, hi, 2);
+    const double S = tot > 0.0 ? log10(hi / tot) : -INFINITY;
+    const double pp = pp_sigma(S, A.s0, A.kappa);
+    double sig = A.mode == 0 ? 0.0 : pp;  // sensor off: no viscosity
+    if (mine && t == 0) {
+      if (A.S_out) A.S_out[cur.e1_base + e] = (float)S;
+      if (A.sig_out) A.sig_out[cur.e1_base + e] = (float)pp;
+    }
+    if (A.mode == 2 || A.feat_out) {  // unit-norm modal coefficients
+      const double inv = tot > 0.0 ? 1.0 / sqrt(tot) : 0.0;
+      for (int j = t; j < NP; j += 4) {
+        const float f = (float)(uh[e * NPS + j] * inv);
+        x[e * NP + j] = f;
+        if (mine && A.feat_out) A.feat_out[cur.feat_base + (int64_t)e * NP + j] = f;
       }
-      suh[e * NP + i] = uh;
-      for (int d = 0; d < 3; ++d) {
-        double q = A.geo[d][nb + i] * ur + A.geo[3 + d][nb + i] * us + A.geo[6 + d][nb + i] * ut;
-        const double *fl = sfl + (d * TE + e) * NF;
-#pragma unroll 6
-        for (int m = 0; m < NF; ++m) q = fma(sL[i * NF + m], fl[m], q);
-        A.q[d][nb + i] = q;
-      }
+      __syncwarp();
     }
-    __syncthreads();
-    // sensor: energy ratio, features, PP activation
-    if (act && i == 0) {
-      double tot = 0.0, hi = 0.0;
-#pragma unroll 5
-      for (int j = 0; j < NP; ++j) {
-        const double v = suh[e * NP + j];
-        tot += v * v;
-        if (A.top[j]) hi += v * v;
-      }
-      const double S = tot > 0.0 ? log10(hi / tot) : -INFINITY;
-      const double pp = pp_sigma(S, A.s0, A.kappa);
-      ssig[e] = A.mode == 0 ? 0.0 : pp;  // sensor off: no viscosity
-      sfmax[e] = tot > 0.0 ? 1.0 / sqrt(tot) : 0.0;  // feature scale: unit-norm modal coefficients
-      if (A.S_out) A.S_out[tl.e1_base + e] = (float)S;
-      if (A.sig_out) A.sig_out[tl.e1_base + e] = (float)pp;
-    }
-    __syncthreads();
-    if (act) {
-      const double f = suh[e * NP + i] * sfmax[e];
-      suh[e * NP + i] = f;
-      // FP32 copy for the network, in the flux buffer (dead once q is written)
-      reinterpret_cast<float *>(sfl)[e * NP + i] = (float)f;
-      if (A.feat_out) A.feat_out[tl.feat_base + (int64_t)e * NP + i] = (float)f;
-    }
-    __syncthreads();
     if (A.mode == 2) {
-      // MLP on the unit-norm modal coefficients: FP16 weights, FP32 sums
-      const __half *W1 = sW, *b1 = W1 + kHid * NP, *W2 = b1 + kHid, *b2 = W2 + kHid * kHid, *w3 = b2 + kHid,
+      // FP16 weights, FP32 sums in two chains per unit (lane) and element
+      const __half *W1 = m.w, *b1 = W1 + kHid * NP, *W2 = b1 + kHid, *b2 = W2 + kHid * kHid, *w3 = b2 + kHid,
                    *b3 = w3 + kHid;
-      if (act)
-        for (int o = i; o < kHid; o += NP) {
-          // FP16 weights, FP32 sums in two chains over the FP32 features
-          const float *x = reinterpret_cast<const float *>(sfl) + e * NP;
-          float s0 = __half2float(b1[o]), s1 = 0.f;
+      float s0[8], s1[8];
 #pragma unroll
-          for (int j = 0; j + 1 < NP; j += 2) {
-            s0 = fmaf(__half2float(W1[o * NP + j]), x[j], s0);
-            s1 = fmaf(__half2float(W1[o * NP + j + 1]), x[j + 1], s1);
-          }
-          if (NP & 1) s0 = fmaf(__half2float(W1[o * NP + NP - 1]), x[NP - 1], s0);
-          sh1[e * kHid + o] = tanhf(s0 + s1);
-        }
-      __syncthreads();
-      if (act)
-        for (int o = i; o < kHid; o += NP) {
-          float s0 = __half2float(b2[o]), s1 = 0.f;
-#pragma unroll
-          for (int j = 0; j < kHid; j += 2) {
-            s0 = fmaf(__half2float(W2[o * kHid + j]), sh1[e * kHid + j], s0);
-            s1 = fmaf(__half2float(W2[o * kHid + j + 1]), sh1[e * kHid + j + 1], s1);
-          }
-          sh2[e * kHid + o] = tanhf(s0 + s1);
-        }
-      __syncthreads();
-      if (act && i == 0) {
-        float z = __half2float(b3[0]);
-        for (int j = 0; j < kHid; ++j) z = fmaf(__half2float(w3[j]), sh2[e * kHid + j], z);
-        const float sg = 1.f / (1.f + expf(-z));
-        if (!(sg > A.conf_lo && sg < A.conf_hi)) {
-          ssig[e] = sg;
-        } else if (A.fallback_count) {
-          atomicAdd(A.fallback_count, 1u);
-        }
-        if (A.mlp_out) A.mlp_out[tl.e1_base + e] = sg;
+      for (int k = 0; k < 8; ++k) {
+        s0[k] = __half2float(b1[lane]);
+        s1[k] = 0.f;
       }
-      __syncthreads();
+#pragma unroll 1
+      for (int j = 0; j + 1 < NP; j += 2) {
+        const float wa = __half2float(W1[lane * NP + j]), wb = __half2float(W1[lane * NP + j + 1]);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          s0[k] = fmaf(wa, x[k * NP + j], s0[k]);
+          s1[k] = fmaf(wb, x[k * NP + j + 1], s1[k]);
+        }
+      }
+      if (NP & 1) {
+        const float wa = __half2float(W1[lane * NP + NP - 1]);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s0[k] = fmaf(wa, x[k * NP + NP - 1], s0[k]);
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) h1[k * kHid + lane] = tanhf(s0[k] + s1[k]);
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        s0[k] = __half2float(b2[lane]);
+        s1[k] = 0.f;
+      }
+#pragma unroll 2
+      for (int j = 0; j < kHid; j += 2) {
+        const float wa = __half2float(W2[lane * kHid + j]), wb = __half2float(W2[lane * kHid + j + 1]);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          s0[k] = fmaf(wa, h1[k * kHid + j], s0[k]);
+          s1[k] = fmaf(wb, h1[k * kHid + j + 1], s1[k]);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) h2[k * kHid + lane] = tanhf(s0[k] + s1[k]);
+      __syncwarp();
+      float z = __half2float(b3[0]);
+      for (int j = 0; j < kHid; ++j) z = fmaf(__half2float(w3[j]), h2[e * kHid + j], z);
+      const float sg = 1.f / (1.f + expf(-z));
+      if (!(sg > A.conf_lo && sg < A.conf_hi)) {
+        sig = sg;
+      } else if (A.fallback_count && mine && t == 0) {
+        atomicAdd(A.fallback_count, 1u);
+      }
+      if (A.mlp_out && mine && t == 0) A.mlp_out[cur.e1_base + e] = sg;
     }
-    if (act) A.eps[nb + i] = A.eps0 * ssig[e] * A.h_over_n[tl.elem_base + e];
-    __syncthreads();
+    if (A.eps) {
+      const double eps = mine ? A.eps0 * sig * A.h_over_n[cur.elem_base + e] : 0.0;
+#pragma unroll
+      for (int q = 0; q < FILL; ++q) {
+        const int i = lane + 32 * q;
+        const double w = __shfl_sync(0xffffffffu, eps, 4 * min(i / NP, 7));
+        if (i < cne * NP) A.eps[cur.node_base + i] = w;
+      }
+    }
+    __syncwarp();  // the warp's buffers are free for its next group
   }
 }
 
-template <int N>
-__global__ void __launch_bounds__(AvCfg<N>::THREADS) av_rhs_kernel(const AvArgs A) {
+// ---- BR1 gradient (RHS = false) and right-hand side with the LSERK4 update (RHS = true) ----
+//
+// Persistent CTAs, one consumer warp per (8-row m-tile, 8-element n-tile) with its A fragments of Dr, Ds, Dt and LIFT
+// in registers.  A tile's node and face arrays stream through a two-slot ring of 1-D bulk copies; its neighbour values
+// are gathered straight into the registers of the threads that form the face terms, one tile ahead (their gather
+// indices two tiles ahead), so a tile waits for one memory round trip at most.  A bulk copy starts on 16 bytes: a
+// tile may start on an odd value (odd Np and an odd element count before it), and is then copied from the value before.
+// Two barriers per tile: the face terms are complete; the slot is free.
+// Order 4, 82,944 elements: gradient 129 us (505 MB, 3.9 TB/s), right-hand side 126 us (598 MB, 4.7 TB/s; eps = 0), a
+// stage 270 us with the sensor.  With one thread per node, the matrices in shared memory (a load per FMA) and the
+// tile's loads, products and stores one after the other, the sensor and gradient took 719 us and the right-hand side 366.
+// Bound by HBM and by the latency within a tile: two CTAs (98 KB of ring each) share an SM at order 4.
+template <int N, bool RHS>
+struct FluxCfg : AvCfg<N> {
   using C = AvCfg<N>;
-  constexpr int NP = C::NP, NFP = C::NFP, NF = C::NF, TE = C::TE;
-  extern __shared__ __align__(16) unsigned char sm[];
-  double *sDr = reinterpret_cast<double *>(sm);
-  double *sDs = sDr + NP * NP, *sDt = sDs + NP * NP, *sL = sDt + NP * NP;
-  double *su = sL + NP * NF;    // [TE][NP]
-  double *sq = su + TE * NP;    // [3][TE][NP]
-  double *sfl = sq + 3 * TE * NP;  // [TE][NF]
-  int *sfm = reinterpret_cast<int *>(sfl + TE * NF);
-  const int tid = threadIdx.x;
-  for (int x = tid; x < NP * NP; x += blockDim.x) {
-    sDr[x] = A.Dr[x];
-    sDs[x] = A.Ds[x];
-    sDt[x] = A.Dt[x];
+  static constexpr int THREADS = 32 * C::MT * C::NT;
+  static constexpr int NA = RHS ? 14 : 10;  // node arrays: u, 9 metrics; and q (3), resu
+  static constexpr int F = RHS ? 1 : 3;     // face-term fields
+  static constexpr int G = RHS ? 5 : 1;     // gathered values per face point: u; and eps, q (3)
+  static constexpr uint32_t NODE_B = C::TE * C::NP * 8 + 16, FACE_B = C::TE * C::NF * 8 + 16;
+  static constexpr uint32_t STAGE_B = NA * NODE_B + 4 * FACE_B;
+  static constexpr size_t SMEM = 2 * (size_t)STAGE_B + F * C::TE * C::NFS * 8 + C::NF * 4 + 16;
+  static constexpr int PER = (int)((227 * 1024) / (SMEM + 1024));  // CTAs that share an SM
+  static constexpr int MINB = PER < 1 ? 1 : PER > 3 ? 3 : PER;
+  static constexpr int NJ = (C::TE * C::NF + THREADS - 1) / THREADS;  // face points per thread
+  static_assert(NODE_B % 16 == 0 && FACE_B % 16 == 0, "slots stay 16-byte aligned");
+};
+
+template <int N, bool RHS>
+__device__ __forceinline__ void flux_issue(const AvArgs &A, const AvTile &tl, char *stage, uint64_t *bar) {
+  using C = FluxCfg<N, RHS>;
+  const int64_t nb = tl.node_base & ~(int64_t)1, fb = tl.face_base & ~(int64_t)1;
+  const uint32_t nbytes = round16((uint32_t)((tl.nelem * C::NP + (int)(tl.node_base - nb)) * 8));
+  const uint32_t fbytes = round16((uint32_t)((tl.nelem * C::NF + (int)(tl.face_base - fb)) * 8));
+  mbar_expect_tx(bar, C::NA * nbytes + 4 * fbytes);
+  bulk_g2s(stage, A.u + nb, nbytes, bar);
+#pragma unroll
+  for (int m = 0; m < 9; ++m) bulk_g2s(stage + (1 + m) * C::NODE_B, A.geo[m] + nb, nbytes, bar);
+  if (RHS) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) bulk_g2s(stage + (10 + d) * C::NODE_B, A.q[d] + nb, nbytes, bar);
+    bulk_g2s(stage + 13 * C::NODE_B, A.resu + nb, nbytes, bar);
   }
-  for (int x = tid; x < NP * NF; x += blockDim.x) sL[x] = A.LIFT[x];
-  for (int x = tid; x < NF; x += blockDim.x) sfm[x] = A.fmask[x];
+#pragma unroll
+  for (int m = 0; m < 4; ++m) bulk_g2s(stage + C::NA * C::NODE_B + m * C::FACE_B, A.face[m] + fb, fbytes, bar);
+}
+
+template <int N, bool RHS>
+__global__ void __launch_bounds__(FluxCfg<N, RHS>::THREADS, FluxCfg<N, RHS>::MINB) av_flux_kernel(const AvArgs A) {
+  using C = FluxCfg<N, RHS>;
+  constexpr int NP = C::NP, NF = C::NF, NFS = C::NFS, TE = C::TE, MT = C::MT, KT = C::KT, KL = C::KL, NJ = C::NJ;
+  constexpr int THREADS = C::THREADS, NS = (int)(C::NODE_B / 8), FS = (int)(C::FACE_B / 8);  // array strides within a slot
+  extern __shared__ __align__(128) unsigned char sm[];
+  char *ring = reinterpret_cast<char *>(sm);
+  double *sf = reinterpret_cast<double *>(ring + 2 * C::STAGE_B);  // [F][TE][NFS] face terms
+  uint64_t *full = reinterpret_cast<uint64_t *>(sf + C::F * TE * NFS);
+  int *sfm = reinterpret_cast<int *>(full + 2);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, step = gridDim.x;
+  const int ntiles = A.ntiles;
+  if (tid == 0) {
+    mbar_init(&full[0], 1);
+    mbar_init(&full[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int i = tid; i < NF; i += THREADS) sfm[i] = A.fmask[i];
   __syncthreads();
-  const int e = tid / NP, i = tid - e * NP;
+  const int mt = warp % MT, nt = warp / MT, ac = lane & 3, ar = lane >> 2;
+  const int row = 8 * mt + ar;           // output node
+  const int be = 8 * nt + ar;            // element of the B fragment
+  const int ce = 8 * nt + 2 * ac;        // first of the two elements of the C fragment
+  AvTile t0 = A.tiles[blockIdx.x], t1{};
+  if (blockIdx.x + step < ntiles) t1 = A.tiles[blockIdx.x + step];
+  if (tid == 0) {
+    flux_issue<N, RHS>(A, t0, ring, &full[0]);
+    if (blockIdx.x + step < ntiles) flux_issue<N, RHS>(A, t1, ring + C::STAGE_B, &full[1]);
+  }
+  // this thread's face points: gather indices (two tiles ahead), gathered values (one tile ahead)
+  int32_t idx[NJ];
+  double gv[NJ][C::G], eM[NJ], eB = 0.0;
+  uint32_t bad = 0;  // points whose index is out of range: the interior trace stands for the neighbour's
+  auto load_idx = [&](const AvTile &tl) {
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int k = tid + j * THREADS;
+      idx[j] = k < tl.nelem * NF ? __ldcs(A.gmap + tl.face_base + k) : 0;
+    }
+  };
+  auto gather = [&](const AvTile &tl) {
+    bad = 0;
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int k = tid + j * THREADS;
+      const bool in = k < tl.nelem * NF, ok = (uint64_t)(int64_t)idx[j] < (uint64_t)A.n_u_values;
+      if (in && !ok) {
+        bad |= 1u << j;
+        atomicExch(A.status, kStatusBadGather);
+      }
+      gv[j][0] = in && ok ? A.u[idx[j]] : 0.0;
+      if (RHS) {
+        gv[j][1] = in && ok ? A.eps[idx[j]] : 0.0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) gv[j][2 + d] = in && ok ? A.q[d][idx[j]] : 0.0;
+        eM[j] = in ? A.eps[tl.node_base + (k / NF) * NP] : 0.0;  // eps is constant over an element
+      }
+    }
+    if (RHS) eB = be < tl.nelem ? A.eps[tl.node_base + be * NP] : 0.0;
+  };
+  load_idx(t0);
+  double aD[3][KT], aL[KL];
+#pragma unroll
+  for (int kk = 0; kk < KT; ++kk) {
+    const int j = 4 * kk + ac;
+    const bool in = row < NP && j < NP;
+    aD[0][kk] = in ? A.Dr[row * NP + j] : 0.0;
+    aD[1][kk] = in ? A.Ds[row * NP + j] : 0.0;
+    aD[2][kk] = in ? A.Dt[row * NP + j] : 0.0;
+  }
+#pragma unroll
+  for (int kk = 0; kk < KL; ++kk) aL[kk] = row < NP ? A.LIFT[row * NF + 4 * kk + ac] : 0.0;
+  gather(t0);
+  if (blockIdx.x + step < ntiles) load_idx(t1);
   const double a = A.a, b = A.b, dt = A.dt;
-  for (int t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
-    const AvTile tl = A.tiles[t];
-    const bool act = tid < TE * NP && e < tl.nelem;
-    const int64_t nb = tl.node_base + (int64_t)e * NP, fb = tl.face_base + (int64_t)e * NF;
-    if (act) {
-      su[e * NP + i] = A.u[nb + i];
-      for (int d = 0; d < 3; ++d) sq[(d * TE + e) * NP + i] = A.q[d][nb + i];
-    }
-    __syncthreads();
-    if (act) {
-      const double epsM = A.eps[nb];  // constant per element
-      for (int m = i; m < NF; m += NP) {
-        const int32_t g = A.gmap[fb + m];
-        const int jM = sfm[m];
-        const double uM = su[e * NP + jM];
-        double uP, eP, qP[3];
-        if ((uint64_t)g < (uint64_t)A.n_u_values) {
-          uP = A.u[g];
-          eP = A.eps[g];
-          for (int d = 0; d < 3; ++d) qP[d] = A.q[d][g];
-        } else {
-          uP = uM;
-          eP = epsM;
-          for (int d = 0; d < 3; ++d) qP[d] = sq[(d * TE + e) * NP + jM];
-          atomicExch(A.status, kStatusBadGather);
-        }
-        const double nx = A.face[0][fb + m], ny = A.face[1][fb + m], nz = A.face[2][fb + m];
-        const double fs = A.face[3][fb + m];
-        const double ns = nx + ny + nz;
-        const double fM = 0.5 * uM * uM * ns, fP = 0.5 * uP * uP * ns;
-        const double C = fmax(fabs(uM) * fabs(ns), fabs(uP) * fabs(ns));
-        const double du = fM - (0.5 * (fM + fP) + 0.5 * C * (uM - uP));
-        const double nv[3] = {nx, ny, nz};
-        double vis = 0.0;
-        for (int d = 0; d < 3; ++d) vis += nv[d] * (eP * qP[d] - epsM * sq[(d * TE + e) * NP + jM]);
-        sfl[e * NF + m] = fs * du + 0.5 * fs * vis;
-      }
-    }
-    __syncthreads();
-    if (act) {
-      const double *ue = su + e * NP;
-      double ur = 0.0, us = 0.0, ut = 0.0;
-#pragma unroll 5
-      for (int j = 0; j < NP; ++j) {
-        ur = fma(sDr[i * NP + j], ue[j], ur);
-        us = fma(sDs[i * NP + j], ue[j], us);
-        ut = fma(sDt[i * NP + j], ue[j], ut);
-      }
-      const double ux = A.geo[0][nb + i] * ur + A.geo[3][nb + i] * us + A.geo[6][nb + i] * ut;
-      const double uy = A.geo[1][nb + i] * ur + A.geo[4][nb + i] * us + A.geo[7][nb + i] * ut;
-      const double uz = A.geo[2][nb + i] * ur + A.geo[5][nb + i] * us + A.geo[8][nb + i] * ut;
-      double rhs = -ue[i] * (ux + uy + uz);
-      const double eps = A.eps[nb + i];
-      if (eps != 0.0) {
-        double div = 0.0;
-        for (int d = 0; d < 3; ++d) {
-          const double *qd = sq + (d * TE + e) * NP;
-          double qr = 0.0, qs = 0.0, qt = 0.0;
-    #pragma unroll 5
-      for (int j = 0; j < NP; ++j) {
-            qr = fma(sDr[i * NP + j], qd[j], qr);
-            qs = fma(sDs[i * NP + j], qd[j], qs);
-            qt = fma(sDt[i * NP + j], qd[j], qt);
+  int k = 0;
+  for (int t = blockIdx.x; t < ntiles; t += step, ++k) {
+    const int s = k & 1;
+    const bool has1 = t + step < ntiles, has2 = t + 2 * step < ntiles;
+    AvTile t2{};
+    if (has2) t2 = A.tiles[t + 2 * step];
+    const bool ready = mbar_wait_bounded(&full[s], (uint32_t)(k >> 1) & 1u, kSpinLimit);
+    const int ne = t0.nelem, nfc = ne * NF;
+    const char *stage = ring + s * C::STAGE_B;
+    const double *su = reinterpret_cast<const double *>(stage) + (t0.node_base & 1);
+    const double *sg = su + NS, *sq = su + 10 * NS, *sr = su + 13 * NS;
+    const double *sfc = reinterpret_cast<const double *>(stage + C::NA * C::NODE_B) + (t0.face_base & 1);
+    // face terms of this thread's points
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int x = tid + j * THREADS;
+      if (x < nfc) {
+        const int e = x / NF, m = x - e * NF, o = e * NP + sfm[m];
+        const bool rejected = (bad >> j) & 1u;
+        const double uM = su[o], uP = rejected ? uM : gv[j][0];
+        const double nx = sfc[x], ny = sfc[FS + x], nz = sfc[2 * FS + x], fs = sfc[3 * FS + x];
+        if (RHS) {
+          const double ns = nx + ny + nz;
+          const double fM = 0.5 * uM * uM * ns, fP = 0.5 * uP * uP * ns;
+          const double lam = fmax(fabs(uM) * fabs(ns), fabs(uP) * fabs(ns));
+          const double du = fM - (0.5 * (fM + fP) + 0.5 * lam * (uM - uP));
+          const double eP = rejected ? eM[j] : gv[j][C::G > 1 ? 1 : 0];
+          const double nv[3] = {nx, ny, nz};
+          double vis = 0.0;
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            const double qM = sq[d * NS + o], qP = rejected ? qM : gv[j][C::G > 1 ? 2 + d : 0];
+            vis += nv[d] * (eP * qP - eM[j] * qM);
           }
-          div += A.geo[d][nb + i] * qr + A.geo[3 + d][nb + i] * qs + A.geo[6 + d][nb + i] * qt;
+          sf[e * NFS + m] = fs * du + 0.5 * fs * vis;
+        } else {
+          const double jump = 0.5 * (uP - uM) * fs;
+          sf[e * NFS + m] = nx * jump;
+          sf[TE * NFS + e * NFS + m] = ny * jump;
+          sf[2 * TE * NFS + e * NFS + m] = nz * jump;
         }
-        rhs += eps * div;
       }
-      const double *fl = sfl + e * NF;
-      double lift = 0.0;
-#pragma unroll 6
-      for (int m = 0; m < NF; ++m) lift = fma(sL[i * NF + m], fl[m], lift);
-      rhs += lift;
-      const double r = a * A.resu[nb + i] + dt * rhs;
-      A.resu[nb + i] = r;
-      A.u_out[nb + i] = ue[i] + b * r;
     }
-    __syncthreads();
+    const double eCur = eB;
+    // in flight from here on: the next tile's neighbour values and the indices after them
+    if (has1) gather(t1);
+    if (has2) load_idx(t2);
+    // derivatives at (row, ce), (row, ce + 1)
+    double out[3][2];  // GRAD: q; RHS: out[0] = the volume terms
+    {
+      double c[3][2] = {};
+#pragma unroll
+      for (int kk = 0; kk < KT; ++kk) {
+        const int j = 4 * kk + ac;
+        const double bv = (j < NP && be < ne) ? su[be * NP + j] : 0.0;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) av_dmma(c[m][0], c[m][1], aD[m][kk], bv);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int o = (ce + h) * NP + row;
+        const bool in = row < NP && ce + h < ne;
+        double g[3] = {};
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+          if (in) g[d] = sg[d * NS + o] * c[0][h] + sg[(3 + d) * NS + o] * c[1][h] + sg[(6 + d) * NS + o] * c[2][h];
+        if (RHS) {
+          out[0][h] = in ? -su[o] * (g[0] + g[1] + g[2]) : 0.0;
+        } else {
+#pragma unroll
+          for (int d = 0; d < 3; ++d) out[d][h] = g[d];
+        }
+      }
+    }
+    if (RHS) {
+      // eps div q where an element of the n-tile has viscosity
+      if (__any_sync(0xffffffffu, eCur != 0.0)) {
+        double div[2] = {};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          double c[3][2] = {};
+#pragma unroll
+          for (int kk = 0; kk < KT; ++kk) {
+            const int j = 4 * kk + ac;
+            const double bv = (j < NP && be < ne) ? sq[d * NS + be * NP + j] : 0.0;
+#pragma unroll
+            for (int m = 0; m < 3; ++m) av_dmma(c[m][0], c[m][1], aD[m][kk], bv);
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int o = (ce + h) * NP + row;
+            if (row < NP && ce + h < ne)
+              div[h] += sg[d * NS + o] * c[0][h] + sg[(3 + d) * NS + o] * c[1][h] + sg[(6 + d) * NS + o] * c[2][h];
+          }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const double e = __shfl_sync(0xffffffffu, eCur, 4 * (2 * ac + h));  // element ce + h
+          if (e != 0.0) out[0][h] += e * div[h];
+        }
+      }
+    }
+    if (!__syncthreads_and(ready)) {  // face terms complete; a wait that gave up ends every thread here
+      if (tid == 0) atomicExch(A.status, kStatusTimeoutCode);
+      mbar_wait_bounded(&full[s], (uint32_t)(k >> 1) & 1u, kSpinLimit);  // copies in flight land before the CTA goes
+      if (has1) mbar_wait_bounded(&full[s ^ 1], (uint32_t)((k + 1) >> 1) & 1u, kSpinLimit);
+      return;
+    }
+    // LIFT times the face terms
+    {
+      double c[3][2] = {};  // GRAD: the three directions; RHS: three chains of one sum
+#pragma unroll
+      for (int kk = 0; kk < KL; ++kk) {
+        if (RHS) {
+          av_dmma(c[kk % 3][0], c[kk % 3][1], aL[kk], be < ne ? sf[be * NFS + 4 * kk + ac] : 0.0);
+        } else {
+#pragma unroll
+          for (int d = 0; d < 3; ++d)
+            av_dmma(c[d][0], c[d][1], aL[kk], be < ne ? sf[(d * TE + be) * NFS + 4 * kk + ac] : 0.0);
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int o = (ce + h) * NP + row;
+        if (row < NP && ce + h < ne) {
+          if (RHS) {
+            const double rhs = out[0][h] + (c[0][h] + c[1][h] + c[2][h]);
+            const double r = a * sr[o] + dt * rhs;
+            __stcs(A.resu + t0.node_base + o, r);
+            __stcs(A.u_out + t0.node_base + o, su[o] + b * r);
+          } else {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) A.q[d][t0.node_base + o] = out[d][h] + c[d][h];
+          }
+        }
+      }
+    }
+    __syncthreads();  // every read of slot s and of the face terms is done
+    if (tid == 0 && has2) {
+      fence_async_smem();
+      flux_issue<N, RHS>(A, t2, ring + s * C::STAGE_B, &full[s]);
+    }
+    t0 = t1;
+    t1 = t2;
   }
 }
 
-template <int N>
-size_t prep_smem(int np_, int nf_) {
-  using C = AvCfg<N>;
-  (void)np_;
-  (void)nf_;
-  constexpr int NP = C::NP, NF = C::NF, TE = C::TE;
-  size_t b = sizeof(double) * (4 * NP * NP + NP * NF + 2 * TE * NP + 3 * TE * NF + 2 * TE);
-  b += sizeof(float) * 2 * TE * kHid;
-  b += sizeof(__half) * ((mlp_params(NP) + 7) & ~7);
-  b += sizeof(int) * NF;
-  return b;
-}
-
-template <int N>
-size_t rhs_smem() {
-  using C = AvCfg<N>;
-  constexpr int NP = C::NP, NF = C::NF, TE = C::TE;
-  return sizeof(double) * (3 * NP * NP + NP * NF + 4 * TE * NP + TE * NF) + sizeof(int) * NF;
+template <typename K>
+int av_attr(K kernel, int threads, size_t smem) {
+  cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "av smem");
+  int per = 0;
+  cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem), "av occupancy");
+  return std::max(1, per);
 }
 
 template <int N>
 void launch_av_n(const AvArgs &A, int num_sms, cudaStream_t st) {
-  using C = AvCfg<N>;
-  const size_t s1 = prep_smem<N>(C::NP, C::NF), s2 = rhs_smem<N>();
-  cuda_check(cudaFuncSetAttribute(av_prep_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1),
-             "av_prep smem");
-  cuda_check(cudaFuncSetAttribute(av_rhs_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2),
-             "av_rhs smem");
-  const int grid = std::max(1, std::min(A.ntiles, num_sms * 8));
-  av_prep_kernel<N><<<grid, C::THREADS, s1, st>>>(A);
-  cuda_check(cudaGetLastError(), "av_prep_kernel launch");
+  const size_t s0 = sizeof(SensorSmem<N>);
+  const int ps = av_attr(av_sensor_kernel<N>, 32 * kSensorWarps, s0);
+  const int groups = A.ntiles * (AvCfg<N>::TE / 8);
+  const int gs = std::max(1, std::min((groups + kSensorWarps - 1) / kSensorWarps, ps * num_sms));
+  av_sensor_kernel<N><<<gs, 32 * kSensorWarps, s0, st>>>(A);
+  cuda_check(cudaGetLastError(), "av_sensor_kernel launch");
   if (A.prep_only) return;
-  av_rhs_kernel<N><<<grid, C::THREADS, s2, st>>>(A);
-  cuda_check(cudaGetLastError(), "av_rhs_kernel launch");
+  using Cg = FluxCfg<N, false>;
+  using Cr = FluxCfg<N, true>;
+  const int pg = av_attr(av_flux_kernel<N, false>, Cg::THREADS, Cg::SMEM);
+  av_flux_kernel<N, false><<<std::min(A.ntiles, pg * num_sms), Cg::THREADS, Cg::SMEM, st>>>(A);
+  cuda_check(cudaGetLastError(), "av_flux_kernel (gradient) launch");
+  const int pr = av_attr(av_flux_kernel<N, true>, Cr::THREADS, Cr::SMEM);
+  av_flux_kernel<N, true><<<std::min(A.ntiles, pr * num_sms), Cr::THREADS, Cr::SMEM, st>>>(A);
+  cuda_check(cudaGetLastError(), "av_flux_kernel (right-hand side) launch");
 }
 
 // ---------------- MLP: forward, loss gradient (mean squared error), Adam, FP32 -> FP16 ----------------
@@ -608,7 +811,7 @@ __global__ void mlp_forward16_kernel(const __half *p, const float *X, int64_t n,
 
 int mlp_param_count(int nin) { return mlp_params(nin); }
 
-int av_tile_elems(int N) { return N <= 2 ? AvCfg<2>::TE : AvCfg<3>::TE; }
+int av_tile_elems(int N) { return N == 1 ? AvCfg<1>::TE : N == 2 ? AvCfg<2>::TE : AvCfg<3>::TE; }
 
 void launch_av(int N, const AvArgs &A, int num_sms, cudaStream_t st) {
   switch (N) {

@@ -932,7 +932,7 @@ struct AvOp : Op {
   float lo = 0.1f, hi = 0.9f;
   Binding *u, *unext = nullptr, *resu = nullptr, *geo[9], *face[4], *gmap, *eps = nullptr, *q[3] = {};
   Binding *mlp = nullptr, *feat = nullptr, *sig = nullptr, *mlps = nullptr;
-  DevBuf tiles, dr, ds, dt, vinv, lift, fmask, top, hon, mlp16, qs[3], epsb;
+  DevBuf tiles, dr, ds, dt, vinv, lift, fmask, top, hon, mlp16;
   AvOp(Runner &r, Roles &R, int feats) : features(feats) {
     static const char *gn[9] = {"Rx", "Ry", "Rz", "Sx", "Sy", "Sz", "Tx", "Ty", "Tz"};
     static const char *fn[4] = {"nx", "ny", "nz", "Fscale"};
@@ -980,10 +980,6 @@ struct AvOp : Op {
       require(feat->dev_dtype == DGK_FLOAT32 && feat->values_per_elem == np, R.kname + ": feat is float32, Np per element");
       require(sig->dev_dtype == DGK_FLOAT32 && sig->values_per_elem == 1, R.kname + ": sigma is float32, 1 per element");
       if (mlps) same_layout(*sig, *mlps, R.kname);
-      // the gradient and viscosity outputs of the sensor pass go to operator-owned scratch
-      const size_t nb = sizeof(double) * (size_t)u->offsets.back();
-      for (auto &b : qs) b.alloc(nb);
-      epsb.alloc(nb);
     } else {
       unext = R.array("uNext");
       resu = R.array("resu");
@@ -1072,8 +1068,6 @@ struct AvOp : Op {
       A.mlp16 = mlp16.get<unsigned short>();
     }
     if (features) {
-      for (int d = 0; d < 3; ++d) A.q[d] = qs[d].get<double>();
-      A.eps = epsb.get<double>();
       A.feat_out = reinterpret_cast<float *>(feat->dptr);
       A.sig_out = reinterpret_cast<float *>(sig->dptr);
       A.mlp_out = mlps ? reinterpret_cast<float *>(mlps->dptr) : nullptr;
