@@ -28,6 +28,14 @@ int tma_tile_elems(int N);  // 0 when the order has no TMA form
 // FP64 form with TMA streaming and the element-local products on the FP64 tensor path (kernels_tma.cu).
 bool launch_rhs_dmma(int N, const RhsArgs<double> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info);
 int dmma_tile_elems(int N);  // 0 when the order has no such form
+// FP64 form of orders 6 and 7 with the matrices streamed in fragment order (kernels_wide.cu).  wide_pack lays out
+// `nmats` stacked row-major rows x cols matrices (cols a multiple of 4) for it; A.Dmat = wide_pack(Dr, Ds, Dt) and
+// A.LIFT = wide_pack(LIFT).  wide_tile_elems: elements per tile for a problem of nelems elements.
+bool wide_supported(int N);
+int wide_tile_elems(int64_t nelems, int num_sms);
+std::vector<double> wide_pack(const std::vector<double> &mats, int nmats, int rows, int cols);
+void launch_rhs_wide(int N, int tile_elems, const RhsArgs<double> &A, int rhs_only, int num_sms, cudaStream_t st,
+                     LaunchInfo *info);
 
 // Mixed-precision stage (mixed.cu) with 4, 8 or 11 consumer warps per CTA and at most ring_max ring slots
 // (0: as many as shared memory holds); returns false when the order or the warp count has no such form.

@@ -1,0 +1,282 @@
+// Fused strong-form Lax-Friedrichs RHS + LSERK4 stage in FP64 at orders 6 and 7, where the reference matrices (237 and
+// 483 KB) fit neither registers nor shared memory.
+//
+// The products run on the FP64 tensor path (mma.sync m8n8k4) with the matrices streamed from L2: the operator stores
+// them in fragment order, so a warp's A fragment is 256 consecutive bytes, and every fragment is used for NT n-tiles of
+// 8 elements before the next one, which is loaded two k-steps ahead.  At NT = 4 that is 16 bytes of matrix per clock
+// and SM at the full FP64 rate (64 FMAs per clock and SM).  A CTA holds one tile of 8 NT elements: state, volume terms
+// and face terms in shared memory (100 KB at NT = 4), rows stored at strides of 4 or 12 mod 16 values, which keeps the
+// fragment loads free of bank conflicts.  The nine metrics and four face arrays are read once, straight from global
+// memory, 64 consecutive bytes per element, and brought into L2 one tile ahead by bulk prefetches.  Two CTAs share an
+// SM and drift apart, so one's memory phases run under the other's products; each warp owns one or two 8-row m-tiles.
+//
+// Bound by the FP64 rate (60,480 FMAs per element at order 7).
+// @WIDE@
+#include <algorithm>
+#include <cstdint>
+
+#include "dg_kernels.cuh"
+#include "kernels.hpp"
+#include "runner.hpp"
+
+namespace dgk {
+
+namespace {
+
+template <int N, int NT>
+struct WideCfg {
+  using O = Order<N>;
+  static constexpr int NP = O::NP, NF = O::NF;
+  static constexpr int TE = 8 * NT;
+  static constexpr int MT = (NP + 7) / 8, KT = NP / 4, KL = NF / 4;
+  static constexpr int WARPS = (MT + 1) / 2;  // one or two m-tiles per warp
+  static constexpr int THREADS = 32 * WARPS;
+  static constexpr int SU = (NP + 7) / 16 * 16 + (NP % 16 <= 4 ? 4 : 12);  // row strides: 4 or 12 mod 16
+  static constexpr int SF = NF / 16 * 16 + 4;
+  static constexpr size_t SMEM = sizeof(double) * (size_t)TE * (2 * SU + SF) + sizeof(int) * NF;
+  static constexpr int DEPTH = 3;  // A fragments in flight
+  static_assert(NP % 4 == 0 && NF % 16 == 0 && KT % DEPTH == 0, "whole k-steps");
+  static_assert(SU >= NP && (SU % 16 == 4 || SU % 16 == 12) && SF >= NF, "row strides");
+};
+
+__device__ __forceinline__ void wide_dmma(double &c0, double &c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+
+// L2 prefetch of a contiguous range, widened to 16-byte granules (the runner's arrays sit in 256-byte aligned slots)
+__device__ __forceinline__ void wide_prefetch(const void *p, size_t bytes) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p) & ~uintptr_t(15);
+  const uintptr_t e = (reinterpret_cast<uintptr_t>(p) + bytes + 15) & ~uintptr_t(15);
+  if (e > a) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(e - a)) : "memory");
+}
+
+// lanes 0..15 of a warp each prefetch one of the streams that a tile reads
+__device__ __forceinline__ void wide_prefetch_tile(const RhsArgs<double> &A, const Tile &tl, int np, int nf, int lane) {
+  const size_t nn = (size_t)tl.nelem * np * sizeof(double), fn = (size_t)tl.nelem * nf;
+  if (lane < 9) wide_prefetch(A.geo[lane] + tl.node_base, nn);
+  else if (lane < 13) wide_prefetch(A.face[lane - 9] + tl.face_base, fn * sizeof(double));
+  else if (lane == 13) wide_prefetch(A.u_in + tl.node_base, nn);
+  else if (lane == 14 && A.resu) wide_prefetch(A.resu + tl.node_base, nn);
+  else if (lane == 15) wide_prefetch(A.gmap + tl.face_base, fn * sizeof(int32_t));
+}
+
+template <int N, int NT>
+__global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, 2) rhs_stage_wide_kernel(const RhsArgs<double> A, int rhs_only) {
+  using C = WideCfg<N, NT>;
+  constexpr int NP = C::NP, NF = C::NF, MT = C::MT, KT = C::KT, KL = C::KL, SU = C::SU, SF = C::SF, TE = C::TE;
+  constexpr int THREADS = C::THREADS, W = C::WARPS, DEPTH = C::DEPTH;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double *su = reinterpret_cast<double *>(smem_raw);  // [TE][SU] state
+  double *sv = su + TE * SU;                          // [TE][SU] volume terms
+  double *sf = sv + TE * SU;                          // [TE][SF] neighbour traces, then face terms
+  int *sfm = reinterpret_cast<int *>(sf + TE * SF);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ar = lane >> 2, ac = lane & 3;
+  for (int i = tid; i < NF; i += THREADS) sfm[i] = A.fmask[i];
+  if (warp == 0) wide_prefetch_tile(A, A.tiles[blockIdx.x], NP, NF, lane);
+  const double a = A.a, b = A.b, dt = A.dt;
+  __syncthreads();
+  for (int t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
+    const Tile tl = A.tiles[t];
+    const int ne = tl.nelem, nn = ne * NP, nfc = ne * NF;
+    // state, and neighbour traces of this thread's face points (index batch, then gather batch)
+    constexpr int CH = 6;
+    for (int x0 = tid; x0 < nn; x0 += CH * THREADS) {
+      double v[CH];
+#pragma unroll
+      for (int j = 0; j < CH; ++j) v[j] = x0 + j * THREADS < nn ? A.u_in[tl.node_base + x0 + j * THREADS] : 0.0;
+#pragma unroll
+      for (int j = 0; j < CH; ++j) {
+        const int x = x0 + j * THREADS, e = x / NP;
+        if (x < nn) su[e * SU + x - e * NP] = v[j];
+      }
+    }
+    __syncthreads();
+    for (int x0 = tid; x0 < nfc; x0 += CH * THREADS) {
+      int32_t src[CH];
+      double up[CH], fc[CH][4];
+#pragma unroll
+      for (int j = 0; j < CH; ++j) src[j] = x0 + j * THREADS < nfc ? __ldcs(A.gmap + tl.face_base + x0 + j * THREADS) : 0;
+#pragma unroll
+      for (int j = 0; j < CH; ++j)
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          fc[j][m] = x0 + j * THREADS < nfc ? __ldcs(A.face[m] + tl.face_base + x0 + j * THREADS) : 0.0;
+#pragma unroll
+      for (int j = 0; j < CH; ++j) {
+        const bool ok = src[j] >= 0 && (int64_t)src[j] < A.n_u_values;
+        up[j] = ok ? A.u_in[src[j]] : 0.0;
+      }
+#pragma unroll
+      for (int j = 0; j < CH; ++j) {
+        const int x = x0 + j * THREADS;
+        if (x < nfc) {
+          const int e = x / NF, q = x - e * NF;
+          const double uM = su[e * SU + sfm[q]];
+          double uP = up[j];
+          if (!(src[j] >= 0 && (int64_t)src[j] < A.n_u_values)) {  // rejected index: report it, use the interior trace
+            atomicExch(A.status, kStatusBadGather);
+            uP = uM;
+          }
+          const double nsum = fc[j][0] + fc[j][1] + fc[j][2];
+          const double fM = 0.5 * uM * uM * nsum, fP = 0.5 * uP * uP * nsum;
+          const double an = fabs(nsum);
+          const double lam = fmax(fabs(uM) * an, fabs(uP) * an);
+          sf[e * SF + q] = fc[j][3] * (fM - (0.5 * (fM + fP) + 0.5 * lam * (uM - uP)));
+        }
+      }
+    }
+    if (warp == W - 1 && t + (int)gridDim.x < A.ntiles) wide_prefetch_tile(A, A.tiles[t + gridDim.x], NP, NF, lane);
+    // volume terms of this warp's m-tiles
+#pragma unroll 1
+    for (int mt = warp; mt < MT; mt += W) {
+      const double *ap = A.Dmat + (size_t)mt * KT * 96 + lane;
+      double c[3][NT][2];
+#pragma unroll
+      for (int m = 0; m < 3; ++m)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) c[m][n][0] = c[m][n][1] = 0.0;
+      double f[DEPTH][3];
+#pragma unroll
+      for (int d = 0; d < DEPTH - 1; ++d)
+#pragma unroll
+        for (int m = 0; m < 3; ++m) f[d][m] = __ldg(ap + d * 96 + m * 32);
+#pragma unroll 1
+      for (int k0 = 0; k0 < KT; k0 += DEPTH) {
+#pragma unroll
+        for (int d = 0; d < DEPTH; ++d) {
+          const int kk = k0 + d, kn = min(kk + DEPTH - 1, KT - 1);
+#pragma unroll
+          for (int m = 0; m < 3; ++m) f[(d + DEPTH - 1) % DEPTH][m] = __ldg(ap + kn * 96 + m * 32);
+#pragma unroll
+          for (int n = 0; n < NT; ++n) {
+            double bv = su[(8 * n + ar) * SU + 4 * kk + ac];
+            if (A.conservative) bv = 0.5 * bv * bv;
+#pragma unroll
+            for (int m = 0; m < 3; ++m) wide_dmma(c[m][n][0], c[m][n][1], f[d][m], bv);
+          }
+        }
+      }
+      const int row = 8 * mt + ar;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        double g[2][9];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int e = 8 * n + 2 * ac + h;
+#pragma unroll
+          for (int m = 0; m < 9; ++m)
+            g[h][m] = (row < NP && e < ne) ? __ldcs(A.geo[m] + tl.node_base + e * NP + row) : 0.0;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int e = 8 * n + 2 * ac + h;
+          const double ur = c[0][n][h], us = c[1][n][h], ut = c[2][n][h];
+          const double ux = g[h][0] * ur + g[h][3] * us + g[h][6] * ut;
+          const double uy = g[h][1] * ur + g[h][4] * us + g[h][7] * ut;
+          const double uz = g[h][2] * ur + g[h][5] * us + g[h][8] * ut;
+          if (row < NP && e < ne) sv[e * SU + row] = A.conservative ? -(ux + uy + uz) : -su[e * SU + row] * (ux + uy + uz);
+        }
+      }
+    }
+    __syncthreads();  // face terms complete
+    // LIFT times the face terms, then the update; each lane reads back the volume terms it wrote
+#pragma unroll 1
+    for (int mt = warp; mt < MT; mt += W) {
+      const double *ap = A.LIFT + (size_t)mt * KL * 32 + lane;
+      const int row = 8 * mt + ar;
+      double c[NT][2], rs[NT][2];
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int e = 8 * n + 2 * ac + h;
+          c[n][h] = 0.0;
+          rs[n][h] = (!rhs_only && row < NP && e < ne) ? __ldcs(A.resu + tl.node_base + e * NP + row) : 0.0;
+        }
+      double f[4];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) f[d] = __ldg(ap + d * 32);
+#pragma unroll 1
+      for (int k0 = 0; k0 < KL; k0 += 4) {
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
+          const int kk = k0 + d;
+          f[(d + 3) % 4] = __ldg(ap + min(kk + 3, KL - 1) * 32);
+#pragma unroll
+          for (int n = 0; n < NT; ++n) wide_dmma(c[n][0], c[n][1], f[d], sf[(8 * n + ar) * SF + 4 * kk + ac]);
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int e = 8 * n + 2 * ac + h;
+          if (row < NP && e < ne) {
+            const int64_t gi = tl.node_base + e * NP + row;
+            const double rhs = sv[e * SU + row] + c[n][h];
+            if (rhs_only) {
+              __stcs(A.rhs_out + gi, rhs);
+            } else {
+              const double res = a * rs[n][h] + dt * rhs;
+              __stcs(A.resu + gi, res);
+              __stcs(A.u_out + gi, su[e * SU + row] + b * res);
+            }
+          }
+        }
+    }
+    __syncthreads();  // the tile's buffers are free
+  }
+}
+
+template <int N, int NT>
+void wide_launch_n(const RhsArgs<double> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info) {
+  using C = WideCfg<N, NT>;
+  auto k = rhs_stage_wide_kernel<N, NT>;
+  cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM), "smem attr");
+  int per = 0;
+  cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, C::THREADS, C::SMEM), "occupancy");
+  per = std::max(1, per);
+  const int grid = std::min(A.ntiles, per * num_sms);
+  if (info) *info = {grid, C::THREADS, (int)C::SMEM, per};
+  if (grid > 0) k<<<grid, C::THREADS, C::SMEM, st>>>(A, rhs_only);
+}
+
+}  // namespace
+
+bool wide_supported(int N) { return N == 6 || N == 7; }
+
+int wide_tile_elems(int64_t nelems, int num_sms) {
+  for (int te : {32, 16})
+    if ((nelems + te - 1) / te >= 2 * (int64_t)num_sms) return te;
+  return 8;
+}
+
+std::vector<double> wide_pack(const std::vector<double> &mats, int nmats, int rows, int cols) {
+  const int mt = (rows + 7) / 8, kt = cols / 4;
+  std::vector<double> out((size_t)mt * kt * nmats * 32, 0.0);
+  for (int t = 0; t < mt; ++t)
+    for (int k = 0; k < kt; ++k)
+      for (int m = 0; m < nmats; ++m)
+        for (int l = 0; l < 32; ++l) {
+          const int i = 8 * t + (l >> 2), j = 4 * k + (l & 3);
+          if (i < rows) out[(((size_t)t * kt + k) * nmats + m) * 32 + l] = mats[((size_t)m * rows + i) * cols + j];
+        }
+  return out;
+}
+
+void launch_rhs_wide(int N, int tile_elems, const RhsArgs<double> &A, int rhs_only, int num_sms, cudaStream_t st,
+                     LaunchInfo *info) {
+  const int nt = tile_elems / 8;
+  if (N == 6 && nt == 4) wide_launch_n<6, 4>(A, rhs_only, num_sms, st, info);
+  else if (N == 6 && nt == 2) wide_launch_n<6, 2>(A, rhs_only, num_sms, st, info);
+  else if (N == 6 && nt == 1) wide_launch_n<6, 1>(A, rhs_only, num_sms, st, info);
+  else if (N == 7 && nt == 4) wide_launch_n<7, 4>(A, rhs_only, num_sms, st, info);
+  else if (N == 7 && nt == 2) wide_launch_n<7, 2>(A, rhs_only, num_sms, st, info);
+  else if (N == 7 && nt == 1) wide_launch_n<7, 1>(A, rhs_only, num_sms, st, info);
+  else throw Error(DGK_ERR_UNSUPPORTED, "wide FP64 stage: orders 6 and 7, tiles of 8, 16 or 32 elements");
+}
+
+}  // namespace dgk

@@ -261,16 +261,28 @@ struct RhsOp : Op {
       require(m->rows == np && m->cols == np, R.kname + ": " + m->name + " must be Np x Np");
       d.insert(d.end(), m->mat.begin(), m->mat.end());
     }
+    if constexpr (std::is_same<T, double>::value)
+      if (wide_supported(N)) {
+        int64_t nelems = 0;
+        for (int p = 0; p < tile_parts; ++p) nelems += r.K[p];
+        wide_te = wide_tile_elems(nelems, r.num_sms);
+      }
     auto dt = padded_rows<T>(d, 3 * np, np);
-    dmat.upload(dt.data(), dt.size() * sizeof(T));
     auto lt = padded_rows<T>(L->mat, np, nf);
+    if constexpr (std::is_same<T, double>::value)
+      if (wide_te) {
+        dt = wide_pack(d, 3, (int)np, (int)np);
+        lt = wide_pack(L->mat, 1, (int)np, nf);
+      }
+    dmat.upload(dt.data(), dt.size() * sizeof(T));
     lift.upload(lt.data(), lt.size() * sizeof(T));
     std::vector<int32_t> fmi(fm->mat.begin(), fm->mat.end());
     for (int32_t v : fmi) require(v >= 0 && v < np, R.kname + ": Fmask entry out of range");
     fmask.upload(fmi.data(), fmi.size() * sizeof(int32_t));
     // TMA-pipelined form when the order has one and every tile's streams start on 16-byte boundaries
     // (cp.async.bulk requirement); otherwise the register-staged form.
-    // FP64: TMA streaming + element-local products on the FP64 tensor path; FP32: register-staged form.
+    // FP64: TMA streaming + element-local products on the FP64 tensor path (orders 6 and 7: the form that streams
+    // the matrices); FP32: register-staged form.
     const char *no_tma = std::getenv("DGK_DISABLE_TMA");
     const bool tma_ok = !(no_tma && no_tma[0] == '1') && std::is_same<T, double>::value;
     const int te_tma = tma_ok ? dmma_tile_elems(N) : 0;
@@ -292,12 +304,13 @@ struct RhsOp : Op {
       throw Error(DGK_ERR_UNSUPPORTED, R.kname + ": compact=1 is built for the FP64 tensor-path stage (orders 1..5, "
                                                  "16-byte aligned partitions)");
     if (!use_tma) {
-      auto tl = make_tiles(r, *u, face[0], tile_elems(N), (int)np, nf, tile_parts);
+      auto tl = make_tiles(r, *u, face[0], wide_te ? wide_te : tile_elems(N), (int)np, nf, tile_parts);
       ntiles = (int)tl.size();
       tiles.upload(tl.data(), tl.size() * sizeof(Tile));
     }
   }
   bool use_tma = false;
+  int wide_te = 0;  // FP64 orders 6 and 7: elements per tile
   // The compact form's inputs, derived once from the bound arrays: the per-element geometry (checked
   // straight-sided), the gather map as neighbour bases and face-order codes, and each tile's first slot.
   void build_compact(Runner &r, Roles &R, const std::vector<Tile> &tl, int np, int nfp, int tile_parts) {
@@ -391,7 +404,12 @@ struct RhsOp : Op {
     }
     bool done = false;
     if constexpr (std::is_same<T, double>::value)
-      if (use_tma) done = launch_rhs_dmma(N, A, rhs_only, r.num_sms, r.stream(), &info);
+      if (use_tma) {
+        done = launch_rhs_dmma(N, A, rhs_only, r.num_sms, r.stream(), &info);
+      } else if (wide_te) {
+        launch_rhs_wide(N, wide_te, A, rhs_only, r.num_sms, r.stream(), &info);
+        done = true;
+      }
     if (!done) launch_rhs<T>(N, A, rhs_only, r.num_sms, r.stream(), &info);
     if (!rhs_only) std::swap(u->dptr, unext->dptr);  // "u" always names the newest state
   }
