@@ -2,16 +2,18 @@
 // 483 KB) fit neither registers nor shared memory.
 //
 // The products run on the FP64 tensor path (mma.sync m8n8k4) with the matrices streamed from L2: the operator stores
-// them in fragment order, so a warp's A fragment is 256 consecutive bytes, and every fragment is used for NT n-tiles of
-// 8 elements before the next one, which is loaded two k-steps ahead.  At NT = 4 that is 16 bytes of matrix per clock
-// and SM at the full FP64 rate (64 FMAs per clock and SM).  A CTA holds one tile of 8 NT elements: state, volume terms
-// and face terms in shared memory (100 KB at NT = 4), rows stored at strides of 4 or 12 mod 16 values, which keeps the
-// fragment loads free of bank conflicts.  The nine metrics and four face arrays are read once, straight from global
-// memory, 64 consecutive bytes per element, and brought into L2 one tile ahead by bulk prefetches.  Two CTAs share an
-// SM and drift apart, so one's memory phases run under the other's products; each warp owns one or two 8-row m-tiles.
+// them in fragment order, so a warp's A fragment is 256 consecutive bytes, loaded two k-steps ahead and used for NT
+// n-tiles of 8 elements.  A CTA holds one tile of 8 NT elements: state, volume terms and face terms in shared memory
+// (51 KB at order 7 and NT = 2), rows stored at strides of 4 or 12 mod 16 values, which keeps the fragment loads free
+// of bank conflicts.  The nine metrics and four face arrays are read once, straight from global memory, 64 consecutive
+// bytes per element.  They are brought into L2 by bulk prefetches shortly before their phase: prefetched a whole tile
+// ahead, the CTAs' tiles together outgrow L2, and prefetched ahead of a phase that loads itself, they delay it (order 7,
+// 16^3 x 6: 1012 us per LSERK4 step a tile ahead, 860 as here, with NT = 4).  Several small CTAs share an SM and drift
+// apart, so one's memory phases run under another's products: three CTAs of 16 elements take
+// 775 us, two of 16 take 840 and two of 32 take 860.  Each warp owns one or two 8-row m-tiles.
 //
-// Bound by the FP64 rate (60,480 FMAs per element at order 7).
-// @WIDE@
+// Bound by the FP64 rate (60,480 FMAs per element at order 7, 82 us of the 155 us per stage) and by the latency of
+// the memory phases.  The form before it read a matrix entry per FMA through L1: 655 us per stage.
 #include <algorithm>
 #include <cstdint>
 
@@ -31,6 +33,7 @@ struct WideCfg {
   static constexpr int MT = (NP + 7) / 8, KT = NP / 4, KL = NF / 4;
   static constexpr int WARPS = (MT + 1) / 2;  // one or two m-tiles per warp
   static constexpr int THREADS = 32 * WARPS;
+  static constexpr int MINB = N == 6 ? 4 : 3;  // CTAs per SM
   static constexpr int SU = (NP + 7) / 16 * 16 + (NP % 16 <= 4 ? 4 : 12);  // row strides: 4 or 12 mod 16
   static constexpr int SF = NF / 16 * 16 + 4;
   static constexpr size_t SMEM = sizeof(double) * (size_t)TE * (2 * SU + SF) + sizeof(int) * NF;
@@ -45,6 +48,13 @@ __device__ __forceinline__ void wide_dmma(double &c0, double &c1, double a, doub
                : "d"(a), "d"(b));
 }
 
+// A matrix fragment's load, kept where it is written: as a plain load the compiler moves it down to its use
+__device__ __forceinline__ double wide_ldf(const double *p) {
+  double v;
+  asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+
 // L2 prefetch of a contiguous range, widened to 16-byte granules (the runner's arrays sit in 256-byte aligned slots)
 __device__ __forceinline__ void wide_prefetch(const void *p, size_t bytes) {
   const uintptr_t a = reinterpret_cast<uintptr_t>(p) & ~uintptr_t(15);
@@ -52,18 +62,23 @@ __device__ __forceinline__ void wide_prefetch(const void *p, size_t bytes) {
   if (e > a) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(e - a)) : "memory");
 }
 
-// lanes 0..15 of a warp each prefetch one of the streams that a tile reads
-__device__ __forceinline__ void wide_prefetch_tile(const RhsArgs<double> &A, const Tile &tl, int np, int nf, int lane) {
-  const size_t nn = (size_t)tl.nelem * np * sizeof(double), fn = (size_t)tl.nelem * nf;
+// lanes 0..9 of a warp each prefetch one of the streams that a tile reads after its volume products
+__device__ __forceinline__ void wide_prefetch_late(const RhsArgs<double> &A, const Tile &tl, int np, int lane) {
+  const size_t nn = (size_t)tl.nelem * np * sizeof(double);
   if (lane < 9) wide_prefetch(A.geo[lane] + tl.node_base, nn);
-  else if (lane < 13) wide_prefetch(A.face[lane - 9] + tl.face_base, fn * sizeof(double));
-  else if (lane == 13) wide_prefetch(A.u_in + tl.node_base, nn);
-  else if (lane == 14 && A.resu) wide_prefetch(A.resu + tl.node_base, nn);
-  else if (lane == 15) wide_prefetch(A.gmap + tl.face_base, fn * sizeof(int32_t));
+  else if (lane == 9 && A.resu) wide_prefetch(A.resu + tl.node_base, nn);
+}
+
+// lanes 0..5: the streams that a tile reads first
+__device__ __forceinline__ void wide_prefetch_early(const RhsArgs<double> &A, const Tile &tl, int np, int nf, int lane) {
+  const size_t fn = (size_t)tl.nelem * nf;
+  if (lane < 4) wide_prefetch(A.face[lane] + tl.face_base, fn * sizeof(double));
+  else if (lane == 4) wide_prefetch(A.u_in + tl.node_base, (size_t)tl.nelem * np * sizeof(double));
+  else if (lane == 5) wide_prefetch(A.gmap + tl.face_base, fn * sizeof(int32_t));
 }
 
 template <int N, int NT>
-__global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, 2) rhs_stage_wide_kernel(const RhsArgs<double> A, int rhs_only) {
+__global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB) rhs_stage_wide_kernel(const RhsArgs<double> A, int rhs_only) {
   using C = WideCfg<N, NT>;
   constexpr int NP = C::NP, NF = C::NF, MT = C::MT, KT = C::KT, KL = C::KL, SU = C::SU, SF = C::SF, TE = C::TE;
   constexpr int THREADS = C::THREADS, W = C::WARPS, DEPTH = C::DEPTH;
@@ -75,14 +90,14 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, 2) rhs_stage_wide_ker
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ar = lane >> 2, ac = lane & 3;
   for (int i = tid; i < NF; i += THREADS) sfm[i] = A.fmask[i];
-  if (warp == 0) wide_prefetch_tile(A, A.tiles[blockIdx.x], NP, NF, lane);
+  if (warp == 0) wide_prefetch_early(A, A.tiles[blockIdx.x], NP, NF, lane);
   const double a = A.a, b = A.b, dt = A.dt;
   __syncthreads();
   for (int t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
     const Tile tl = A.tiles[t];
     const int ne = tl.nelem, nn = ne * NP, nfc = ne * NF;
     // state, and neighbour traces of this thread's face points (index batch, then gather batch)
-    constexpr int CH = 6;
+    constexpr int CH = 4;
     for (int x0 = tid; x0 < nn; x0 += CH * THREADS) {
       double v[CH];
 #pragma unroll
@@ -128,8 +143,7 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, 2) rhs_stage_wide_ker
         }
       }
     }
-    if (warp == W - 1 && t + (int)gridDim.x < A.ntiles) wide_prefetch_tile(A, A.tiles[t + gridDim.x], NP, NF, lane);
-    // volume terms of this warp's m-tiles
+    if (warp == 0) wide_prefetch_late(A, tl, NP, lane);
 #pragma unroll 1
     for (int mt = warp; mt < MT; mt += W) {
       const double *ap = A.Dmat + (size_t)mt * KT * 96 + lane;
@@ -142,14 +156,14 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, 2) rhs_stage_wide_ker
 #pragma unroll
       for (int d = 0; d < DEPTH - 1; ++d)
 #pragma unroll
-        for (int m = 0; m < 3; ++m) f[d][m] = __ldg(ap + d * 96 + m * 32);
+        for (int m = 0; m < 3; ++m) f[d][m] = wide_ldf(ap + d * 96 + m * 32);
 #pragma unroll 1
       for (int k0 = 0; k0 < KT; k0 += DEPTH) {
 #pragma unroll
         for (int d = 0; d < DEPTH; ++d) {
           const int kk = k0 + d, kn = min(kk + DEPTH - 1, KT - 1);
 #pragma unroll
-          for (int m = 0; m < 3; ++m) f[(d + DEPTH - 1) % DEPTH][m] = __ldg(ap + kn * 96 + m * 32);
+          for (int m = 0; m < 3; ++m) f[(d + DEPTH - 1) % DEPTH][m] = wide_ldf(ap + kn * 96 + m * 32);
 #pragma unroll
           for (int n = 0; n < NT; ++n) {
             double bv = su[(8 * n + ar) * SU + 4 * kk + ac];
@@ -182,6 +196,7 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, 2) rhs_stage_wide_ker
       }
     }
     __syncthreads();  // face terms complete
+    if (warp == W - 1 && t + (int)gridDim.x < A.ntiles) wide_prefetch_early(A, A.tiles[t + gridDim.x], NP, NF, lane);
     // LIFT times the face terms, then the update; each lane reads back the volume terms it wrote
 #pragma unroll 1
     for (int mt = warp; mt < MT; mt += W) {
@@ -198,13 +213,13 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, 2) rhs_stage_wide_ker
         }
       double f[4];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) f[d] = __ldg(ap + d * 32);
+      for (int d = 0; d < 3; ++d) f[d] = wide_ldf(ap + d * 32);
 #pragma unroll 1
       for (int k0 = 0; k0 < KL; k0 += 4) {
 #pragma unroll
         for (int d = 0; d < 4; ++d) {
           const int kk = k0 + d;
-          f[(d + 3) % 4] = __ldg(ap + min(kk + 3, KL - 1) * 32);
+          f[(d + 3) % 4] = wide_ldf(ap + min(kk + 3, KL - 1) * 32);
 #pragma unroll
           for (int n = 0; n < NT; ++n) wide_dmma(c[n][0], c[n][1], f[d], sf[(8 * n + ar) * SF + 4 * kk + ac]);
         }
@@ -248,10 +263,9 @@ void wide_launch_n(const RhsArgs<double> &A, int rhs_only, int num_sms, cudaStre
 
 bool wide_supported(int N) { return N == 6 || N == 7; }
 
+// Tiles of 16 elements reuse a matrix fragment twice; below two such tiles per SM, tiles of 8 keep more SMs busy.
 int wide_tile_elems(int64_t nelems, int num_sms) {
-  for (int te : {32, 16})
-    if ((nelems + te - 1) / te >= 2 * (int64_t)num_sms) return te;
-  return 8;
+  return (nelems + 15) / 16 >= 2 * (int64_t)num_sms ? 16 : 8;
 }
 
 std::vector<double> wide_pack(const std::vector<double> &mats, int nmats, int rows, int cols) {
@@ -270,13 +284,11 @@ std::vector<double> wide_pack(const std::vector<double> &mats, int nmats, int ro
 void launch_rhs_wide(int N, int tile_elems, const RhsArgs<double> &A, int rhs_only, int num_sms, cudaStream_t st,
                      LaunchInfo *info) {
   const int nt = tile_elems / 8;
-  if (N == 6 && nt == 4) wide_launch_n<6, 4>(A, rhs_only, num_sms, st, info);
-  else if (N == 6 && nt == 2) wide_launch_n<6, 2>(A, rhs_only, num_sms, st, info);
+  if (N == 6 && nt == 2) wide_launch_n<6, 2>(A, rhs_only, num_sms, st, info);
   else if (N == 6 && nt == 1) wide_launch_n<6, 1>(A, rhs_only, num_sms, st, info);
-  else if (N == 7 && nt == 4) wide_launch_n<7, 4>(A, rhs_only, num_sms, st, info);
   else if (N == 7 && nt == 2) wide_launch_n<7, 2>(A, rhs_only, num_sms, st, info);
   else if (N == 7 && nt == 1) wide_launch_n<7, 1>(A, rhs_only, num_sms, st, info);
-  else throw Error(DGK_ERR_UNSUPPORTED, "wide FP64 stage: orders 6 and 7, tiles of 8, 16 or 32 elements");
+  else throw Error(DGK_ERR_UNSUPPORTED, "wide FP64 stage: orders 6 and 7, tiles of 8 or 16 elements");
 }
 
 }  // namespace dgk

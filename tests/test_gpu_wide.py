@@ -1,4 +1,4 @@
-"""FP64 stage of orders 6 and 7 at each of its tile sizes (8, 16 and 32 elements by problem size), with partial tiles,
+"""FP64 stage of orders 6 and 7 at both tile sizes (8 or 16 elements by problem size), with partial tiles,
 both volume forms, against a numpy evaluation on the problem's own arrays.  Bound per value: the rounding of the sums
 in either order, (terms) * 2^-52 times the sum of the terms' magnitudes."""
 import numpy as np
