@@ -108,6 +108,7 @@ constexpr int kMixedConnWords = 5;   // neighbour base per face, 4 packed 8-bit 
 struct MTile {
   int64_t node_base;  // value index of the slot's first node in the hi/lo/resu arrays
   int64_t elem_slot;  // index of the slot's first element in the compact geometry/connectivity arrays
+  int64_t face_base;  // value index of the slot's first face point in the gather map
   int32_t nelem;      // elements in the slot (<= kMixedSlotElems)
   int32_t part;       // partition (or instance)
 };
@@ -120,6 +121,7 @@ struct MixedArgs {
   float *resu;                   // LSERK residual, updated in place
   const float *geo;              // kMixedGeoWords per element slot
   const int32_t *conn;           // kMixedConnWords per element slot (tensor-core form: 4 tile-local words)
+  const int32_t *gmap;           // row form: the gather map (neighbour value index per face point)
   int64_t n_u_values;            // bound of every gathered value index
   const float *Dm;               // [NP][NPJ][3]: Dr, Ds, Dt entries interleaved per column, zero-padded
   const float *lift;             // [NP][4 Nfp]

@@ -43,6 +43,11 @@ bool launch_rhs_mixed(int N, const MixedArgs &A, int consumer_warps, int ring_ma
                       LaunchInfo *info);
 void prepare_rhs_mixed(int N, int consumer_warps);  // attributes, before any stream capture
 uint32_t mixed_slot_bytes(int N);  // 0 when the order has no such form
+// The same stage, bit for bit, with a matrix row per thread (rows.cu): orders 1..4, tiles of at most
+// rows_tile_elems(N) elements; rows_faster says whether a problem of nelems elements takes it.
+int rows_tile_elems(int N);
+bool rows_faster(int N, int64_t nelems, int num_sms);
+void launch_rhs_rows(int N, const MixedArgs &A, int num_sms, cudaStream_t st, LaunchInfo *info);
 // Mixed stage with the element-local products on the tensor cores (tcm.cu), orders 1..4: tiles of at most
 // tcm_tile_elems() elements and tcm_halo_capacity() halo faces (tile_halo, with halo positions from
 // tcm_halo_floats(N)); the operand buffer comes from tcm_pack_operands (Dr, Ds, Dt, LIFT row-major FP64).

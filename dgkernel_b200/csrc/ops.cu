@@ -481,8 +481,9 @@ struct MatmulOp : Op {
 // matrices Dr, Ds, Dt, LIFT, Fmask and Bary (Np x 4 barycentric coordinates of the nodes).
 struct MixedOp : Op {
   int N = 0, ntiles = 0, conservative = 0, ncodes = 0, warps = 11, ring = 0, tensor = 0, mma = 0;
+  bool rows = false;  // the form with a matrix row per thread (warps has no meaning there, a ring depth asks for the other)
   Binding *uhi, *ulo, *uhin, *ulon, *resu;
-  DevBuf tiles, geoE, conn, dm, lift, bary, vtx, ftab, fmask, amat, rexp, bmat;
+  DevBuf gown, tiles, geoE, conn, dm, lift, bary, vtx, ftab, fmask, amat, rexp, bmat;
   DevBuf tconn, hoff, hlist;  // tensor-core form: tile-local connectivity and the tiles' halo lists
   // learned-sensor viscosity (sensor=pp|mlp|mlp0 with mma=1)
   int lmode = 0;
@@ -666,15 +667,18 @@ struct MixedOp : Op {
       tcm_pack_operands(N, Dr->mat.data(), Ds->mat.data(), Dt->mat.data(), L->mat.data(), packed);
       bmat.upload(packed.data(), packed.size() * sizeof(uint16_t));
     }
-    const int te = tensor ? oz_tile_elems() : kMixedSlotElems;
+    rows = !tensor && !mma && ring == 0 && rows_faster(N, r.ktotal, r.num_sms);
+    if (rows) gown.upload(gm.data(), gm.size() * sizeof(int32_t));  // the map as it is now, like the compact form
+    const int te = tensor ? oz_tile_elems() : rows ? rows_tile_elems(N) : kMixedSlotElems;
     std::vector<MTile> tl;
     auto add_tile = [&](int p, int64_t s0, int64_t ne) {
       MTile x;
       x.node_base = uhi->offsets[p] + s0 * np;
       x.elem_slot = slot_prefix[p] + s0;
+      x.face_base = gmap->offsets[p] + s0 * nf;
       x.nelem = (int32_t)ne;
       x.part = p;
-      require((x.node_base * 4) % 16 == 0, R.kname + ": partition offsets of uhi must be 16-byte aligned");
+      require((uhi->offsets[p] * 4) % 16 == 0, R.kname + ": partition offsets of uhi must be 16-byte aligned");
       tl.push_back(x);
     };
     if (mma) {
@@ -820,7 +824,7 @@ struct MixedOp : Op {
       prepare_rhs_tcm(N, warps);
     else if (tensor)
       prepare_rhs_oz(N);
-    else
+    else if (!rows)
       prepare_rhs_mixed(N, warps);
   }
   void launch_tensor(Runner &r, const std::vector<double> &s) {
@@ -893,7 +897,10 @@ struct MixedOp : Op {
       std::swap(ulo->dptr, ulon->dptr);
       return;
     }
-    if (!launch_rhs_mixed(N, A, warps, ring, r.num_sms, r.stream(), &info))
+    A.gmap = gown.get<int32_t>();
+    if (rows)
+      launch_rhs_rows(N, A, r.num_sms, r.stream(), &info);
+    else if (!launch_rhs_mixed(N, A, warps, ring, r.num_sms, r.stream(), &info))
       throw Error(DGK_ERR_UNSUPPORTED, "mixed stage: no launch shape fits shared memory for this order");
     std::swap(uhi->dptr, uhin->dptr);  // "uhi"/"ulo" always name the newest state
     std::swap(ulo->dptr, ulon->dptr);
