@@ -19,8 +19,7 @@
 #include <cstdint>
 
 #include "dg_kernels.cuh"
-#include "kernels.hpp"
-#include "runner.hpp"
+#include "launch.cuh"
 #include "tma.cuh"
 
 namespace dgk {
@@ -80,6 +79,7 @@ __global__ void __launch_bounds__(32 * kSensorWarps) av_sensor_kernel(const AvAr
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int x = tid; x < NP * NP; x += blockDim.x) m.vinv[x] = A.Vinv[x];
   for (int x = tid; x < NP; x += blockDim.x) m.top[x] = A.top[x];
+  pdl_wait();
   if (A.mode == 2)
     for (int x = tid; x < mlp_params(NP); x += blockDim.x) m.w[x] = __ushort_as_half(A.mlp16[x]);
   __syncthreads();
@@ -105,6 +105,7 @@ __global__ void __launch_bounds__(32 * kSensorWarps) av_sensor_kernel(const AvAr
   for (int g = g0; g < ngroups; g += gstep) {
     const AvTile cur = tl;
     const int cne = ne;
+    if (lane == 0 && g + gstep >= ngroups) pdl_trigger();
 #pragma unroll
     for (int q = 0; q < FILL; ++q) {
       const int i = lane + 32 * q, e = i / NP;
@@ -306,6 +307,18 @@ __global__ void __launch_bounds__(FluxCfg<N, RHS>::THREADS, FluxCfg<N, RHS>::MIN
   const int ce = 8 * nt + 2 * ac;        // first of the two elements of the C fragment
   AvTile t0 = A.tiles[blockIdx.x], t1{};
   if (blockIdx.x + step < ntiles) t1 = A.tiles[blockIdx.x + step];
+  double aD[3][KT], aL[KL];
+#pragma unroll
+  for (int kk = 0; kk < KT; ++kk) {
+    const int j = 4 * kk + ac;
+    const bool in = row < NP && j < NP;
+    aD[0][kk] = in ? A.Dr[row * NP + j] : 0.0;
+    aD[1][kk] = in ? A.Ds[row * NP + j] : 0.0;
+    aD[2][kk] = in ? A.Dt[row * NP + j] : 0.0;
+  }
+#pragma unroll
+  for (int kk = 0; kk < KL; ++kk) aL[kk] = row < NP ? A.LIFT[row * NF + 4 * kk + ac] : 0.0;
+  pdl_wait();
   if (tid == 0) {
     flux_issue<N, RHS>(A, t0, ring, &full[0]);
     if (blockIdx.x + step < ntiles) flux_issue<N, RHS>(A, t1, ring + C::STAGE_B, &full[1]);
@@ -342,17 +355,6 @@ __global__ void __launch_bounds__(FluxCfg<N, RHS>::THREADS, FluxCfg<N, RHS>::MIN
     if (RHS) eB = be < tl.nelem ? A.eps[tl.node_base + be * NP] : 0.0;
   };
   load_idx(t0);
-  double aD[3][KT], aL[KL];
-#pragma unroll
-  for (int kk = 0; kk < KT; ++kk) {
-    const int j = 4 * kk + ac;
-    const bool in = row < NP && j < NP;
-    aD[0][kk] = in ? A.Dr[row * NP + j] : 0.0;
-    aD[1][kk] = in ? A.Ds[row * NP + j] : 0.0;
-    aD[2][kk] = in ? A.Dt[row * NP + j] : 0.0;
-  }
-#pragma unroll
-  for (int kk = 0; kk < KL; ++kk) aL[kk] = row < NP ? A.LIFT[row * NF + 4 * kk + ac] : 0.0;
   gather(t0);
   if (blockIdx.x + step < ntiles) load_idx(t1);
   const double a = A.a, b = A.b, dt = A.dt;
@@ -360,6 +362,7 @@ __global__ void __launch_bounds__(FluxCfg<N, RHS>::THREADS, FluxCfg<N, RHS>::MIN
   for (int t = blockIdx.x; t < ntiles; t += step, ++k) {
     const int s = k & 1;
     const bool has1 = t + step < ntiles, has2 = t + 2 * step < ntiles;
+    if (tid == 0 && !has1) pdl_trigger();
     AvTile t2{};
     if (has2) t2 = A.tiles[t + 2 * step];
     const bool ready = mbar_wait_bounded(&full[s], (uint32_t)(k >> 1) & 1u, kSpinLimit);
@@ -503,31 +506,20 @@ __global__ void __launch_bounds__(FluxCfg<N, RHS>::THREADS, FluxCfg<N, RHS>::MIN
   }
 }
 
-template <typename K>
-int av_attr(K kernel, int threads, size_t smem) {
-  cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "av smem");
-  int per = 0;
-  cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem), "av occupancy");
-  return std::max(1, per);
-}
-
 template <int N>
-void launch_av_n(const AvArgs &A, int num_sms, cudaStream_t st) {
+void launch_av_n(const AvArgs &A, int num_sms, cudaStream_t st, LaunchInfo (&info)[3]) {
   const size_t s0 = sizeof(SensorSmem<N>);
-  const int ps = av_attr(av_sensor_kernel<N>, 32 * kSensorWarps, s0);
+  const int ps = info[0].per_sm = resident_ctas(av_sensor_kernel<N>, 32 * kSensorWarps, s0, &info[0]);
   const int groups = A.ntiles * (AvCfg<N>::TE / 8);
   const int gs = std::max(1, std::min((groups + kSensorWarps - 1) / kSensorWarps, ps * num_sms));
-  av_sensor_kernel<N><<<gs, 32 * kSensorWarps, s0, st>>>(A);
-  cuda_check(cudaGetLastError(), "av_sensor_kernel launch");
+  launch_pdl(av_sensor_kernel<N>, gs, 32 * kSensorWarps, s0, st, A);
   if (A.prep_only) return;
   using Cg = FluxCfg<N, false>;
   using Cr = FluxCfg<N, true>;
-  const int pg = av_attr(av_flux_kernel<N, false>, Cg::THREADS, Cg::SMEM);
-  av_flux_kernel<N, false><<<std::min(A.ntiles, pg * num_sms), Cg::THREADS, Cg::SMEM, st>>>(A);
-  cuda_check(cudaGetLastError(), "av_flux_kernel (gradient) launch");
-  const int pr = av_attr(av_flux_kernel<N, true>, Cr::THREADS, Cr::SMEM);
-  av_flux_kernel<N, true><<<std::min(A.ntiles, pr * num_sms), Cr::THREADS, Cr::SMEM, st>>>(A);
-  cuda_check(cudaGetLastError(), "av_flux_kernel (right-hand side) launch");
+  const int pg = info[1].per_sm = resident_ctas(av_flux_kernel<N, false>, Cg::THREADS, Cg::SMEM, &info[1]);
+  launch_pdl(av_flux_kernel<N, false>, std::min(A.ntiles, pg * num_sms), Cg::THREADS, Cg::SMEM, st, A);
+  const int pr = info[2].per_sm = resident_ctas(av_flux_kernel<N, true>, Cr::THREADS, Cr::SMEM, &info[2]);
+  launch_pdl(av_flux_kernel<N, true>, std::min(A.ntiles, pr * num_sms), Cr::THREADS, Cr::SMEM, st, A);
 }
 
 // ---------------- MLP: forward, loss gradient (mean squared error), Adam, FP32 -> FP16 ----------------
@@ -813,13 +805,13 @@ int mlp_param_count(int nin) { return mlp_params(nin); }
 
 int av_tile_elems(int N) { return N == 1 ? AvCfg<1>::TE : N == 2 ? AvCfg<2>::TE : AvCfg<3>::TE; }
 
-void launch_av(int N, const AvArgs &A, int num_sms, cudaStream_t st) {
+void launch_av(int N, const AvArgs &A, int num_sms, cudaStream_t st, LaunchInfo (&info)[3]) {
   switch (N) {
-    case 1: launch_av_n<1>(A, num_sms, st); break;
-    case 2: launch_av_n<2>(A, num_sms, st); break;
-    case 3: launch_av_n<3>(A, num_sms, st); break;
-    case 4: launch_av_n<4>(A, num_sms, st); break;
-    case 5: launch_av_n<5>(A, num_sms, st); break;
+    case 1: launch_av_n<1>(A, num_sms, st, info); break;
+    case 2: launch_av_n<2>(A, num_sms, st, info); break;
+    case 3: launch_av_n<3>(A, num_sms, st, info); break;
+    case 4: launch_av_n<4>(A, num_sms, st, info); break;
+    case 5: launch_av_n<5>(A, num_sms, st, info); break;
     default: throw Error(DGK_ERR_UNSUPPORTED, "artificial-viscosity stage: orders 1..5");
   }
 }

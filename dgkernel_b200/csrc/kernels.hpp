@@ -84,7 +84,7 @@ void prepare_ls(int N);  // attributes, before any stream capture
 void launch_ls(int N, const LsArgs &A, int num_sms, cudaStream_t st);
 
 // Artificial-viscosity stage and the sensor MLP (av.cu).
-void launch_av(int N, const AvArgs &A, int num_sms, cudaStream_t st);
+void launch_av(int N, const AvArgs &A, int num_sms, cudaStream_t st, LaunchInfo (&info)[3]);
 int mlp_param_count(int nin);
 int av_tile_elems(int N);  // elements per tile of the viscosity kernels
 void launch_to_half(const float *in, void *out, int64_t n, cudaStream_t st);

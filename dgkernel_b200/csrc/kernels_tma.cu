@@ -14,6 +14,7 @@
 #include <type_traits>
 
 #include "dg_kernels.cuh"
+#include "launch.cuh"
 #include "tma.cuh"
 #include "kernels.hpp"
 #include "runner.hpp"
@@ -512,6 +513,7 @@ __global__ void __launch_bounds__(DmmaCfg<N, CP>::THREADS, DmmaCfg<N, CP>::MINB)
   __syncthreads();
 
   if (tid >= CONS) {
+    pdl_wait();
     // ---------------- producer warp: neighbour traces ----------------
     // Software-pipelined over the CTA's tiles: while the traces of tile t are gathered, the loads of tile t + G's
     // gather indices (from its descriptor, loaded one tile earlier) and of tile t + 2G's descriptor are in
@@ -594,6 +596,7 @@ __global__ void __launch_bounds__(DmmaCfg<N, CP>::THREADS, DmmaCfg<N, CP>::MINB)
     }
 #pragma unroll
   for (int kk = 0; kk < KL; ++kk) aL[kk] = arow < NP ? A.LIFT[arow * LDL + 4 * kk + acol] : 0.0;
+  pdl_wait();
   if (tid == 0) {
     for (int j = 0; j < 2; ++j)
       if ((int)blockIdx.x + j * G < A.ntiles) {
@@ -613,6 +616,7 @@ __global__ void __launch_bounds__(DmmaCfg<N, CP>::THREADS, DmmaCfg<N, CP>::MINB)
     const int s = k & 1;
     const uint32_t parity = (k >> 1) & 1;
     const bool has2 = t + 2 * G < A.ntiles;
+    if (tid == 0 && t + G >= A.ntiles) pdl_trigger();
     Tile t2 = {};
     int64_t slot2 = 0;
     if (has2) {
@@ -757,13 +761,10 @@ static bool dmma_launch_n(const RhsArgs<double> &A, int rhs_only, int num_sms, c
   using C = DmmaCfg<N, CP>;
   if (C::SMEM > 227 * 1024) return false;
   auto k = rhs_stage_dmma_kernel<N, CP>;
-  cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM), "smem attr");
-  int per = 0;
-  cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, C::THREADS, C::SMEM), "occupancy");
-  per = std::max(1, per);
+  const int per = resident_ctas(k, C::THREADS, C::SMEM, info);
   const int grid = std::min(A.ntiles, per * num_sms);
   if (info) *info = {grid, C::THREADS, (int)C::SMEM, per};
-  if (grid > 0) k<<<grid, C::THREADS, C::SMEM, st>>>(A, rhs_only);
+  if (grid > 0) launch_pdl(k, grid, C::THREADS, C::SMEM, st, A, rhs_only);
   return true;
 }
 

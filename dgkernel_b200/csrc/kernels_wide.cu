@@ -18,8 +18,7 @@
 #include <cstdint>
 
 #include "dg_kernels.cuh"
-#include "kernels.hpp"
-#include "runner.hpp"
+#include "launch.cuh"
 
 namespace dgk {
 
@@ -90,12 +89,14 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ar = lane >> 2, ac = lane & 3;
   for (int i = tid; i < NF; i += THREADS) sfm[i] = A.fmask[i];
+  pdl_wait();
   if (warp == 0) wide_prefetch_early(A, A.tiles[blockIdx.x], NP, NF, lane);
   const double a = A.a, b = A.b, dt = A.dt;
   __syncthreads();
   for (int t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
     const Tile tl = A.tiles[t];
     const int ne = tl.nelem, nn = ne * NP, nfc = ne * NF;
+    if (tid == 0 && t + (int)gridDim.x >= A.ntiles) pdl_trigger();
     // state, and neighbour traces of this thread's face points (index batch, then gather batch)
     constexpr int CH = 4;
     for (int x0 = tid; x0 < nn; x0 += CH * THREADS) {
@@ -250,13 +251,10 @@ template <int N, int NT>
 void wide_launch_n(const RhsArgs<double> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info) {
   using C = WideCfg<N, NT>;
   auto k = rhs_stage_wide_kernel<N, NT>;
-  cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM), "smem attr");
-  int per = 0;
-  cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, C::THREADS, C::SMEM), "occupancy");
-  per = std::max(1, per);
+  const int per = resident_ctas(k, C::THREADS, C::SMEM, info);
   const int grid = std::min(A.ntiles, per * num_sms);
   if (info) *info = {grid, C::THREADS, (int)C::SMEM, per};
-  if (grid > 0) k<<<grid, C::THREADS, C::SMEM, st>>>(A, rhs_only);
+  if (grid > 0) launch_pdl(k, grid, C::THREADS, C::SMEM, st, A, rhs_only);
 }
 
 }  // namespace

@@ -26,8 +26,7 @@
 #include <cstdint>
 
 #include "dg_kernels.cuh"
-#include "kernels.hpp"
-#include "runner.hpp"
+#include "launch.cuh"
 #include "tma.cuh"
 
 namespace dgk {
@@ -124,6 +123,7 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1) rhs_stage_mixed_kernel(const
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  pdl_wait();
 
   if (warp == CW) {  // producer: lane 0 streams the slots of this CTA's tiles through the ring
     if (lane == 0) {
@@ -141,6 +141,7 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1) rhs_stage_mixed_kernel(const
           bad = true;
           break;
         }
+        if (t + G >= A.ntiles) pdl_trigger();
         *reinterpret_cast<volatile int *>(&sTag[s]) = k;  // fill k/NS of slot s is issued (k-NS was consumed)
         issue_slot<N>(A, A.tiles[t], ring + (size_t)s * C::SLOT_B, &full[s]);
       }
@@ -371,8 +372,7 @@ bool launch_mixed_n(const MixedArgs &A0, int ring_max, int num_sms, cudaStream_t
   auto kern = rhs_stage_mixed_kernel<N, CW>;
   mixed_attr<N, CW>();
   const int grid = std::max(1, std::min(num_sms, A.ntiles));
-  kern<<<grid, 32 * (CW + 1), smem, st>>>(A);
-  cuda_check(cudaGetLastError(), "rhs_stage_mixed_kernel launch");
+  launch_pdl(kern, grid, 32 * (CW + 1), smem, st, A);
   if (info) *info = LaunchInfo{grid, 32 * (CW + 1), (int)smem, 1};
   return true;
 }

@@ -958,6 +958,7 @@ struct AvOp : Op {
   Binding *u, *unext = nullptr, *resu = nullptr, *geo[9], *face[4], *gmap, *eps = nullptr, *q[3] = {};
   Binding *mlp = nullptr, *feat = nullptr, *sig = nullptr, *mlps = nullptr;
   DevBuf tiles, dr, ds, dt, vinv, lift, fmask, top, hon, mlp16;
+  LaunchInfo info[3];
   AvOp(Runner &r, Roles &R, int feats) : features(feats) {
     static const char *gn[9] = {"Rx", "Ry", "Rz", "Sx", "Sy", "Sz", "Tx", "Ty", "Tz"};
     static const char *fn[4] = {"nx", "ny", "nz", "Fscale"};
@@ -1097,7 +1098,7 @@ struct AvOp : Op {
       A.sig_out = reinterpret_cast<float *>(sig->dptr);
       A.mlp_out = mlps ? reinterpret_cast<float *>(mlps->dptr) : nullptr;
       A.prep_only = 1;
-      launch_av(N, A, r.num_sms, r.stream());
+      launch_av(N, A, r.num_sms, r.stream(), info);
       return;
     }
     A.u_out = reinterpret_cast<double *>(unext->dptr);
@@ -1107,7 +1108,7 @@ struct AvOp : Op {
     A.a = s[0];
     A.b = s[1];
     A.dt = s[2];
-    launch_av(N, A, r.num_sms, r.stream());
+    launch_av(N, A, r.num_sms, r.stream(), info);
     std::swap(u->dptr, unext->dptr);
   }
 };

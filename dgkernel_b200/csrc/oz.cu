@@ -45,7 +45,7 @@
 #include <vector>
 
 #include "dg_kernels.cuh"
-#include "kernels.hpp"
+#include "launch.cuh"
 #include "runner.hpp"
 #include "tcgen05.cuh"
 #include "tma.cuh"
@@ -237,6 +237,7 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = (uint32_t)sMisc[1];
+  pdl_wait();
 
   if (warp == kOzCW + 1) {
     // producer, lane 0: the state slots (two ahead at most) and the matrix chunks of every tile in order.  The
@@ -273,6 +274,7 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
       for (int k = 0; !bad; ++k) {
         const int t = blockIdx.x + k * G;
         if (t >= A.ntiles) break;
+        if (t + G >= A.ntiles) pdl_trigger();
         for (int j = 0; j < S * CT; ++j, ++g) {
           const int rs = (int)(g % kOzRing);
           if (g >= kOzRing) {
@@ -645,7 +647,7 @@ bool launch_oz_n(const OzArgs &A, int num_sms, cudaStream_t st, LaunchInfo *info
   if (smem > 227u * 1024u) return false;
   oz_attr<N, CONS>();
   const int grid = std::max(1, std::min(num_sms, A.ntiles));
-  rhs_stage_oz_kernel<N, kOzDigits, CONS><<<grid, 32 * (kOzCW + 2), smem, st>>>(A);
+  launch_pdl(rhs_stage_oz_kernel<N, kOzDigits, CONS>, grid, 32 * (kOzCW + 2), smem, st, A);
   cuda_check(cudaGetLastError(), "rhs_stage_oz_kernel launch");
   if (info) *info = LaunchInfo{grid, 32 * (kOzCW + 2), (int)smem, 1};
   return true;

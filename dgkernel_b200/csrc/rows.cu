@@ -24,8 +24,7 @@
 #include <cstdint>
 
 #include "dg_kernels.cuh"
-#include "kernels.hpp"
-#include "runner.hpp"
+#include "launch.cuh"
 
 namespace dgk {
 
@@ -122,6 +121,7 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS, RowCfg<N>::MINB) rhs_stage
     if (bad) atomicExch(A.status, kStatusBadGather);
   };
   MTile t0 = A.tiles[blockIdx.x], t1{}, t2{};
+  pdl_wait();
   load_idx(t0);
   load_tile(t0);
   if (blockIdx.x + step < ntiles) {
@@ -133,6 +133,7 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS, RowCfg<N>::MINB) rhs_stage
   int p = 0;
   for (int t = blockIdx.x; t < ntiles; t += step, p ^= 1) {
     const int ne = t0.nelem;
+    if (tid == 0 && t + step >= ntiles) pdl_trigger();
     // (1) the tile's state and geometry into shared memory
     double u[G];
     float h[G], r[G], uP[G][NJ];
@@ -246,31 +247,13 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS, RowCfg<N>::MINB) rhs_stage
   }
 }
 
-// CTAs that share an SM, asked once per device
-template <int N, bool CONS>
-int rows_per_sm() {
-  static int per[64] = {};
-  int dev = 0;
-  cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-  const bool known = dev >= 0 && dev < 64;
-  int n = known ? per[dev] : 0;
-  if (n == 0) {
-    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rhs_stage_rows_kernel<N, CONS>, RowCfg<N>::THREADS, 0),
-               "rows occupancy");
-    n = std::max(1, n);
-    if (known) per[dev] = n;
-  }
-  return n;
-}
-
 template <int N, bool CONS>
 void rows_launch_n(const MixedArgs &A, int num_sms, cudaStream_t st, LaunchInfo *info) {
   using C = RowCfg<N>;
-  const int per = rows_per_sm<N, CONS>();
+  const int per = resident_ctas(rhs_stage_rows_kernel<N, CONS>, C::THREADS, 0, info);
   const int grid = std::min(A.ntiles, per * num_sms);
   if (info) *info = {grid, C::THREADS, (int)sizeof(RowSmem<N>), per};
-  if (grid > 0) rhs_stage_rows_kernel<N, CONS><<<grid, C::THREADS, 0, st>>>(A);
-  cuda_check(cudaGetLastError(), "rhs_stage_rows_kernel launch");
+  if (grid > 0) launch_pdl(rhs_stage_rows_kernel<N, CONS>, grid, C::THREADS, 0, st, A);
 }
 
 template <int N>

@@ -449,6 +449,8 @@ void Runner::configure_kernel(const char *kname, int n, const char *const *param
     Binding *b = find(params[i]);
     if (!b) throw Error(DGK_ERR_NOT_FOUND, "parameter configuration has no binding (" + std::string(params[i]) + ")");
     cfg.params.push_back({b, actions ? actions[i] : 0u});
+    if (b->is_scalar) cfg.scalars.push_back(b);
+    else if (cfg.params.back().actions & (DGK_COPY_TO | DGK_COPY_BACK)) cfg.copies = true;
   }
   configs_[kname] = std::move(cfg);
 }
@@ -457,6 +459,13 @@ void Runner::build_kernel(const char *kname, const char *op_id) {
   need_device(__func__);
   KernelConfig &cfg = config(kname);
   cfg.op = make_op(*this, cfg, op_id ? op_id : kname);
+  cfg.scalar_at.clear();
+  for (const std::string &s : cfg.op->scalar_names()) {
+    int at = -1;
+    for (size_t i = 0; i < cfg.scalars.size(); ++i)
+      if (cfg.scalars[i]->name == s) at = (int)i;
+    cfg.scalar_at.push_back(at);
+  }
 }
 
 void Runner::validate_offsets(const char *context) {
@@ -500,25 +509,21 @@ void Runner::check_status(const char *what) {
 // reference's warning), explicit values are taken in configuration order, and the result is ordered as the
 // operator consumes them.
 static std::vector<double> resolve_scalars(KernelConfig &cfg, int nscalars, const double *scalars) {
-  std::map<std::string, double> sv;
-  int sidx = 0;
-  for (auto &pu : cfg.params) {
-    if (!pu.b->is_scalar) continue;
-    if (pu.b->scalar_bound) {
-      if (sidx < nscalars && scalars[sidx] != pu.b->scalar_value)
-        std::fprintf(stderr, "dgk: WARNING scalar %s is bound to %g; the explicit value %g is ignored\n",
-                     pu.b->name.c_str(), pu.b->scalar_value, scalars[sidx]);
-      sv[pu.b->name] = pu.b->scalar_value;
-    } else if (sidx < nscalars) {
-      sv[pu.b->name] = scalars[sidx];
-    }
-    ++sidx;
+  for (size_t i = 0; i < cfg.scalars.size() && (int)i < nscalars; ++i) {
+    const Binding &b = *cfg.scalars[i];
+    if (b.scalar_bound && scalars[i] != b.scalar_value)
+      std::fprintf(stderr, "dgk: WARNING scalar %s is bound to %g; the explicit value %g is ignored\n", b.name.c_str(),
+                   b.scalar_value, scalars[i]);
   }
-  std::vector<double> vals;
-  for (const std::string &s : cfg.op->scalar_names()) {
-    auto f = sv.find(s);
-    if (f == sv.end()) throw Error(DGK_ERR_INVALID, "scalar " + s + " not provided");
-    vals.push_back(f->second);
+  std::vector<double> vals(cfg.scalar_at.size());
+  for (size_t k = 0; k < vals.size(); ++k) {
+    const int at = cfg.scalar_at[k];
+    if (at >= 0 && cfg.scalars[(size_t)at]->scalar_bound)
+      vals[k] = cfg.scalars[(size_t)at]->scalar_value;
+    else if (at >= 0 && at < nscalars)
+      vals[k] = scalars[at];
+    else
+      throw Error(DGK_ERR_INVALID, "scalar " + cfg.op->scalar_names()[k] + " not provided");
   }
   return vals;
 }
@@ -531,8 +536,9 @@ void Runner::execute_kernel(const char *kname, int nscalars, const double *scala
   need_device(__func__);
   if (!cfg.op) throw Error(DGK_ERR_STATE, "kernel " + std::string(kname) + " not compiled - use BuildKernel first");
   if (validate_) validate_offsets((std::string("before kernel ") + kname).c_str());
+  const bool copies = cfg.copies && host_ptrs;
   // pre-kernel copies (CopyTo)
-  for (size_t i = 0; i < cfg.params.size(); ++i)
+  for (size_t i = 0; copies && i < cfg.params.size(); ++i)
     if ((cfg.params[i].actions & DGK_COPY_TO) && host_ptrs && host_ptrs[i]) {
       Binding &b = *cfg.params[i].b;
       if (b.is_scalar) continue;
@@ -543,7 +549,7 @@ void Runner::execute_kernel(const char *kname, int nscalars, const double *scala
   cuda_check(cudaGetLastError(), "kernel launch");
   if (validate_) validate_offsets((std::string("after kernel ") + kname).c_str());
   bool back = false;
-  for (size_t i = 0; i < cfg.params.size(); ++i)
+  for (size_t i = 0; copies && i < cfg.params.size(); ++i)
     if ((cfg.params[i].actions & DGK_COPY_BACK) && host_ptrs && host_ptrs[i]) {
       Binding &b = *cfg.params[i].b;
       if (b.is_scalar) continue;

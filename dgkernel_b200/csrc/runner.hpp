@@ -73,6 +73,11 @@ struct KernelConfig {
   std::string name;
   std::vector<ParamUse> params;
   std::unique_ptr<Op> op;
+  // collected once, so that a launch does not walk the parameter list: whether any array is copied, the scalar
+  // parameters in order, and for each scalar of the operator its place among them (set by BuildKernel)
+  bool copies = false;
+  std::vector<Binding *> scalars;
+  std::vector<int> scalar_at;
 };
 
 class Runner {

@@ -35,7 +35,7 @@
 #include <cstdint>
 
 #include "dg_kernels.cuh"
-#include "kernels.hpp"
+#include "launch.cuh"
 #include "runner.hpp"
 #include "tcgen05.cuh"
 #include "tma.cuh"
@@ -223,6 +223,7 @@ __global__ void __launch_bounds__(32 * (CW + 2), 1) rhs_stage_tcm_kernel(const M
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = (uint32_t)sMisc[1];
+  pdl_wait();
 
   if (warp == CW + 1) {
     // producer warp, lane 0.  Slot s holds tile k, then k + 2.  Per tile: wait until every consumer thread has
@@ -279,6 +280,7 @@ __global__ void __launch_bounds__(32 * (CW + 2), 1) rhs_stage_tcm_kernel(const M
             request_list(k + 1);
           }
           held[s] = tl;
+          if (t + G >= A.ntiles) pdl_trigger();
           const uint32_t nb = round16((uint32_t)(tl.nelem * NP * 4));
           const uint32_t gb = (uint32_t)tl.nelem * kMixedGeoWords * 4;
           const uint32_t cb = (uint32_t)tl.nelem * 16u;
@@ -624,7 +626,7 @@ bool launch_tcm_n(const MixedArgs &A, int num_sms, cudaStream_t st, LaunchInfo *
   if (smem > 227u * 1024u) return false;
   tcm_attr<N, CW, CONS>();
   const int grid = std::max(1, std::min(num_sms, A.ntiles));
-  rhs_stage_tcm_kernel<N, CW, CONS><<<grid, 32 * (CW + 2), smem, st>>>(A);
+  launch_pdl(rhs_stage_tcm_kernel<N, CW, CONS>, grid, 32 * (CW + 2), smem, st, A);
   cuda_check(cudaGetLastError(), "rhs_stage_tcm_kernel launch");
   if (info) *info = LaunchInfo{grid, 32 * (CW + 2), (int)smem, 1};
   return true;

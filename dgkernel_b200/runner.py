@@ -159,7 +159,18 @@ class ParamConfig:
     """Per-kernel copy actions of a binding (runner/kernel_config.go:151-181)."""
 
     def __init__(self, name: str, known: bool):
-        self.name, self.known, self.actions = name, known, NoAction
+        self.name, self.known, self._actions = name, known, NoAction
+        self.kernels: list = []  # configurations that hold this parameter
+
+    @property
+    def actions(self) -> int:
+        return self._actions
+
+    @actions.setter
+    def actions(self, value: int):
+        self._actions = value
+        for k in self.kernels:
+            k.copies = None
 
     def CopyTo(self):
         self.actions |= CopyTo
@@ -194,6 +205,8 @@ class _Binding:
 class _Kernel:
     params: List[ParamConfig] = field(default_factory=list)
     built: bool = False
+    cname: bytes = b""
+    copies: Optional[list] = None  # (index, parameter) of those with copy actions; None: to be collected
 
 
 def _ptr(a: np.ndarray):
@@ -383,8 +396,10 @@ class Runner:
         names = (C.c_char_p * len(params))(*[p.name.encode() for p in params])
         acts = (C.c_uint32 * len(params))(*[p.actions for p in params])
         self._check(lib().dgk_configure_kernel(self._h, name.encode(), len(params), names, acts))
-        self.KernelConfigs[name] = _Kernel(list(params))
-        return self.KernelConfigs[name]
+        kc = self.KernelConfigs[name] = _Kernel(list(params), cname=name.encode())
+        for p in params:
+            p.kernels.append(kc)
+        return kc
 
     def GetKernelSignatureForConfig(self, name: str) -> str:
         """GetKernelSignatureForConfig (runner/kernel_execution.go:230-237)."""
@@ -415,11 +430,12 @@ class Runner:
         if name not in self.KernelConfigs:
             raise DGKError(2, f"kernel {name} not configured - use ConfigureKernel first")
         kc = self.KernelConfigs[name]
-        ptrs = (C.c_void_p * max(1, len(kc.params)))()
-        keep, later = [], []
-        for i, p in enumerate(kc.params):
+        if kc.copies is None:
+            kc.copies = [(i, p) for i, p in enumerate(kc.params) if p.actions & Copy]
+        ptrs, keep, later = None, [], []
+        for i, p in kc.copies:
             b = self.Bindings[p.name]
-            if b.is_scalar or b.host is None or not (p.actions & Copy):
+            if b.is_scalar or b.host is None:
                 continue
             if isinstance(b.host, (list, tuple)):  # partitioned: per-partition copies around the launch
                 if p.actions & CopyTo:
@@ -429,12 +445,20 @@ class Runner:
                 continue
             a = self._host_view(b, b.host)
             keep.append(a)
+            if ptrs is None:
+                ptrs = (C.c_void_p * len(kc.params))()
             ptrs[i] = a.ctypes.data
-        sv = np.ascontiguousarray(np.asarray(scalar_values, dtype=np.float64))
-        self._check(lib().dgk_execute_kernel(self._h, name.encode(), len(sv), sv.ctypes.data_as(C.POINTER(C.c_double)),
-                                             ptrs))
-        for n in later:
-            self._copy(n, False)
+        n = len(scalar_values)
+        try:
+            sv = (C.c_double * n)(*scalar_values)
+        except TypeError:
+            a = np.ascontiguousarray(np.asarray(scalar_values, dtype=np.float64))
+            sv = a.ctypes.data_as(C.POINTER(C.c_double))
+        rc = lib().dgk_execute_kernel(self._h, kc.cname, n, sv, ptrs)
+        if rc:
+            self._check(rc)
+        for nm in later:
+            self._copy(nm, False)
 
     def CaptureGraph(self, name: str, scalar_rows) -> Graph:
         """Record len(scalar_rows) (even) launches of kernel `name`, row l giving launch l's scalars, into one
