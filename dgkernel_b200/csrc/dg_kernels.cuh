@@ -73,6 +73,8 @@ struct RhsArgs {
   int64_t n_u_values;    // bound of gmap entries
   const T *Dmat;         // [3][NP][pad(NP)] Dr, Ds, Dt; rows padded to an even length (16-byte pairs)
   const T *LIFT;         // [NP][pad(NF)]
+  const double *D64, *L64;  // the same in FP64 for the forms on the FP64 tensor path (kernels_tma.cu: the layouts
+                            // above; kernels_wide.cu: wide_pack)
   const int32_t *fmask;  // [NF]
   T a, b, dt;            // LSERK stage coefficients
   int conservative;      // 0: -u (ux+uy+uz) (reference form), 1: -div(u^2/2 (1,1,1))

@@ -501,12 +501,7 @@ void launch_rhs(int N, const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStrea
     case 3: rhs_launch_n<T, 3>(A, rhs_only, num_sms, st, info); break;
     case 4: rhs_launch_n<T, 4>(A, rhs_only, num_sms, st, info); break;
     case 5: rhs_launch_n<T, 5>(A, rhs_only, num_sms, st, info); break;
-    default:
-      if constexpr (sizeof(T) == 4) {  // FP64 has its own form at these orders (launch_rhs_wide)
-        if (N == 6) return rhs_launch_n<T, 6>(A, rhs_only, num_sms, st, info);
-        if (N == 7) return rhs_launch_n<T, 7>(A, rhs_only, num_sms, st, info);
-      }
-      throw Error(DGK_ERR_UNSUPPORTED, "order N must be 1..7");
+    default: throw Error(DGK_ERR_UNSUPPORTED, "order N must be 1..5");  // 6 and 7: launch_rhs_wide
   }
 }
 

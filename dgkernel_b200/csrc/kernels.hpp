@@ -20,21 +20,19 @@ template <typename T>
 void launch_update(const Tile *tiles, int ntiles, int np, T *u, T *resu, const T *rhs, double c0, double c1, double c2,
                    int mode, int num_sms, cudaStream_t st);
 int tile_elems(int N);
-// TMA-pipelined form of the fused stage (kernels_tma.cu); returns false when the order has no TMA form.
+// Form with TMA streaming and the element-local products on the FP64 tensor path (kernels_tma.cu), orders 1..5.
 template <typename T>
-bool launch_rhs_tma(int N, const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info);
+bool launch_rhs_dmma(int N, const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info);
 template <typename T>
-int tma_tile_elems(int N);  // 0 when the order has no TMA form
-// FP64 form with TMA streaming and the element-local products on the FP64 tensor path (kernels_tma.cu).
-bool launch_rhs_dmma(int N, const RhsArgs<double> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info);
 int dmma_tile_elems(int N);  // 0 when the order has no such form
-// FP64 form of orders 6 and 7 with the matrices streamed in fragment order (kernels_wide.cu).  wide_pack lays out
-// `nmats` stacked row-major rows x cols matrices (cols a multiple of 4) for it; A.Dmat = wide_pack(Dr, Ds, Dt) and
-// A.LIFT = wide_pack(LIFT).  wide_tile_elems: elements per tile for a problem of nelems elements.
+// Form of orders 6 and 7 with the matrices streamed in fragment order (kernels_wide.cu).  wide_pack lays out
+// `nmats` stacked row-major rows x cols matrices (cols a multiple of 4) for it; A.D64 = wide_pack(Dr, Ds, Dt) and
+// A.L64 = wide_pack(LIFT).  wide_tile_elems: elements per tile for a problem of nelems elements.
 bool wide_supported(int N);
 int wide_tile_elems(int64_t nelems, int num_sms);
 std::vector<double> wide_pack(const std::vector<double> &mats, int nmats, int rows, int cols);
-void launch_rhs_wide(int N, int tile_elems, const RhsArgs<double> &A, int rhs_only, int num_sms, cudaStream_t st,
+template <typename T>
+void launch_rhs_wide(int N, int tile_elems, const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st,
                      LaunchInfo *info);
 
 // Mixed-precision stage (mixed.cu) with 4, 8 or 11 consumer warps per CTA and at most ring_max ring slots

@@ -1,4 +1,4 @@
-// Fused strong-form Lax-Friedrichs RHS + LSERK4 stage in FP64 at orders 6 and 7, where the reference matrices (237 and
+// Fused strong-form Lax-Friedrichs RHS + LSERK4 stage at orders 6 and 7, arrays in FP64 or FP32 (ST), where the reference matrices (237 and
 // 483 KB) fit neither registers nor shared memory.
 //
 // The products run on the FP64 tensor path (mma.sync m8n8k4) with the matrices streamed from L2: the operator stores
@@ -62,22 +62,25 @@ __device__ __forceinline__ void wide_prefetch(const void *p, size_t bytes) {
 }
 
 // lanes 0..9 of a warp each prefetch one of the streams that a tile reads after its volume products
-__device__ __forceinline__ void wide_prefetch_late(const RhsArgs<double> &A, const Tile &tl, int np, int lane) {
-  const size_t nn = (size_t)tl.nelem * np * sizeof(double);
+template <typename T>
+__device__ __forceinline__ void wide_prefetch_late(const RhsArgs<T> &A, const Tile &tl, int np, int lane) {
+  const size_t nn = (size_t)tl.nelem * np * sizeof(T);
   if (lane < 9) wide_prefetch(A.geo[lane] + tl.node_base, nn);
   else if (lane == 9 && A.resu) wide_prefetch(A.resu + tl.node_base, nn);
 }
 
 // lanes 0..5: the streams that a tile reads first
-__device__ __forceinline__ void wide_prefetch_early(const RhsArgs<double> &A, const Tile &tl, int np, int nf, int lane) {
+template <typename T>
+__device__ __forceinline__ void wide_prefetch_early(const RhsArgs<T> &A, const Tile &tl, int np, int nf, int lane) {
   const size_t fn = (size_t)tl.nelem * nf;
-  if (lane < 4) wide_prefetch(A.face[lane] + tl.face_base, fn * sizeof(double));
-  else if (lane == 4) wide_prefetch(A.u_in + tl.node_base, (size_t)tl.nelem * np * sizeof(double));
+  if (lane < 4) wide_prefetch(A.face[lane] + tl.face_base, fn * sizeof(T));
+  else if (lane == 4) wide_prefetch(A.u_in + tl.node_base, (size_t)tl.nelem * np * sizeof(T));
   else if (lane == 5) wide_prefetch(A.gmap + tl.face_base, fn * sizeof(int32_t));
 }
 
-template <int N, int NT>
-__global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB) rhs_stage_wide_kernel(const RhsArgs<double> A, int rhs_only) {
+template <int N, int NT, typename T>
+__global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB)
+    rhs_stage_wide_kernel(const RhsArgs<T> A, int rhs_only) {
   using C = WideCfg<N, NT>;
   constexpr int NP = C::NP, NF = C::NF, MT = C::MT, KT = C::KT, KL = C::KL, SU = C::SU, SF = C::SF, TE = C::TE;
   constexpr int THREADS = C::THREADS, W = C::WARPS, DEPTH = C::DEPTH;
@@ -91,7 +94,7 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB)
   for (int i = tid; i < NF; i += THREADS) sfm[i] = A.fmask[i];
   pdl_wait();
   if (warp == 0) wide_prefetch_early(A, A.tiles[blockIdx.x], NP, NF, lane);
-  const double a = A.a, b = A.b, dt = A.dt;
+  const T a = A.a, b = A.b, dt = A.dt;
   __syncthreads();
   for (int t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
     const Tile tl = A.tiles[t];
@@ -100,9 +103,9 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB)
     // state, and neighbour traces of this thread's face points (index batch, then gather batch)
     constexpr int CH = 4;
     for (int x0 = tid; x0 < nn; x0 += CH * THREADS) {
-      double v[CH];
+      T v[CH];
 #pragma unroll
-      for (int j = 0; j < CH; ++j) v[j] = x0 + j * THREADS < nn ? A.u_in[tl.node_base + x0 + j * THREADS] : 0.0;
+      for (int j = 0; j < CH; ++j) v[j] = x0 + j * THREADS < nn ? A.u_in[tl.node_base + x0 + j * THREADS] : T(0);
 #pragma unroll
       for (int j = 0; j < CH; ++j) {
         const int x = x0 + j * THREADS, e = x / NP;
@@ -112,42 +115,42 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB)
     __syncthreads();
     for (int x0 = tid; x0 < nfc; x0 += CH * THREADS) {
       int32_t src[CH];
-      double up[CH], fc[CH][4];
+      T up[CH], fc[CH][4];
 #pragma unroll
       for (int j = 0; j < CH; ++j) src[j] = x0 + j * THREADS < nfc ? __ldcs(A.gmap + tl.face_base + x0 + j * THREADS) : 0;
 #pragma unroll
       for (int j = 0; j < CH; ++j)
 #pragma unroll
         for (int m = 0; m < 4; ++m)
-          fc[j][m] = x0 + j * THREADS < nfc ? __ldcs(A.face[m] + tl.face_base + x0 + j * THREADS) : 0.0;
+          fc[j][m] = x0 + j * THREADS < nfc ? __ldcs(A.face[m] + tl.face_base + x0 + j * THREADS) : T(0);
 #pragma unroll
       for (int j = 0; j < CH; ++j) {
         const bool ok = src[j] >= 0 && (int64_t)src[j] < A.n_u_values;
-        up[j] = ok ? A.u_in[src[j]] : 0.0;
+        up[j] = ok ? A.u_in[src[j]] : T(0);
       }
 #pragma unroll
       for (int j = 0; j < CH; ++j) {
         const int x = x0 + j * THREADS;
         if (x < nfc) {
           const int e = x / NF, q = x - e * NF;
-          const double uM = su[e * SU + sfm[q]];
-          double uP = up[j];
+          const T uM = (T)su[e * SU + sfm[q]];
+          T uP = up[j];
           if (!(src[j] >= 0 && (int64_t)src[j] < A.n_u_values)) {  // rejected index: report it, use the interior trace
             atomicExch(A.status, kStatusBadGather);
             uP = uM;
           }
-          const double nsum = fc[j][0] + fc[j][1] + fc[j][2];
-          const double fM = 0.5 * uM * uM * nsum, fP = 0.5 * uP * uP * nsum;
-          const double an = fabs(nsum);
-          const double lam = fmax(fabs(uM) * an, fabs(uP) * an);
-          sf[e * SF + q] = fc[j][3] * (fM - (0.5 * (fM + fP) + 0.5 * lam * (uM - uP)));
+          const T nsum = fc[j][0] + fc[j][1] + fc[j][2];
+          const T fM = T(0.5) * uM * uM * nsum, fP = T(0.5) * uP * uP * nsum;
+          const T an = fabs(nsum);
+          const T lam = fmax(fabs(uM) * an, fabs(uP) * an);
+          sf[e * SF + q] = fc[j][3] * (fM - (T(0.5) * (fM + fP) + T(0.5) * lam * (uM - uP)));
         }
       }
     }
     if (warp == 0) wide_prefetch_late(A, tl, NP, lane);
 #pragma unroll 1
     for (int mt = warp; mt < MT; mt += W) {
-      const double *ap = A.Dmat + (size_t)mt * KT * 96 + lane;
+      const double *ap = A.D64 + (size_t)mt * KT * 96 + lane;
       double c[3][NT][2];
 #pragma unroll
       for (int m = 0; m < 3; ++m)
@@ -177,7 +180,7 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB)
       const int row = 8 * mt + ar;
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
-        double g[2][9];
+        T g[2][9];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int e = 8 * n + 2 * ac + h;
@@ -188,11 +191,11 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int e = 8 * n + 2 * ac + h;
-          const double ur = c[0][n][h], us = c[1][n][h], ut = c[2][n][h];
-          const double ux = g[h][0] * ur + g[h][3] * us + g[h][6] * ut;
-          const double uy = g[h][1] * ur + g[h][4] * us + g[h][7] * ut;
-          const double uz = g[h][2] * ur + g[h][5] * us + g[h][8] * ut;
-          if (row < NP && e < ne) sv[e * SU + row] = A.conservative ? -(ux + uy + uz) : -su[e * SU + row] * (ux + uy + uz);
+          const T ur = (T)c[0][n][h], us = (T)c[1][n][h], ut = (T)c[2][n][h];
+          const T ux = g[h][0] * ur + g[h][3] * us + g[h][6] * ut;
+          const T uy = g[h][1] * ur + g[h][4] * us + g[h][7] * ut;
+          const T uz = g[h][2] * ur + g[h][5] * us + g[h][8] * ut;
+          if (row < NP && e < ne) sv[e * SU + row] = A.conservative ? -(ux + uy + uz) : -(T)su[e * SU + row] * (ux + uy + uz);
         }
       }
     }
@@ -201,16 +204,17 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB)
     // LIFT times the face terms, then the update; each lane reads back the volume terms it wrote
 #pragma unroll 1
     for (int mt = warp; mt < MT; mt += W) {
-      const double *ap = A.LIFT + (size_t)mt * KL * 32 + lane;
+      const double *ap = A.L64 + (size_t)mt * KL * 32 + lane;
       const int row = 8 * mt + ar;
-      double c[NT][2], rs[NT][2];
+      double c[NT][2];
+      T rs[NT][2];
 #pragma unroll
       for (int n = 0; n < NT; ++n)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int e = 8 * n + 2 * ac + h;
           c[n][h] = 0.0;
-          rs[n][h] = (!rhs_only && row < NP && e < ne) ? __ldcs(A.resu + tl.node_base + e * NP + row) : 0.0;
+          rs[n][h] = (!rhs_only && row < NP && e < ne) ? __ldcs(A.resu + tl.node_base + e * NP + row) : T(0);
         }
       double f[4];
 #pragma unroll
@@ -232,13 +236,13 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB)
           const int e = 8 * n + 2 * ac + h;
           if (row < NP && e < ne) {
             const int64_t gi = tl.node_base + e * NP + row;
-            const double rhs = sv[e * SU + row] + c[n][h];
+            const T rhs = (T)sv[e * SU + row] + (T)c[n][h];
             if (rhs_only) {
               __stcs(A.rhs_out + gi, rhs);
             } else {
-              const double res = a * rs[n][h] + dt * rhs;
+              const T res = a * rs[n][h] + dt * rhs;
               __stcs(A.resu + gi, res);
-              __stcs(A.u_out + gi, su[e * SU + row] + b * res);
+              __stcs(A.u_out + gi, (T)su[e * SU + row] + b * res);
             }
           }
         }
@@ -247,10 +251,10 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB)
   }
 }
 
-template <int N, int NT>
-void wide_launch_n(const RhsArgs<double> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info) {
+template <int N, int NT, typename T>
+void wide_launch_n(const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info) {
   using C = WideCfg<N, NT>;
-  auto k = rhs_stage_wide_kernel<N, NT>;
+  auto k = rhs_stage_wide_kernel<N, NT, T>;
   const int per = resident_ctas(k, C::THREADS, C::SMEM, info);
   const int grid = std::min(A.ntiles, per * num_sms);
   if (info) *info = {grid, C::THREADS, (int)C::SMEM, per};
@@ -279,14 +283,18 @@ std::vector<double> wide_pack(const std::vector<double> &mats, int nmats, int ro
   return out;
 }
 
-void launch_rhs_wide(int N, int tile_elems, const RhsArgs<double> &A, int rhs_only, int num_sms, cudaStream_t st,
+template <typename T>
+void launch_rhs_wide(int N, int tile_elems, const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st,
                      LaunchInfo *info) {
   const int nt = tile_elems / 8;
-  if (N == 6 && nt == 2) wide_launch_n<6, 2>(A, rhs_only, num_sms, st, info);
-  else if (N == 6 && nt == 1) wide_launch_n<6, 1>(A, rhs_only, num_sms, st, info);
-  else if (N == 7 && nt == 2) wide_launch_n<7, 2>(A, rhs_only, num_sms, st, info);
-  else if (N == 7 && nt == 1) wide_launch_n<7, 1>(A, rhs_only, num_sms, st, info);
+  if (N == 6 && nt == 2) wide_launch_n<6, 2, T>(A, rhs_only, num_sms, st, info);
+  else if (N == 6 && nt == 1) wide_launch_n<6, 1, T>(A, rhs_only, num_sms, st, info);
+  else if (N == 7 && nt == 2) wide_launch_n<7, 2, T>(A, rhs_only, num_sms, st, info);
+  else if (N == 7 && nt == 1) wide_launch_n<7, 1, T>(A, rhs_only, num_sms, st, info);
   else throw Error(DGK_ERR_UNSUPPORTED, "wide FP64 stage: orders 6 and 7, tiles of 8 or 16 elements");
 }
+
+template void launch_rhs_wide<double>(int, int, const RhsArgs<double> &, int, int, cudaStream_t, LaunchInfo *);
+template void launch_rhs_wide<float>(int, int, const RhsArgs<float> &, int, int, cudaStream_t, LaunchInfo *);
 
 }  // namespace dgk

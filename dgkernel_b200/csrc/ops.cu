@@ -214,7 +214,7 @@ template <typename T>
 struct RhsOp : Op {
   int N, ntiles, rhs_only, conservative;
   Binding *u, *unext = nullptr, *resu = nullptr, *rhs = nullptr, *geo[9], *face[4], *gmap;
-  DevBuf dmat, lift, fmask, tiles;
+  DevBuf dmat, lift, d64, l64, fmask, tiles;
   // compact=1 (FP64): per-element geometry, compact connectivity and face-order table, each tile's first slot
   int compact = 0, ncodes = 0;
   DevBuf geoc, cconn, cftab, tslot;
@@ -261,39 +261,39 @@ struct RhsOp : Op {
       require(m->rows == np && m->cols == np, R.kname + ": " + m->name + " must be Np x Np");
       d.insert(d.end(), m->mat.begin(), m->mat.end());
     }
-    if constexpr (std::is_same<T, double>::value)
-      if (wide_supported(N)) {
-        int64_t nelems = 0;
-        for (int p = 0; p < tile_parts; ++p) nelems += r.K[p];
-        wide_te = wide_tile_elems(nelems, r.num_sms);
-      }
-    auto dt = padded_rows<T>(d, 3 * np, np);
-    auto lt = padded_rows<T>(L->mat, np, nf);
-    if constexpr (std::is_same<T, double>::value)
-      if (wide_te) {
-        dt = wide_pack(d, 3, (int)np, (int)np);
-        lt = wide_pack(L->mat, 1, (int)np, nf);
-      }
-    dmat.upload(dt.data(), dt.size() * sizeof(T));
-    lift.upload(lt.data(), lt.size() * sizeof(T));
+    if (wide_supported(N)) {
+      int64_t nelems = 0;
+      for (int p = 0; p < tile_parts; ++p) nelems += r.K[p];
+      wide_te = wide_tile_elems(nelems, r.num_sms);
+    }
+    const char *no_tma = std::getenv("DGK_DISABLE_TMA");
+    const int te_tma = no_tma && no_tma[0] == '1' ? 0 : dmma_tile_elems<T>(N);
+    // matrices in FP64 for the forms on the FP64 tensor path, in the state's type for the register-staged form
+    if (te_tma > 0 || wide_te) {
+      auto dt = wide_te ? wide_pack(d, 3, (int)np, (int)np) : padded_rows<double>(d, 3 * np, np);
+      auto lt = wide_te ? wide_pack(L->mat, 1, (int)np, nf) : padded_rows<double>(L->mat, np, nf);
+      d64.upload(dt.data(), dt.size() * sizeof(double));
+      l64.upload(lt.data(), lt.size() * sizeof(double));
+    } else {
+      auto dt = padded_rows<T>(d, 3 * np, np);
+      auto lt = padded_rows<T>(L->mat, np, nf);
+      dmat.upload(dt.data(), dt.size() * sizeof(T));
+      lift.upload(lt.data(), lt.size() * sizeof(T));
+    }
     std::vector<int32_t> fmi(fm->mat.begin(), fm->mat.end());
     for (int32_t v : fmi) require(v >= 0 && v < np, R.kname + ": Fmask entry out of range");
     fmask.upload(fmi.data(), fmi.size() * sizeof(int32_t));
-    // TMA-pipelined form when the order has one and every tile's streams start on 16-byte boundaries
-    // (cp.async.bulk requirement); otherwise the register-staged form.
-    // FP64: TMA streaming + element-local products on the FP64 tensor path (orders 6 and 7: the form that streams
-    // the matrices); FP32: register-staged form.
-    const char *no_tma = std::getenv("DGK_DISABLE_TMA");
-    const bool tma_ok = !(no_tma && no_tma[0] == '1') && std::is_same<T, double>::value;
-    const int te_tma = tma_ok ? dmma_tile_elems(N) : 0;
+    // Orders 1..5: TMA streaming with the products on the FP64 tensor path (a tile that does not start on 16 bytes is
+    // copied from the 16 bytes that hold its start); orders 6 and 7: the form that streams the matrices; the
+    // register-staged form where the environment turns the copies off.
     use_tma = false;
     if (te_tma > 0) {
       auto tl = make_tiles(r, *u, face[0], te_tma, (int)np, nf, tile_parts);
-      bool aligned = true;
+      bool aligned = true;  // the compact form asks for it
       for (const Tile &x : tl)
         aligned = aligned && (x.node_base * (int64_t)sizeof(T)) % 16 == 0 &&
                   (x.face_base * (int64_t)sizeof(T)) % 16 == 0 && (x.face_base * 4) % 16 == 0;
-      if (aligned) {
+      if ((aligned && std::is_same<T, double>::value) || !compact) {
         use_tma = true;
         ntiles = (int)tl.size();
         tiles.upload(tl.data(), tl.size() * sizeof(Tile));
@@ -310,7 +310,7 @@ struct RhsOp : Op {
     }
   }
   bool use_tma = false;
-  int wide_te = 0;  // FP64 orders 6 and 7: elements per tile
+  int wide_te = 0;  // orders 6 and 7: elements per tile
   // The compact form's inputs, derived once from the bound arrays: the per-element geometry (checked
   // straight-sided), the gather map as neighbour bases and face-order codes, and each tile's first slot.
   void build_compact(Runner &r, Roles &R, const std::vector<Tile> &tl, int np, int nfp, int tile_parts) {
@@ -387,6 +387,8 @@ struct RhsOp : Op {
     A.n_u_values = u->offsets.back();
     A.Dmat = dmat.get<T>();
     A.LIFT = lift.get<T>();
+    A.D64 = d64.get<double>();
+    A.L64 = l64.get<double>();
     A.fmask = fmask.get<int32_t>();
     if (!rhs_only) {
       A.a = (T)s[0];
@@ -402,15 +404,12 @@ struct RhsOp : Op {
       A.ncodes = ncodes;
       A.tile_slot = tslot.get<int64_t>();
     }
-    bool done = false;
-    if constexpr (std::is_same<T, double>::value)
-      if (use_tma) {
-        done = launch_rhs_dmma(N, A, rhs_only, r.num_sms, r.stream(), &info);
-      } else if (wide_te) {
-        launch_rhs_wide(N, wide_te, A, rhs_only, r.num_sms, r.stream(), &info);
-        done = true;
-      }
-    if (!done) launch_rhs<T>(N, A, rhs_only, r.num_sms, r.stream(), &info);
+    if (use_tma)
+      launch_rhs_dmma<T>(N, A, rhs_only, r.num_sms, r.stream(), &info);
+    else if (wide_te)
+      launch_rhs_wide<T>(N, wide_te, A, rhs_only, r.num_sms, r.stream(), &info);
+    else
+      launch_rhs<T>(N, A, rhs_only, r.num_sms, r.stream(), &info);
     if (!rhs_only) std::swap(u->dptr, unext->dptr);  // "u" always names the newest state
   }
 };
