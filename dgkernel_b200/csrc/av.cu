@@ -33,7 +33,7 @@ __host__ __device__ constexpr int mlp_params(int nin) { return kHid * nin + kHid
 template <int N>
 struct AvCfg {
   using O = Order<N>;
-  static constexpr int NP = O::NP, NFP = O::NFP, NF = O::NF, NFS = O::NFS;
+  static constexpr int NP = O::NP, NFP = O::NFP, NF = O::NF, NFS = frag_stride(NF);
   static constexpr int TE = N == 1 ? 32 : N == 2 ? 16 : 8;  // elements per tile: about 100 KB of ring for two CTAs per SM
   static constexpr int MT = (NP + 7) / 8, KT = (NP + 3) / 4, KL = NF / 4, NT = TE / 8;
 };

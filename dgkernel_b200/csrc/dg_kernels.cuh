@@ -30,6 +30,13 @@ enum : int { kStatusOk = 0, kStatusBadGather = 1 };
 // Even row stride of matrices as the kernels read them (pairs of entries load as one vector).
 __host__ __device__ constexpr int pad_even(int c) { return (c + 1) & ~1; }
 
+// Row stride (>= c) of FP64 operand rows in shared memory that mma.sync m8n8k4 B fragments are read from: 4 or 12 mod
+// 16 values, which puts the four rows of a half warp in different banks.
+__host__ __device__ constexpr int frag_stride(int c) {
+  while (c % 16 != 4 && c % 16 != 12) ++c;
+  return c;
+}
+
 template <int N>
 struct Order {
   static constexpr int NP = (N + 1) * (N + 2) * (N + 3) / 6;

@@ -48,7 +48,7 @@ struct DmmaShape {
 template <int N, bool CP, typename T>
 struct DmmaCfg {
   using O = Order<N>;
-  static constexpr int NP = O::NP, NF = O::NF, NFS = O::NFS;
+  static constexpr int NP = O::NP, NF = O::NF, NFS = frag_stride(NF);
   static constexpr int TE = DmmaShape<N, T>::TE, NW = DmmaShape<N, T>::NW;
   static constexpr int MT = (NP + 7) / 8;  // m-tiles (8 rows)
   static constexpr int KT = (NP + 3) / 4;  // k-steps of the derivative matrices

@@ -33,12 +33,10 @@ struct WideCfg {
   static constexpr int WARPS = (MT + 1) / 2;  // one or two m-tiles per warp
   static constexpr int THREADS = 32 * WARPS;
   static constexpr int MINB = N == 6 ? 4 : 3;  // CTAs per SM
-  static constexpr int SU = (NP + 7) / 16 * 16 + (NP % 16 <= 4 ? 4 : 12);  // row strides: 4 or 12 mod 16
-  static constexpr int SF = NF / 16 * 16 + 4;
+  static constexpr int SU = frag_stride(NP), SF = frag_stride(NF);
   static constexpr size_t SMEM = sizeof(double) * (size_t)TE * (2 * SU + SF) + sizeof(int) * NF;
   static constexpr int DEPTH = 3;  // A fragments in flight
   static_assert(NP % 4 == 0 && NF % 16 == 0 && KT % DEPTH == 0, "whole k-steps");
-  static_assert(SU >= NP && (SU % 16 == 4 || SU % 16 == 12) && SF >= NF, "row strides");
 };
 
 __device__ __forceinline__ void wide_dmma(double &c0, double &c1, double a, double b) {
