@@ -106,7 +106,8 @@ struct DiffArgs {
   const T *geo[9];
   T *out[3];   // differentiate: DuDx, DuDy, DuDz;  computeRHS: out[0] = rhsu
   int mode;    // 0 = differentiate, 1 = reference volume-only computeRHS
-  const T *Dmat;  // [3][NP][pad(NP)], rows padded to an even length
+  const double *D64;  // Dr, Ds, Dt: [3][NP][pad(NP)], rows padded to an even length (orders 6 and 7: wide_pack)
+  int *status;
 };
 
 // ---- mixed-precision stage (mixed.cu) ----

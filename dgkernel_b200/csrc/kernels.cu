@@ -377,81 +377,35 @@ __global__ void __launch_bounds__(Cfg<N>::THREADS, 2) rhs_stage_kernel(RhsArgs<T
   }
 }
 
-// Volume derivative microbench (`differentiate`) and the reference's volume-only computeRHS.
-template <typename T, int N, bool MSMEM>
-__global__ void __launch_bounds__(Cfg<N>::THREADS) diff_kernel(DiffArgs<T> A) {
-  using O = Order<N>;
-  using C = Cfg<N>;
-  constexpr int NP = O::NP, NPS = O::NPS, TE = C::TE, RG = C::RG;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *sD = reinterpret_cast<T *>(smem_raw);
-  T *su = sD + (MSMEM ? 3 * NP * Pad<NP>::V : 0);
-  T *sd = su + TE * NPS;
-  const int tid = threadIdx.x, nth = blockDim.x;
-  if (MSMEM)
-    for (int i = tid; i < 3 * NP * Pad<NP>::V; i += nth) sD[i] = A.Dmat[i];
-  const T *Dm = MSMEM ? sD : A.Dmat;
-  const int e_own = tid % TE, g_own = tid / TE;
-  __syncthreads();
-  for (int t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
-    const Tile tl = A.tiles[t];
-    const int ne = tl.nelem;
-    for (int idx = tid; idx < ne * NP; idx += nth) {
-      const int e = idx / NP, i = idx - e * NP;
-      su[e * NPS + i] = lds(A.u + tl.node_base + idx);
-    }
-    __syncthreads();
-    if (e_own < ne) {
-      T acc[3][RG];
-      rows_matvec<T, NP, NP, RG, 3, false>(Dm, su + e_own * NPS, g_own, acc);
-#pragma unroll
-      for (int r = 0; r < RG; ++r) {
-        const int i = g_own * RG + r;
-        if (i < NP) {
-#pragma unroll
-          for (int m = 0; m < 3; ++m) sd[m * TE * NPS + e_own * NPS + i] = acc[m][r];
-        }
-      }
-    }
-    __syncthreads();
-    for (int idx = tid; idx < ne * NP; idx += nth) {
-      const int e = idx / NP, i = idx - e * NP;
-      const int64_t gi = tl.node_base + idx;
-      const int so = e * NPS + i;
-      const T ur = sd[so], us = sd[TE * NPS + so], ut = sd[2 * TE * NPS + so];
-      const T ux = lds(A.geo[0] + gi) * ur + lds(A.geo[3] + gi) * us + lds(A.geo[6] + gi) * ut;
-      const T uy = lds(A.geo[1] + gi) * ur + lds(A.geo[4] + gi) * us + lds(A.geo[7] + gi) * ut;
-      const T uz = lds(A.geo[2] + gi) * ur + lds(A.geo[5] + gi) * us + lds(A.geo[8] + gi) * ut;
-      if (A.mode == 0) {
-        sts(A.out[0] + gi, ux);
-        sts(A.out[1] + gi, uy);
-        sts(A.out[2] + gi, uz);
-      } else {
-        sts(A.out[0] + gi, -su[so] * (ux + uy + uz));
-      }
-    }
-    __syncthreads();
-  }
-}
-
 // Elementwise updates over tiles: mode 0 = the reference's updateSolution
 // (resu = rka*resu + rkb*rhsu; u += resu), mode 1 = standard LSERK4 (resu = a*resu + dt*rhs; u += b*resu).
+// Bound by HBM; a thread's loads are issued four values at a time.
 template <typename T>
 __global__ void update_kernel(const Tile *tiles, int ntiles, int np, T *u, T *resu, const T *rhs, T c0, T c1, T c2,
                               int mode) {
+  constexpr int CH = 4;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const Tile tl = tiles[t];
     const int n = tl.nelem * np;
-    for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
-      const int64_t gi = tl.node_base + idx;
-      if (mode == 0) {
-        const T r = c0 * resu[gi] + c1 * rhs[gi];
-        resu[gi] = r;
-        u[gi] = u[gi] + r;
-      } else {
-        const T r = c0 * resu[gi] + c2 * rhs[gi];
-        resu[gi] = r;
-        u[gi] = u[gi] + c1 * r;
+    for (int x0 = threadIdx.x; x0 < n; x0 += CH * blockDim.x) {
+      T r[CH], v[CH], w[CH];
+#pragma unroll
+      for (int j = 0; j < CH; ++j) {
+        const int x = x0 + j * blockDim.x;
+        const int64_t gi = tl.node_base + x;
+        r[j] = x < n ? resu[gi] : T(0);
+        v[j] = x < n ? u[gi] : T(0);
+        w[j] = x < n ? rhs[gi] : T(0);
+      }
+#pragma unroll
+      for (int j = 0; j < CH; ++j) {
+        const int x = x0 + j * blockDim.x;
+        const int64_t gi = tl.node_base + x;
+        if (x < n) {
+          const T res = mode == 0 ? c0 * r[j] + c1 * w[j] : c0 * r[j] + c2 * w[j];
+          resu[gi] = res;
+          u[gi] = mode == 0 ? v[j] + res : v[j] + c1 * res;
+        }
       }
     }
   }
@@ -505,42 +459,6 @@ void launch_rhs(int N, const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStrea
   }
 }
 
-template <typename T, int N>
-static void diff_launch_n(const DiffArgs<T> &A, int num_sms, cudaStream_t st, LaunchInfo *info) {
-  using O = Order<N>;
-  using C = Cfg<N>;
-  const int threads = C::THREADS;
-  const size_t base = sizeof(T) * (size_t)(4 * C::TE * O::NPS);
-  const size_t with = base + sizeof(T) * 3 * O::NP * Pad<O::NP>::V;
-  if (with <= 160 * 1024) {
-    auto k = diff_kernel<T, N, true>;
-    const int per = std::max(1, resident(k, threads, with));
-    const int grid = std::min(A.ntiles, per * num_sms);
-    if (info) *info = {grid, threads, (int)with, per};
-    if (grid > 0) k<<<grid, threads, with, st>>>(A);
-  } else {
-    auto k = diff_kernel<T, N, false>;
-    const int per = std::max(1, resident(k, threads, base));
-    const int grid = std::min(A.ntiles, per * num_sms);
-    if (info) *info = {grid, threads, (int)base, per};
-    if (grid > 0) k<<<grid, threads, base, st>>>(A);
-  }
-}
-
-template <typename T>
-void launch_diff(int N, const DiffArgs<T> &A, int num_sms, cudaStream_t st, LaunchInfo *info) {
-  switch (N) {
-    case 1: diff_launch_n<T, 1>(A, num_sms, st, info); break;
-    case 2: diff_launch_n<T, 2>(A, num_sms, st, info); break;
-    case 3: diff_launch_n<T, 3>(A, num_sms, st, info); break;
-    case 4: diff_launch_n<T, 4>(A, num_sms, st, info); break;
-    case 5: diff_launch_n<T, 5>(A, num_sms, st, info); break;
-    case 6: diff_launch_n<T, 6>(A, num_sms, st, info); break;
-    case 7: diff_launch_n<T, 7>(A, num_sms, st, info); break;
-    default: throw Error(DGK_ERR_UNSUPPORTED, "order N must be 1..7");
-  }
-}
-
 template <typename T>
 void launch_update(const Tile *tiles, int ntiles, int np, T *u, T *resu, const T *rhs, double c0, double c1, double c2,
                    int mode, int num_sms, cudaStream_t st) {
@@ -550,8 +468,6 @@ void launch_update(const Tile *tiles, int ntiles, int np, T *u, T *resu, const T
 
 template void launch_rhs<double>(int, const RhsArgs<double> &, int, int, cudaStream_t, LaunchInfo *);
 template void launch_rhs<float>(int, const RhsArgs<float> &, int, int, cudaStream_t, LaunchInfo *);
-template void launch_diff<double>(int, const DiffArgs<double> &, int, cudaStream_t, LaunchInfo *);
-template void launch_diff<float>(int, const DiffArgs<float> &, int, cudaStream_t, LaunchInfo *);
 template void launch_update<double>(const Tile *, int, int, double *, double *, const double *, double, double, double,
                                     int, int, cudaStream_t);
 template void launch_update<float>(const Tile *, int, int, float *, float *, const float *, double, double, double, int,

@@ -14,8 +14,13 @@ struct LaunchInfo {
 
 template <typename T>
 void launch_rhs(int N, const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info);
+// Volume derivative: orders 1..5 in tiles of diff_tile_elems (kernels_tma.cu), orders 6 and 7 in tiles of
+// wide_tile_elems (kernels_wide.cu).
 template <typename T>
 void launch_diff(int N, const DiffArgs<T> &A, int num_sms, cudaStream_t st, LaunchInfo *info);
+int diff_tile_elems(int N);
+template <typename T>
+void launch_diff_wide(int N, int tile_elems, const DiffArgs<T> &A, int num_sms, cudaStream_t st, LaunchInfo *info);
 template <typename T>
 void launch_update(const Tile *tiles, int ntiles, int np, T *u, T *resu, const T *rhs, double c0, double c1, double c2,
                    int mode, int num_sms, cudaStream_t st);

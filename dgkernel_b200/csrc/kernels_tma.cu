@@ -591,4 +591,155 @@ template bool launch_rhs_dmma<float>(int, const RhsArgs<float> &, int, int, cuda
 template int dmma_tile_elems<double>(int);
 template int dmma_tile_elems<float>(int);
 
+// ------------------------------------------------------------------------------------------------
+// Volume derivative (`differentiate`) and the reference's volume-only computeRHS, orders 1..5.
+//
+// The stage's volume part alone: u and the nine metrics through a two-slot ring of bulk copies, Dr, Ds, Dt in registers
+// (one warp per 8-row m-tile and NW n-tiles), products on the FP64 tensor path, results stored from the epilogue.  No
+// data passes between warps, so a tile has one barrier, after which its slot is refilled.  Bound by HBM: two CTAs
+// per SM with 45 KB slots at order 4.  Order 4, 32^3 x 6, FP64: 110-114 us (715 MB, 0.97 of the copy rate) from 176 with
+// the register-staged form on the FP64 cores.  Tiles of 8 elements and three CTAs measured the same (117 against 119 us
+// per call) with twice the tile list to build.
+// ------------------------------------------------------------------------------------------------
+template <int N, typename T>
+struct DiffCfg {
+  using O = Order<N>;
+  static constexpr int NP = O::NP, TE = N == 1 ? 32 : 16, NW = N >= 3 ? 2 : 1;
+  static constexpr int MT = (NP + 7) / 8, KT = (NP + 3) / 4;
+  static constexpr int THREADS = 32 * MT * (TE / 8 / NW);
+  static constexpr int AV = 16 / sizeof(T);
+  static constexpr uint32_t NODE_B = TE * NP * sizeof(T) + 16, STAGE_B = 10 * NODE_B;
+  static constexpr int NS = NODE_B / sizeof(T);
+  static constexpr size_t SMEM = 2 * (size_t)STAGE_B + 16;
+  static constexpr int PER = (int)(227 * 1024 / (SMEM + 1024));  // CTAs that share an SM by shared memory
+  static constexpr int MINB = N == 5 || PER < 3 ? 2 : 3;
+};
+
+template <int N, typename T>
+__device__ __forceinline__ void diff_issue(const DiffArgs<T> &A, const Tile &tl, char *stage, uint64_t *bar) {
+  using C = DiffCfg<N, T>;
+  const int ns = (int)(tl.node_base & (C::AV - 1));
+  const uint32_t nb = round16((uint32_t)((tl.nelem * C::NP + ns) * sizeof(T)));
+  mbar_expect_tx(bar, 10 * nb);
+  bulk_g2s(stage, A.u + tl.node_base - ns, nb, bar);
+#pragma unroll
+  for (int m = 0; m < 9; ++m) bulk_g2s(stage + (1 + m) * C::NODE_B, A.geo[m] + tl.node_base - ns, nb, bar);
+}
+
+template <int N, typename T>
+__global__ void __launch_bounds__(DiffCfg<N, T>::THREADS, DiffCfg<N, T>::MINB) diff_dmma_kernel(const DiffArgs<T> A) {
+  using C = DiffCfg<N, T>;
+  constexpr int NP = C::NP, KT = C::KT, MT = C::MT, NW = C::NW, NS = C::NS, LDD = pad_even(NP);
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  char *ring = reinterpret_cast<char *>(smem_raw);
+  uint64_t *full = reinterpret_cast<uint64_t *>(ring + 2 * C::STAGE_B);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, step = gridDim.x;
+  if (tid == 0) {
+    mbar_init(&full[0], 1);
+    mbar_init(&full[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  const int mt = warp % MT, nt = warp / MT, acol = lane & 3;
+  const int arow = mt * 8 + (lane >> 2);
+  const int be = nt * NW * 8 + (lane >> 2), ce = nt * NW * 8 + 2 * acol;
+  double aD[3][KT];
+#pragma unroll
+  for (int m = 0; m < 3; ++m)
+#pragma unroll
+    for (int kk = 0; kk < KT; ++kk) {
+      const int j = 4 * kk + acol;
+      aD[m][kk] = (arow < NP && j < NP) ? A.D64[(m * NP + arow) * LDD + j] : 0.0;
+    }
+  pdl_wait();
+  Tile t0 = A.tiles[blockIdx.x], t1{};
+  if (blockIdx.x + step < A.ntiles) t1 = A.tiles[blockIdx.x + step];
+  if (tid == 0) {
+    diff_issue<N, T>(A, t0, ring, &full[0]);
+    if (blockIdx.x + step < A.ntiles) diff_issue<N, T>(A, t1, ring + C::STAGE_B, &full[1]);
+  }
+  int k = 0;
+  for (int t = blockIdx.x; t < A.ntiles; t += step, ++k) {
+    const int s = k & 1;
+    const bool has1 = t + step < A.ntiles, has2 = t + 2 * step < A.ntiles;
+    if (tid == 0 && !has1) pdl_trigger();
+    Tile t2{};
+    if (has2) t2 = A.tiles[t + 2 * step];
+    const bool ready = mbar_wait_bounded(&full[s], (uint32_t)(k >> 1) & 1u, kSpinLimit);
+    const int ne = t0.nelem;
+    const T *su = reinterpret_cast<const T *>(ring + s * C::STAGE_B) + (t0.node_base & (C::AV - 1));
+    const T *sg = su + NS;
+    double c[NW][3][2] = {};
+#pragma unroll
+    for (int kk = 0; kk < KT; ++kk) {
+      const int j = 4 * kk + acol;
+#pragma unroll
+      for (int n = 0; n < NW; ++n) {
+        const double bv = (j < NP && be + 8 * n < ne) ? (double)su[(be + 8 * n) * NP + j] : 0.0;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) dmma(c[n][m][0], c[n][m][1], aD[m][kk], bv);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < NW; ++n)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int e = ce + 8 * n + h;
+        if (arow < NP && e < ne) {
+          const int o = e * NP + arow;
+          const int64_t gi = t0.node_base + o;
+          const T ur = (T)c[n][0][h], us = (T)c[n][1][h], ut = (T)c[n][2][h];
+          const T ux = sg[o] * ur + sg[3 * NS + o] * us + sg[6 * NS + o] * ut;
+          const T uy = sg[NS + o] * ur + sg[4 * NS + o] * us + sg[7 * NS + o] * ut;
+          const T uz = sg[2 * NS + o] * ur + sg[5 * NS + o] * us + sg[8 * NS + o] * ut;
+          if (A.mode == 0) {
+            __stcs(A.out[0] + gi, ux);
+            __stcs(A.out[1] + gi, uy);
+            __stcs(A.out[2] + gi, uz);
+          } else {
+            __stcs(A.out[0] + gi, -su[o] * (ux + uy + uz));
+          }
+        }
+      }
+    if (!__syncthreads_and(ready)) {  // the slot is free; a wait that gave up ends every thread here
+      if (tid == 0) atomicExch(A.status, kStatusTimeoutCode);
+      mbar_wait_bounded(&full[s], (uint32_t)(k >> 1) & 1u, kSpinLimit);  // copies in flight land before the CTA goes
+      if (has1) mbar_wait_bounded(&full[s ^ 1], (uint32_t)((k + 1) >> 1) & 1u, kSpinLimit);
+      return;
+    }
+    if (tid == 0 && has2) {
+      fence_async_smem();
+      diff_issue<N, T>(A, t2, ring + s * C::STAGE_B, &full[s]);
+    }
+    t0 = t1;
+    t1 = t2;
+  }
+}
+
+template <int N, typename T>
+static void diff_launch_n(const DiffArgs<T> &A, int num_sms, cudaStream_t st, LaunchInfo *info) {
+  using C = DiffCfg<N, T>;
+  auto k = diff_dmma_kernel<N, T>;
+  const int per = resident_ctas(k, C::THREADS, C::SMEM, info);
+  const int grid = std::min(A.ntiles, per * num_sms);
+  if (info) *info = {grid, C::THREADS, (int)C::SMEM, per};
+  if (grid > 0) launch_pdl(k, grid, C::THREADS, C::SMEM, st, A);
+}
+
+template <typename T>
+void launch_diff(int N, const DiffArgs<T> &A, int num_sms, cudaStream_t st, LaunchInfo *info) {
+  switch (N) {
+    case 1: diff_launch_n<1, T>(A, num_sms, st, info); break;
+    case 2: diff_launch_n<2, T>(A, num_sms, st, info); break;
+    case 3: diff_launch_n<3, T>(A, num_sms, st, info); break;
+    case 4: diff_launch_n<4, T>(A, num_sms, st, info); break;
+    case 5: diff_launch_n<5, T>(A, num_sms, st, info); break;
+    default: throw Error(DGK_ERR_UNSUPPORTED, "order N must be 1..5");
+  }
+}
+template void launch_diff<double>(int, const DiffArgs<double> &, int, cudaStream_t, LaunchInfo *);
+template void launch_diff<float>(int, const DiffArgs<float> &, int, cudaStream_t, LaunchInfo *);
+
+int diff_tile_elems(int N) { return N == 1 ? 32 : 16; }
+
 }  // namespace dgk

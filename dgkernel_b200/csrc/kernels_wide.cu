@@ -76,6 +76,34 @@ __device__ __forceinline__ void wide_prefetch_early(const RhsArgs<T> &A, const T
   else if (lane == 5) wide_prefetch(A.gmap + tl.face_base, fn * sizeof(int32_t));
 }
 
+// Dr, Ds, Dt times the tile's elements for one m-tile: A fragments (3 per k-step) from ap, DEPTH - 1 k-steps ahead
+template <typename C, int NT>
+__device__ __forceinline__ void wide_volume(const double *ap, const double *su, int ar, int ac, int conservative,
+                                            double (&c)[3][NT][2]) {
+  constexpr int KT = C::KT, SU = C::SU, DEPTH = C::DEPTH;
+  double f[DEPTH][3];
+#pragma unroll
+  for (int d = 0; d < DEPTH - 1; ++d)
+#pragma unroll
+    for (int m = 0; m < 3; ++m) f[d][m] = wide_ldf(ap + d * 96 + m * 32);
+#pragma unroll 1
+  for (int k0 = 0; k0 < KT; k0 += DEPTH) {
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d) {
+      const int kk = k0 + d, kn = min(kk + DEPTH - 1, KT - 1);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) f[(d + DEPTH - 1) % DEPTH][m] = wide_ldf(ap + kn * 96 + m * 32);
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        double bv = su[(8 * n + ar) * SU + 4 * kk + ac];
+        if (conservative) bv = 0.5 * bv * bv;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) wide_dmma(c[m][n][0], c[m][n][1], f[d][m], bv);
+      }
+    }
+  }
+}
+
 template <int N, int NT, typename T>
 __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB)
     rhs_stage_wide_kernel(const RhsArgs<T> A, int rhs_only) {
@@ -154,27 +182,7 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB)
       for (int m = 0; m < 3; ++m)
 #pragma unroll
         for (int n = 0; n < NT; ++n) c[m][n][0] = c[m][n][1] = 0.0;
-      double f[DEPTH][3];
-#pragma unroll
-      for (int d = 0; d < DEPTH - 1; ++d)
-#pragma unroll
-        for (int m = 0; m < 3; ++m) f[d][m] = wide_ldf(ap + d * 96 + m * 32);
-#pragma unroll 1
-      for (int k0 = 0; k0 < KT; k0 += DEPTH) {
-#pragma unroll
-        for (int d = 0; d < DEPTH; ++d) {
-          const int kk = k0 + d, kn = min(kk + DEPTH - 1, KT - 1);
-#pragma unroll
-          for (int m = 0; m < 3; ++m) f[(d + DEPTH - 1) % DEPTH][m] = wide_ldf(ap + kn * 96 + m * 32);
-#pragma unroll
-          for (int n = 0; n < NT; ++n) {
-            double bv = su[(8 * n + ar) * SU + 4 * kk + ac];
-            if (A.conservative) bv = 0.5 * bv * bv;
-#pragma unroll
-            for (int m = 0; m < 3; ++m) wide_dmma(c[m][n][0], c[m][n][1], f[d][m], bv);
-          }
-        }
-      }
+      wide_volume<C, NT>(ap, su, ar, ac, A.conservative, c);
       const int row = 8 * mt + ar;
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
@@ -249,6 +257,81 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB)
   }
 }
 
+// Volume derivative (mode 0) and the reference's volume-only right-hand side (mode 1): the same products, results
+// stored from the epilogue.
+template <int N, int NT, typename T>
+__global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB) diff_wide_kernel(const DiffArgs<T> A) {
+  using C = WideCfg<N, NT>;
+  constexpr int NP = C::NP, MT = C::MT, KT = C::KT, SU = C::SU, TE = C::TE, THREADS = C::THREADS, W = C::WARPS;
+  __shared__ double su[TE * SU];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ar = lane >> 2, ac = lane & 3;
+  pdl_wait();
+  for (int t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
+    const Tile tl = A.tiles[t];
+    const int ne = tl.nelem, nn = ne * NP;
+    if (tid == 0 && t + (int)gridDim.x >= A.ntiles) pdl_trigger();
+    constexpr int CH = 4;
+    for (int x0 = tid; x0 < nn; x0 += CH * THREADS) {
+      T v[CH];
+#pragma unroll
+      for (int j = 0; j < CH; ++j) v[j] = x0 + j * THREADS < nn ? __ldcs(A.u + tl.node_base + x0 + j * THREADS) : T(0);
+#pragma unroll
+      for (int j = 0; j < CH; ++j) {
+        const int x = x0 + j * THREADS, e = x / NP;
+        if (x < nn) su[e * SU + x - e * NP] = v[j];
+      }
+    }
+    if (warp == 0 && lane < 9) wide_prefetch(A.geo[lane] + tl.node_base, (size_t)nn * sizeof(T));
+    __syncthreads();
+#pragma unroll 1
+    for (int mt = warp; mt < MT; mt += W) {
+      double c[3][NT][2] = {};
+      wide_volume<C, NT>(A.D64 + (size_t)mt * KT * 96 + lane, su, ar, ac, 0, c);
+      const int row = 8 * mt + ar;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        T g[2][9];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int e = 8 * n + 2 * ac + h;
+#pragma unroll
+          for (int m = 0; m < 9; ++m)
+            g[h][m] = (row < NP && e < ne) ? __ldcs(A.geo[m] + tl.node_base + e * NP + row) : T(0);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int e = 8 * n + 2 * ac + h;
+          if (row < NP && e < ne) {
+            const int64_t gi = tl.node_base + e * NP + row;
+            const T ur = (T)c[0][n][h], us = (T)c[1][n][h], ut = (T)c[2][n][h];
+            const T ux = g[h][0] * ur + g[h][3] * us + g[h][6] * ut;
+            const T uy = g[h][1] * ur + g[h][4] * us + g[h][7] * ut;
+            const T uz = g[h][2] * ur + g[h][5] * us + g[h][8] * ut;
+            if (A.mode == 0) {
+              __stcs(A.out[0] + gi, ux);
+              __stcs(A.out[1] + gi, uy);
+              __stcs(A.out[2] + gi, uz);
+            } else {
+              __stcs(A.out[0] + gi, -(T)su[e * SU + row] * (ux + uy + uz));
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();  // the tile's buffer is free
+  }
+}
+
+template <int N, int NT, typename T>
+void wide_diff_n(const DiffArgs<T> &A, int num_sms, cudaStream_t st, LaunchInfo *info) {
+  using C = WideCfg<N, NT>;
+  auto k = diff_wide_kernel<N, NT, T>;
+  const int per = resident_ctas(k, C::THREADS, 0, info);
+  const int grid = std::min(A.ntiles, per * num_sms);
+  if (info) *info = {grid, C::THREADS, 0, per};
+  if (grid > 0) launch_pdl(k, grid, C::THREADS, 0, st, A);
+}
+
 template <int N, int NT, typename T>
 void wide_launch_n(const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info) {
   using C = WideCfg<N, NT>;
@@ -292,6 +375,18 @@ void launch_rhs_wide(int N, int tile_elems, const RhsArgs<T> &A, int rhs_only, i
   else throw Error(DGK_ERR_UNSUPPORTED, "wide FP64 stage: orders 6 and 7, tiles of 8 or 16 elements");
 }
 
+template <typename T>
+void launch_diff_wide(int N, int tile_elems, const DiffArgs<T> &A, int num_sms, cudaStream_t st, LaunchInfo *info) {
+  const int nt = tile_elems / 8;
+  if (N == 6 && nt == 2) wide_diff_n<6, 2, T>(A, num_sms, st, info);
+  else if (N == 6 && nt == 1) wide_diff_n<6, 1, T>(A, num_sms, st, info);
+  else if (N == 7 && nt == 2) wide_diff_n<7, 2, T>(A, num_sms, st, info);
+  else if (N == 7 && nt == 1) wide_diff_n<7, 1, T>(A, num_sms, st, info);
+  else throw Error(DGK_ERR_UNSUPPORTED, "wide derivative: orders 6 and 7, tiles of 8 or 16 elements");
+}
+
+template void launch_diff_wide<double>(int, int, const DiffArgs<double> &, int, cudaStream_t, LaunchInfo *);
+template void launch_diff_wide<float>(int, int, const DiffArgs<float> &, int, cudaStream_t, LaunchInfo *);
 template void launch_rhs_wide<double>(int, int, const RhsArgs<double> &, int, int, cudaStream_t, LaunchInfo *);
 template void launch_rhs_wide<float>(int, int, const RhsArgs<float> &, int, int, cudaStream_t, LaunchInfo *);
 

@@ -139,7 +139,11 @@ std::vector<T> padded_rows(const std::vector<double> &v, int64_t rows, int64_t c
 std::vector<Tile> make_tiles(const Runner &r, const Binding &node, const Binding *face, int te, int np, int nf,
                              int nparts = -1) {
   std::vector<Tile> t;
-  for (int p = 0; p < (nparts < 0 ? r.npart : nparts); ++p)
+  const int np_ = nparts < 0 ? r.npart : nparts;
+  size_t n = 0;
+  for (int p = 0; p < np_; ++p) n += (size_t)((r.K[p] + te - 1) / te);
+  t.reserve(n);
+  for (int p = 0; p < np_; ++p)
     for (int64_t s = 0; s < r.K[p]; s += te) {
       Tile x;
       x.node_base = node.offsets[p] + s * np;
@@ -164,9 +168,10 @@ void same_layout(const Binding &a, const Binding &b, const std::string &what) {
 // Volume derivative (`differentiate`) and the reference's volume-only computeRHS.
 template <typename T>
 struct DiffOp : Op {
-  int N, mode, ntiles;
+  int N, mode, ntiles, te;
   Binding *u, *geo[9], *out[3];
   DevBuf dmat, tiles;
+  LaunchInfo info;
   DiffOp(Runner &r, Roles &R, int m) : mode(m) {
     static const char *gn[9] = {"Rx", "Ry", "Rz", "Sx", "Sy", "Sz", "Tx", "Ty", "Tz"};
     u = R.array(mode == 0 ? "U" : "u");
@@ -190,9 +195,11 @@ struct DiffOp : Op {
       require(m->rows == np && m->cols == np, R.kname + ": " + m->name + " must be Np x Np");
       d.insert(d.end(), m->mat.begin(), m->mat.end());
     }
-    auto dt = padded_rows<T>(d, 3 * np, np);
-    dmat.upload(dt.data(), dt.size() * sizeof(T));
-    auto tl = make_tiles(r, *u, nullptr, tile_elems(N), (int)np, 0);
+    const bool wide = wide_supported(N);
+    auto dt = wide ? wide_pack(d, 3, (int)np, (int)np) : padded_rows<double>(d, 3 * np, np);
+    dmat.upload(dt.data(), dt.size() * sizeof(double));
+    te = wide ? wide_tile_elems(r.ktotal, r.num_sms) : diff_tile_elems(N);
+    auto tl = make_tiles(r, *u, nullptr, te, (int)np, 0);
     ntiles = (int)tl.size();
     tiles.upload(tl.data(), tl.size() * sizeof(Tile));
   }
@@ -204,8 +211,12 @@ struct DiffOp : Op {
     for (int i = 0; i < 9; ++i) A.geo[i] = reinterpret_cast<const T *>(geo[i]->dptr);
     for (int i = 0; i < 3; ++i) A.out[i] = reinterpret_cast<T *>(out[i]->dptr);
     A.mode = mode;
-    A.Dmat = dmat.get<T>();
-    launch_diff<T>(N, A, r.num_sms, r.stream(), nullptr);
+    A.D64 = dmat.get<double>();
+    A.status = r.status_word();
+    if (wide_supported(N))
+      launch_diff_wide<T>(N, te, A, r.num_sms, r.stream(), &info);
+    else
+      launch_diff<T>(N, A, r.num_sms, r.stream(), &info);
   }
 };
 
