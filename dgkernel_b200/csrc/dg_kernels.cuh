@@ -215,11 +215,12 @@ struct LsArgs {
   int mode;                    // 1 PP, 2 MLP with PP fallback, 3 as 2 with outputs <= lo read as smooth
   double eps0, s0, kappa;
   float conf_lo, conf_hi;
-  const unsigned short *mlp16;
+  const float *mlp;            // the network's parameters (modes 2, 3)
+  double ratio0;               // energy ratios below it have sigma = 0: 10^(s0 - kappa), less a rounding margin
   double *eps;                 // per element slot
   int32_t *aslot;              // per element slot: index in the active list or -1
   int32_t *alist, *tflag, *vslot, *tlist;
-  int32_t *counts;             // [0] active, [1] touched, [2] network fallbacks to PP
+  int32_t *counts;             // [0] active (zero before a stage), [1] touched
   double *eq;                  // [active][Np][3]: eps q (a node's three components adjacent)
   double *visc;                // [touched][Np]: the viscous right-hand side
   int64_t nslots;

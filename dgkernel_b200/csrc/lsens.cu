@@ -7,7 +7,7 @@
 //               sigmoid; FP16 weights, FP32 sums; its hidden layers as TF32 tensor products with two-part
 //               inputs) on uhat / |uhat| with the PP fallback inside (lo, hi) and, in mode 3, outputs <= lo read
 //               as a smooth element; eps_e = eps0 sigma_e h_e / N; elements with eps_e > 0 form the active list.
-//   ls_touch    the active elements and their face neighbours are marked; ls_compact lists them (touched).
+//               The pass marks the active elements and their face neighbours, and ls_compact lists them (touched).
 //   ls_grad     active elements: q_d = D_d u + LIFT (Fscale n_d (uP - uM) / 2) (FP64 tensor path), stored as
 //               eps_e q_d.
 //   ls_div      touched elements: sum_d d/dx_d (eps_e q_d) + LIFT (Fscale / 2 sum_d n_d (epsP qP_d - epsM qM_d)),
@@ -22,15 +22,14 @@
 #include <cstdint>
 
 #include "dg_kernels.cuh"
-#include "kernels.hpp"
-#include "runner.hpp"
+#include "launch.cuh"
 
 namespace dgk {
 
 namespace {
 
 constexpr int kLsHid = 32;
-constexpr int kLsElems = 64;   // sensor pass: elements per block, 4 threads each
+constexpr int kLsWarps = 8;  // sensor pass: warps per block, 8 elements each at a time
 
 __host__ __device__ constexpr int ls_mlp_params(int nin) {
   return kLsHid * nin + kLsHid + kLsHid * kLsHid + kLsHid + kLsHid + 1;
@@ -63,16 +62,11 @@ __device__ __forceinline__ int64_t slot_of_value(const LsArgs &A, int64_t g, int
   return -1;
 }
 
-// TF32 helpers of the network's tensor products: x = hi + lo with both parts TF32 (round to nearest), an FP16
-// weight as its exact TF32 bit pattern (0 outside the matrix), and one m16n8k8 product accumulated into d.
+// TF32 helpers of the network's tensor products: x = hi + lo with both parts TF32 (round to nearest), and one m16n8k8 product accumulated into d.
 __device__ __forceinline__ void ls_tf32_split(float x, uint32_t &hi, uint32_t &lo) {
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
   const float r = x - __uint_as_float(hi);
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(r));
-}
-
-__device__ __forceinline__ uint32_t ls_tf32_w(const __half *W, int i, bool in) {
-  return in ? __float_as_uint(__half2float(W[i])) : 0u;
 }
 
 __device__ __forceinline__ void ls_mma_tf32(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
@@ -82,31 +76,97 @@ __device__ __forceinline__ void ls_mma_tf32(float (&d)[4], const uint32_t (&a)[4
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
+__device__ __forceinline__ void ls_dmma(double &c0, double &c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+
+// Sensor pass.  Each warp walks its own groups of 8 elements with no block barrier; the next group's state, first slot
+// and h / N are loaded while the current one is computed.  Lane (g = l / 4, c = l mod 4) of the tensor products holds
+// output rows g, g + 8, ... of elements 2c and 2c + 1, so the energies are summed and the features formed straight from
+// the accumulators, and every lane ends with one element: 2c + (g mod 2).  Shared memory is what bounds the pass (its
+// pipe was 85 % busy with the matrix and the weights read entry by entry and rows at conflicting strides), so Vinv and
+// the weights lie there in fragment order (one 8-byte load per lane and fragment) and the rows at strides that spread
+// the 8 rows of a fragment over the banks.  The logarithm and the sine of the ramp run only where the energy ratio can
+// reach it.  @LSENS@
 template <int N>
-__global__ void __launch_bounds__(4 * kLsElems, 3) ls_sensor_kernel(const LsArgs A) {
-  using O = Order<N>;
-  constexpr int NP = O::NP;
-  constexpr int NPP = NP + 1;  // padded row of the feature buffer
+struct LsSensorSmem {
+  static constexpr int NP = Order<N>::NP, MT = (NP + 7) / 8, KT = (NP + 3) / 4, K1 = (NP + 7) / 8, K2 = kLsHid / 8;
+  static constexpr int SU = frag_stride(NP);           // nodal values of an element
+  static constexpr int SX = (NP + 3) / 8 * 8 + 4;      // features: 4 mod 8, rows 4 banks apart (in some order)
+  static constexpr int SH = kLsHid + 4;                // hidden units
+  static_assert(SX >= NP && SX % 8 == 4, "feature row stride");
+  double vinv[MT * KT * 32];                           // [m-tile][k-step][lane]
+  double u[kLsWarps][8 * SU];
+  float x[kLsWarps][8 * SX], h[kLsWarps][8 * SH];
+  uint2 w[(K1 + K2) * 2 * 32];                         // FP16 weights: [k-step][m-tile][lane], 4 per lane
+  float b1[kLsHid], b2[kLsHid], w3[kLsHid], b3;
+};
+
+// one hidden layer: o[m-tile] += W x over K k-steps; x(k) is this lane's element g, input k
+template <int K, typename X>
+__device__ __forceinline__ void ls_layer(const uint2 *w, int lane, X &&x, float (&o)[2][4]) {
+#pragma unroll
+  for (int kk = 0; kk < K; ++kk) {
+    const int j0 = 8 * kk + (lane & 3);
+    uint32_t bh[2], bl[2];
+    ls_tf32_split(x(j0), bh[0], bl[0]);
+    ls_tf32_split(x(j0 + 4), bh[1], bl[1]);
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt) {
+      const uint2 q = w[(kk * 2 + mt) * 32 + lane];
+      const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&q.x));
+      const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&q.y));
+      const uint32_t a[4] = {__float_as_uint(lo.x), __float_as_uint(lo.y), __float_as_uint(hi.x), __float_as_uint(hi.y)};
+      ls_mma_tf32(o[mt], a, bh);
+      ls_mma_tf32(o[mt], a, bl);
+    }
+  }
+}
+
+template <int N>
+__global__ void __launch_bounds__(32 * kLsWarps, 3) ls_sensor_kernel(const LsArgs A) {
+  using S = LsSensorSmem<N>;
+  constexpr int NP = S::NP, MT = S::MT, KT = S::KT, SU = S::SU, SX = S::SX, SH = S::SH, K1 = S::K1, K2 = S::K2;
   extern __shared__ __align__(16) unsigned char sm[];
-  double *sVi = reinterpret_cast<double *>(sm);     // [NP][NP]
-  double *su = sVi + NP * NP;                       // [64][NP]
-  float *sf = reinterpret_cast<float *>(su + kLsElems * NP);  // [64][NPP] features
-  float *sh = sf + kLsElems * NPP;                  // [64][32] first hidden layer
-  __half *sW = reinterpret_cast<__half *>(sh + kLsElems * kLsHid);
-  int *sTop = reinterpret_cast<int *>(sW + ((ls_mlp_params(NP) + 7) & ~7));
-  const int tid = threadIdx.x, e = tid >> 2, t = tid & 3;
-  for (int x = tid; x < NP * NP; x += blockDim.x) sVi[x] = A.Vinv[x];
-  for (int x = tid; x < NP; x += blockDim.x) sTop[x] = A.top[x];
-  if (A.mode >= 2)
-    for (int x = tid; x < ls_mlp_params(NP); x += blockDim.x) sW[x] = __ushort_as_half(A.mlp16[x]);
+  S &m = *reinterpret_cast<S *>(sm);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, c = lane & 3;
+  for (int i = tid; i < MT * KT * 32; i += blockDim.x) {
+    const int l = i & 31, kk = (i >> 5) % KT, mt = (i >> 5) / KT, r = 8 * mt + (l >> 2), j = 4 * kk + (l & 3);
+    m.vinv[i] = (r < NP && j < NP) ? A.Vinv[r * NP + j] : 0.0;
+  }
+  uint32_t topmask = 0;  // of this lane's rows, those of modes of total degree N
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+    if (8 * mt + g < NP && A.top[8 * mt + g]) topmask |= 1u << mt;
+  pdl_wait();
+  if (A.mode >= 2) {
+    // the network's parameters, rounded to FP16
+    const float *W1 = A.mlp, *B1 = W1 + kLsHid * NP, *W2 = B1 + kLsHid, *B2 = W2 + kLsHid * kLsHid, *W3 = B2 + kLsHid;
+    auto h16 = [](float v) { return __half2float(__float2half_rn(v)); };
+    for (int i = tid; i < (K1 + K2) * 2 * 32; i += blockDim.x) {
+      const int l = i & 31, mt = (i >> 5) & 1, kk = i >> 6;
+      const bool first = kk < K1;
+      const float *W = first ? W1 : W2;
+      const int nin = first ? NP : kLsHid, r = 16 * mt + (l >> 2), j = 8 * (first ? kk : kk - K1) + (l & 3);
+      auto at = [&](int rr, int jj) { return jj < nin ? W[rr * nin + jj] : 0.f; };
+      const __half2 lo = __floats2half2_rn(at(r, j), at(r + 8, j)), hi = __floats2half2_rn(at(r, j + 4), at(r + 8, j + 4));
+      m.w[i] = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+    }
+    if (tid < kLsHid) {
+      m.b1[tid] = h16(B1[tid]);
+      m.b2[tid] = h16(B2[tid]);
+      m.w3[tid] = h16(W3[tid]);
+    }
+    if (tid == 0) m.b3 = h16(W3[kLsHid]);
+  }
+  if (blockIdx.x == 0 && tid == 0) A.counts[1] = 0;  // the touched list of this stage is counted after this kernel
   __syncthreads();
-  const __half *W1 = sW, *b1 = W1 + kLsHid * NP, *W2 = b1 + kLsHid, *b2 = W2 + kLsHid * kLsHid, *w3 = b2 + kLsHid,
-               *b3 = w3 + kLsHid;
-  // Every warp walks its own groups of 8 elements (16 per 128-element tile) in rows 8 w .. 8 w + 7 of the
-  // block's buffers, with no block barrier; the state of its next group, the group's first element slot and
-  // (lanes 0..7) its elements' h / N are loaded into registers while the current one is computed.
-  const int lane = tid & 31, w0 = (tid >> 5) * 8, nw = blockDim.x >> 5;
-  const int ngroups = 16 * A.ntiles;
+  double *su = m.u[warp];
+  float *sx = m.x[warp], *sh = m.h[warp];
+  const int el = 2 * c + (g & 1);  // this lane's element
+  const int ngroups = 16 * A.ntiles, gstep = gridDim.x * kLsWarps;
   constexpr int FILL = (8 * NP + 31) / 32;  // values per lane
   float fh[FILL], fl[FILL];
   int64_t nslot = 0;
@@ -125,199 +185,127 @@ __global__ void __launch_bounds__(4 * kLsElems, 3) ls_sensor_kernel(const LsArgs
     }
     nslot = tl.elem_slot + e0;
     nne = ne;
-    nh = lane < ne ? A.h_over_n[nslot + lane] : 0.0;
+    nh = (g < 2 && el < ne) ? A.h_over_n[nslot + el] : 0.0;
   };
-  const int g0 = blockIdx.x * nw + (tid >> 5), gstep = gridDim.x * nw;
+  const int g0 = blockIdx.x * kLsWarps + warp;
   if (g0 < ngroups) load(g0);
   for (int gi = g0; gi < ngroups; gi += gstep) {
-    const int64_t slot0 = nslot;  // this group's first element slot, its element count and h / N (lanes 0..7)
+    const int64_t slot = nslot + el;
     const int ne = nne;
-    const double hg = nh;
+    const double hh = nh;
+    if (lane == 0 && gi + gstep >= ngroups) pdl_trigger();
 #pragma unroll
     for (int q = 0; q < FILL; ++q) {
-      const int x = lane + 32 * q;
-      if (x < 8 * NP) su[w0 * NP + x] = (double)fh[q] + (double)fl[q];
+      const int x = lane + 32 * q, e = x / NP;
+      if (x < 8 * NP) su[e * SU + x - e * NP] = (double)fh[q] + (double)fl[q];
     }
     __syncwarp();
     if (gi + gstep < ngroups) load(gi + gstep);
-    if (ne == 0) continue;  // past the tile's last element (warp-uniform)
-    const bool valid = (e & 7) < ne;
-    // modal coefficients uhat = Vinv u of this warp's 8 elements on the FP64 tensor path (mma.sync m8n8k4):
-    // A = Vinv (8-row m-tiles, 4-column k-steps), B = the elements' nodal values (one element per column);
-    // they overwrite the warp's own rows of su
-    {
-      constexpr int MT = (NP + 7) / 8, KT = (NP + 3) / 4;
-      const int ar = lane >> 2, ac = lane & 3, be = w0 + (lane >> 2);
-      double c[MT][2];
+    if (ne == 0) {
+      __syncwarp();
+      continue;  // past the tile's last element (warp-uniform)
+    }
+    // modal coefficients uhat = Vinv u of the 8 elements on the FP64 tensor path (mma.sync m8n8k4)
+    double uh[MT][2];
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) c[mt][0] = c[mt][1] = 0.0;
+    for (int mt = 0; mt < MT; ++mt) uh[mt][0] = uh[mt][1] = 0.0;
 #pragma unroll
-      for (int kk = 0; kk < KT; ++kk) {
-        const int j = 4 * kk + ac;
-        const double bv = (j < NP && ar < ne) ? su[be * NP + j] : 0.0;
+    for (int kk = 0; kk < KT; ++kk) {
+      const int j = 4 * kk + c;
+      const double bv = j < NP ? su[g * SU + j] : 0.0;
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          const int r = 8 * mt + ar;
-          const double av = (r < NP && j < NP) ? sVi[r * NP + j] : 0.0;
-          asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                       : "+d"(c[mt][0]), "+d"(c[mt][1])
-                       : "d"(av), "d"(bv));
-        }
+      for (int mt = 0; mt < MT; ++mt) ls_dmma(uh[mt][0], uh[mt][1], m.vinv[(mt * KT + kk) * 32 + lane], bv);
+    }
+    // energies: this lane's rows of elements 2c and 2c + 1, one of the two passed on in the first exchange
+    double tot[2] = {0.0, 0.0}, top[2] = {0.0, 0.0};
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        tot[h] = fma(uh[mt][h], uh[mt][h], tot[h]);
+        if ((topmask >> mt) & 1u) top[h] = fma(uh[mt][h], uh[mt][h], top[h]);
       }
-      __syncwarp();  // every lane's reads of the nodal values are done
+    const bool odd = g & 1;
+    double et = (odd ? tot[1] : tot[0]) + __shfl_xor_sync(0xffffffffu, odd ? tot[0] : tot[1], 4);
+    double en = (odd ? top[1] : top[0]) + __shfl_xor_sync(0xffffffffu, odd ? top[0] : top[1], 4);
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        const int r = 8 * mt + ar;
+    for (int x = 8; x <= 16; x <<= 1) {
+      et += __shfl_xor_sync(0xffffffffu, et, x);
+      en += __shfl_xor_sync(0xffffffffu, en, x);
+    }
+    double sig = 0.0;
+    if (A.mode != 0 && et > 0.0 && !(en < A.ratio0 * et)) sig = ls_pp_sigma(log10(en / et), A.s0, A.kappa);
+    if (A.mode >= 2) {
+      const double inv = et > 0.0 ? 1.0 / sqrt(et) : 0.0, other = __shfl_xor_sync(0xffffffffu, inv, 4);
+      const double iv[2] = {odd ? other : inv, odd ? inv : other};
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-          if (r < NP) su[(w0 + 2 * ac + h) * NP + r] = c[mt][h];
-      }
+          if (8 * mt + g < NP) sx[(2 * c + h) * SX + 8 * mt + g] = (float)(uh[mt][h] * iv[h]);
       __syncwarp();
-    }
-    const double *ue = su + (valid ? e : w0) * NP;  // now the element's modal coefficients
-    double tot = 0.0, top = 0.0;
-    double uh[(NP + 3) / 4];
+      // the network on the 8 elements with tensor products (mma.sync m16n8k8, TF32 operands, FP32 sums): every FP16
+      // weight is exact in TF32 and each FP32 input is split into two TF32 parts (hi + lo), so the products keep
+      // FP32-level rounding.  Rows are hidden units (two 16-row m-tiles), columns the warp's elements.
+      float o[2][4];
 #pragma unroll
-    for (int k = 0; k < (NP + 3) / 4; ++k) {
-      const int i = t + 4 * k;
-      double s = 0.0;
-      if (i < NP) {
-        s = ue[i];
-        tot = fma(s, s, tot);
-        if (sTop[i]) top = fma(s, s, top);
+      for (int mt = 0; mt < 2; ++mt) {
+        o[mt][0] = o[mt][1] = m.b1[16 * mt + g];
+        o[mt][2] = o[mt][3] = m.b1[16 * mt + g + 8];
       }
-      uh[k] = s;
-    }
-    tot += __shfl_xor_sync(0xffffffffu, tot, 1);
-    tot += __shfl_xor_sync(0xffffffffu, tot, 2);
-    top += __shfl_xor_sync(0xffffffffu, top, 1);
-    top += __shfl_xor_sync(0xffffffffu, top, 2);
-    const double S = tot > 0.0 ? log10(top / tot) : -INFINITY;
-    double sig = A.mode == 0 ? 0.0 : ls_pp_sigma(S, A.s0, A.kappa);
-    bool fallback = false;
-    if (A.mode >= 2) {
-      const double inv = tot > 0.0 ? 1.0 / sqrt(tot) : 0.0;
+      ls_layer<K1>(m.w, lane, [&](int j) { return j < NP ? sx[g * SX + j] : 0.f; }, o);
 #pragma unroll
-      for (int k = 0; k < (NP + 3) / 4; ++k) {
-        const int i = t + 4 * k;
-        if (i < NP) sf[e * NPP + i] = (float)(uh[k] * inv);
-      }
+      for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int f = 0; f < 4; ++f) sh[(2 * c + (f & 1)) * SH + 16 * mt + g + 8 * (f >> 1)] = tanhf(o[mt][f]);
       __syncwarp();
-      // the network on the warp's 8 elements with tensor products (mma.sync m16n8k8, TF32 operands, FP32
-      // sums): every FP16 weight is exact in TF32 and each FP32 input is split into two TF32 parts (hi + lo),
-      // so the products keep FP32-level rounding.  Rows are hidden units (two 16-row m-tiles), columns the
-      // warp's elements; lane (g = l / 4, c = l mod 4) holds units g, g + 8 (+16) of elements 2c, 2c + 1.
-      const int g = lane >> 2, c = lane & 3;
-      float o2[2][4];  // second-layer pre-activations: [m-tile][fragment]
-      {
-        float o1[2][4];
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-          const float blo = __half2float(b1[16 * mt + g]), bhi = __half2float(b1[16 * mt + g + 8]);
-          o1[mt][0] = o1[mt][1] = blo;
-          o1[mt][2] = o1[mt][3] = bhi;
-        }
-#pragma unroll
-        for (int kk = 0; kk < (NP + 7) / 8; ++kk) {
-          const int j0 = 8 * kk + c, j1 = j0 + 4;
-          const float x0 = j0 < NP ? sf[(w0 + g) * NPP + j0] : 0.f, x1 = j1 < NP ? sf[(w0 + g) * NPP + j1] : 0.f;
-          uint32_t bh[2], bl[2];
-          ls_tf32_split(x0, bh[0], bl[0]);
-          ls_tf32_split(x1, bh[1], bl[1]);
-#pragma unroll
-          for (int mt = 0; mt < 2; ++mt) {
-            const int r0 = 16 * mt + g;
-            const uint32_t a[4] = {ls_tf32_w(W1, r0 * NP + j0, j0 < NP), ls_tf32_w(W1, (r0 + 8) * NP + j0, j0 < NP),
-                                   ls_tf32_w(W1, r0 * NP + j1, j1 < NP), ls_tf32_w(W1, (r0 + 8) * NP + j1, j1 < NP)};
-            ls_mma_tf32(o1[mt], a, bh);
-            ls_mma_tf32(o1[mt], a, bl);
-          }
-        }
-        // first hidden layer -> shared memory [element][unit], the second layer's inputs
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-          for (int f = 0; f < 4; ++f)
-            sh[(w0 + 2 * c + (f & 1)) * kLsHid + 16 * mt + g + 8 * (f >> 1)] = tanhf(o1[mt][f]);
-        __syncwarp();
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-          const float blo = __half2float(b2[16 * mt + g]), bhi = __half2float(b2[16 * mt + g + 8]);
-          o2[mt][0] = o2[mt][1] = blo;
-          o2[mt][2] = o2[mt][3] = bhi;
-        }
-#pragma unroll
-        for (int kk = 0; kk < kLsHid / 8; ++kk) {
-          const int j0 = 8 * kk + c, j1 = j0 + 4;
-          uint32_t bh[2], bl[2];
-          ls_tf32_split(sh[(w0 + g) * kLsHid + j0], bh[0], bl[0]);
-          ls_tf32_split(sh[(w0 + g) * kLsHid + j1], bh[1], bl[1]);
-#pragma unroll
-          for (int mt = 0; mt < 2; ++mt) {
-            const int r0 = 16 * mt + g;
-            const uint32_t a[4] = {ls_tf32_w(W2, r0 * kLsHid + j0, true), ls_tf32_w(W2, (r0 + 8) * kLsHid + j0, true),
-                                   ls_tf32_w(W2, r0 * kLsHid + j1, true), ls_tf32_w(W2, (r0 + 8) * kLsHid + j1, true)};
-            ls_mma_tf32(o2[mt], a, bh);
-            ls_mma_tf32(o2[mt], a, bl);
-          }
-        }
+      for (int mt = 0; mt < 2; ++mt) {
+        o[mt][0] = o[mt][1] = m.b2[16 * mt + g];
+        o[mt][2] = o[mt][3] = m.b2[16 * mt + g + 8];
       }
-      // output unit: this lane's four units for elements 2c and 2c + 1, summed over the lanes of the same c
+      ls_layer<K2>(m.w + K1 * 2 * 32, lane, [&](int j) { return sh[g * SH + j]; }, o);
+      // output unit: this lane's four units of elements 2c and 2c + 1, summed over the lanes of the same c
       float za = 0.f, zb = 0.f;
 #pragma unroll
       for (int mt = 0; mt < 2; ++mt) {
-        const float wlo = __half2float(w3[16 * mt + g]), whi = __half2float(w3[16 * mt + g + 8]);
-        za += wlo * tanhf(o2[mt][0]) + whi * tanhf(o2[mt][2]);
-        zb += wlo * tanhf(o2[mt][1]) + whi * tanhf(o2[mt][3]);
+        const float wlo = m.w3[16 * mt + g], whi = m.w3[16 * mt + g + 8];
+        za += wlo * tanhf(o[mt][0]) + whi * tanhf(o[mt][2]);
+        zb += wlo * tanhf(o[mt][1]) + whi * tanhf(o[mt][3]);
       }
 #pragma unroll
-      for (int m = 4; m <= 16; m <<= 1) {
-        za += __shfl_xor_sync(0xffffffffu, za, m);
-        zb += __shfl_xor_sync(0xffffffffu, zb, m);
+      for (int x = 4; x <= 16; x <<= 1) {
+        za += __shfl_xor_sync(0xffffffffu, za, x);
+        zb += __shfl_xor_sync(0xffffffffu, zb, x);
       }
-      const int el = e & 7;  // this thread's element: held by lane el / 2 (c = el / 2, g = 0)
-      const float zsa = __shfl_sync(0xffffffffu, za, el >> 1), zsb = __shfl_sync(0xffffffffu, zb, el >> 1);
-      const float z = (el & 1) ? zsb : zsa;
-      const float sg = 1.f / (1.f + expf(-(z + __half2float(b3[0]))));
-      if (sg > A.conf_lo && sg < A.conf_hi) {
-        fallback = true;  // low confidence: the PP activation stands
-      } else {
-        sig = (A.mode == 3 && sg <= A.conf_lo) ? 0.0 : (double)sg;
-      }
+      const float sg = 1.f / (1.f + expf(-((odd ? zb : za) + m.b3)));
+      // inside the low-confidence band the PP activation stands
+      if (!(sg > A.conf_lo && sg < A.conf_hi)) sig = (A.mode == 3 && sg <= A.conf_lo) ? 0.0 : (double)sg;
     }
-    const double hh = __shfl_sync(0xffffffffu, hg, e & 7);  // this element's h / N
-    if (valid && t == 0) {
-      const int64_t slot = slot0 + (e & 7);
+    if (g < 2 && el < ne) {
       const double eps = A.eps0 * sig * hh;
       A.eps[slot] = eps;
       int a = -1;
       if (eps > 0.0) {
         a = atomicAdd(&A.counts[0], 1);
         A.alist[a] = (int32_t)slot;
+        A.tflag[slot] = 1;
+        for (int f = 0; f < 4; ++f) {
+          int node;
+          const int64_t ns = slot_of_value(A, (int64_t)(uint32_t)A.conn[slot * kMixedConnWords + f], NP, &node);
+          if (ns >= 0) A.tflag[ns] = 1;
+        }
       }
       A.aslot[slot] = a;
-      if (fallback) atomicAdd(&A.counts[2], 1);
     }
     __syncwarp();  // the warp's rows are free for its next group
   }
 }
 
-// the active elements and their face neighbours
-__global__ void ls_touch_kernel(const LsArgs A, int np) {
-  const int n = *reinterpret_cast<volatile const int *>(&A.counts[0]);
-  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-    const int64_t slot = A.alist[a];
-    A.tflag[slot] = 1;
-    for (int f = 0; f < 4; ++f) {
-      int node;
-      const int64_t ns = slot_of_value(A, (int64_t)(uint32_t)A.conn[slot * kMixedConnWords + f], np, &node);
-      if (ns >= 0) A.tflag[ns] = 1;
-    }
-  }
-}
-
 // touched list and row of every slot (-1 elsewhere); the flags are cleared for the next stage
 __global__ void ls_compact_kernel(const LsArgs A) {
+  pdl_wait();
+  pdl_trigger();
   for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < A.nslots; s += (int64_t)gridDim.x * blockDim.x) {
     if (A.tflag[s]) {
       const int r = atomicAdd(&A.counts[1], 1);
@@ -337,12 +325,6 @@ __global__ void ls_compact_kernel(const LsArgs A) {
 // the few tens of KB stay there); lane l's output row is 8 mt + l / 4, its elements 2 (l mod 4) and
 // 2 (l mod 4) + 1.  The mixed stage requires straight-sided elements, so the metrics are constant over an
 // element and are read once per element.
-__device__ __forceinline__ void ls_dmma(double &c0, double &c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
-}
-
 template <int N>
 struct LsCfg {
   using O = Order<N>;
@@ -396,6 +378,8 @@ __global__ void __launch_bounds__(LsCfg<N>::THREADS) ls_grad_kernel(const LsArgs
   __shared__ LsElem se[8];
   const int tid = threadIdx.x, lane = tid & 31, mt = tid >> 5;
   const int ar = lane >> 2, ac = lane & 3, r = 8 * mt + ar;
+  pdl_wait();
+  pdl_trigger();
   const int n = *reinterpret_cast<volatile const int *>(&A.counts[0]);
   const int ngroups = (n + 7) / 8;
   for (int gi = blockIdx.x; gi < ngroups; gi += gridDim.x) {
@@ -485,7 +469,10 @@ __global__ void __launch_bounds__(LsCfg<N>::THREADS) ls_div_kernel(const LsArgs 
   __shared__ LsElem se[8];
   const int tid = threadIdx.x, lane = tid & 31, mt = tid >> 5;
   const int ar = lane >> 2, ac = lane & 3, r = 8 * mt + ar;
+  pdl_wait();
+  pdl_trigger();
   const int n = *reinterpret_cast<volatile const int *>(&A.counts[1]);
+  if (blockIdx.x == 0 && tid == 0) A.counts[0] = 0;  // the next stage's sensor pass counts from zero
   const int ngroups = (n + 7) / 8;
   for (int gi = blockIdx.x; gi < ngroups; gi += gridDim.x) {
     ls_stage_elems<N>(A, A.tlist, n, gi, se, true);
@@ -586,20 +573,13 @@ __global__ void __launch_bounds__(LsCfg<N>::THREADS) ls_div_kernel(const LsArgs 
 }
 
 template <int N>
-size_t ls_sensor_smem() {
-  constexpr int NP = Order<N>::NP;
-  return sizeof(double) * (NP * NP + kLsElems * NP) + sizeof(float) * (kLsElems * (NP + 1) + kLsElems * kLsHid) +
-         sizeof(__half) * ((ls_mlp_params(NP) + 7) & ~7) + sizeof(int) * NP;
-}
-
-template <int N>
 void ls_attrs() {
   static bool done[64] = {};
   int dev = 0;
   cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
   if (dev >= 0 && dev < 64 && done[dev]) return;
   cuda_check(cudaFuncSetAttribute(ls_sensor_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)ls_sensor_smem<N>()),
+                                  (int)sizeof(LsSensorSmem<N>)),
              "ls_sensor smem");
   if (dev >= 0 && dev < 64) done[dev] = true;
 }
@@ -607,18 +587,11 @@ void ls_attrs() {
 template <int N>
 void launch_ls_n(const LsArgs &A, int num_sms, cudaStream_t st) {
   ls_attrs<N>();
-  cuda_check(cudaMemsetAsync(A.counts, 0, 3 * sizeof(int32_t), st), "reset counts");
-  const int gs = std::max(1, std::min(2 * A.ntiles, num_sms * 8));
-  ls_sensor_kernel<N><<<gs, 4 * kLsElems, ls_sensor_smem<N>(), st>>>(A);
-  cuda_check(cudaGetLastError(), "ls_sensor_kernel launch");
-  ls_touch_kernel<<<num_sms * 2, 256, 0, st>>>(A, Order<N>::NP);
-  cuda_check(cudaGetLastError(), "ls_touch_kernel launch");
-  ls_compact_kernel<<<num_sms * 4, 256, 0, st>>>(A);
-  cuda_check(cudaGetLastError(), "ls_compact_kernel launch");
-  ls_grad_kernel<N><<<num_sms * 8, LsCfg<N>::THREADS, 0, st>>>(A);
-  cuda_check(cudaGetLastError(), "ls_grad_kernel launch");
-  ls_div_kernel<N><<<num_sms * 8, LsCfg<N>::THREADS, 0, st>>>(A);
-  cuda_check(cudaGetLastError(), "ls_div_kernel launch");
+  const int gs = std::max(1, std::min(2 * A.ntiles, num_sms * 3));
+  launch_pdl(ls_sensor_kernel<N>, gs, 32 * kLsWarps, sizeof(LsSensorSmem<N>), st, A);
+  launch_pdl(ls_compact_kernel, num_sms * 4, 256, 0, st, A);
+  launch_pdl(ls_grad_kernel<N>, num_sms * 8, LsCfg<N>::THREADS, 0, st, A);
+  launch_pdl(ls_div_kernel<N>, num_sms * 8, LsCfg<N>::THREADS, 0, st, A);
 }
 
 }  // namespace

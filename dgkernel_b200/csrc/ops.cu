@@ -501,7 +501,7 @@ struct MixedOp : Op {
   float conf_lo = 0.1f, conf_hi = 0.9f;
   int64_t l_nslots = 0;
   Binding *geoB[9] = {}, *faceB[4] = {}, *gmapB = nullptr, *mlpB = nullptr;
-  DevBuf l_dr, l_ds, l_dt, l_vinv, l_lift, l_top, l_hon, l_mlp16, l_sp, l_kp, l_uo, l_go, l_fo, l_eps, l_aslot, l_alist,
+  DevBuf l_dr, l_ds, l_dt, l_vinv, l_lift, l_top, l_hon, l_sp, l_kp, l_uo, l_go, l_fo, l_eps, l_aslot, l_alist,
       l_tflag, l_vslot, l_tlist, l_counts, l_eq, l_visc;
   LaunchInfo info;
 
@@ -737,7 +737,6 @@ struct MixedOp : Op {
         mlpB = R.matrix("MLP");
         require(mlpB->rows * mlpB->cols == mlp_param_count((int)np) && mlpB->dev_dtype == DGK_FLOAT32,
                 R.kname + ": MLP must hold " + std::to_string(mlp_param_count((int)np)) + " float32 parameters");
-        l_mlp16.alloc(sizeof(uint16_t) * ((size_t)mlp_param_count((int)np) + 8));
       }
       std::vector<int32_t> tp;
       for (int i = 0; i <= N; ++i)  // modes ordered i, j, k (vandermonde3d.go:15-42)
@@ -772,7 +771,8 @@ struct MixedOp : Op {
       l_tflag.upload(zero.data(), ns * sizeof(int32_t));
       l_alist.alloc(ns * sizeof(int32_t));
       l_tlist.alloc(ns * sizeof(int32_t));
-      l_counts.alloc(4 * sizeof(int32_t));
+      const int32_t none[4] = {};
+      l_counts.upload(none, sizeof(none));
       l_eq.alloc(ns * 3 * (size_t)np * sizeof(double));  // capacity: every element active
       l_visc.alloc(ns * (size_t)np * sizeof(double));
     }
@@ -810,10 +810,8 @@ struct MixedOp : Op {
     L.kappa = kappa;
     L.conf_lo = conf_lo;
     L.conf_hi = conf_hi;
-    if (lmode >= 2) {
-      launch_to_half(reinterpret_cast<const float *>(mlpB->dptr), l_mlp16.p, mlp_param_count((N + 1) * (N + 2) * (N + 3) / 6), r.stream());
-      L.mlp16 = l_mlp16.get<unsigned short>();
-    }
+    L.ratio0 = std::pow(10.0, s0 - kappa) * (1.0 - 1e-9);
+    L.mlp = lmode >= 2 ? reinterpret_cast<const float *>(mlpB->dptr) : nullptr;
     L.eps = l_eps.get<double>();
     L.aslot = l_aslot.get<int32_t>();
     L.alist = l_alist.get<int32_t>();
