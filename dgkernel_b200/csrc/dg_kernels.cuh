@@ -182,7 +182,7 @@ struct OzArgs {
   const int32_t *conn;          // kMixedConnWords per element slot
   int64_t n_u_values;           // bound of every gathered value index
   const unsigned char *amat;    // matrix digits in 4 KB chunks, digit-major (oz_pack_operands)
-  const int32_t *rexp;          // [2][128]: row exponents of the volume and LIFT rows
+  const int32_t *rexp;          // [2][128]: row exponents of the volume and LIFT rows; [2][6][128]: 128 x digit sums
   const double *bary;           // [NP][3]
   const int32_t *vtx;           // vertex nodes A..D
   const uint8_t *ftab;          // [ncodes][Nfp]

@@ -70,16 +70,23 @@ struct OzCfg {
   static constexpr int NP = O::NP, NFP = O::NFP, NF = O::NF;
   static constexpr int KD = rup32(NP), KV = 3 * KD, KL = rup32(NF), KT = KV + KL;
   static constexpr int CV = KV / 32, CT = KT / 32;       // 32-wide K chunks: volume, all
-  static constexpr int XV = KD / 16, XL = KL / 16;       // 16-wide value groups: per volume direction, LIFT
-  static constexpr int NX = XV + XL;                     // groups per element (a volume group feeds 3 directions)
-  static constexpr int GPT = (NX + 15) / 16;             // groups per thread (16 threads per element)
-  static constexpr uint32_t BCH = 1024;                  // bytes of one element-digit chunk: 32 rows x 32 K
-  static constexpr uint32_t BSLICE = (uint32_t)CT * BCH; // one digit of the tile's element operand
+  // 16-wide value groups that hold values: per volume direction, LIFT; the operand's padding beyond them stays
+  // unwritten (the matrices' digits are zero there)
+  static constexpr int XW = (NP + 15) / 16, XF = (NF + 15) / 16;
+  static constexpr int NY = 3 * XW + XF;                 // digit groups per element, 16 threads per element
+  static_assert(NY <= 33, "two groups per thread, and one more per element at most");
+  // FP64 scratch for the values (in the operand's place until its digits are written): group x of element e at
+  // e STR + 17 x, STR = 2 mod 16, which spreads a half warp's 8 elements x 2 groups over the banks
+  static constexpr int STW = (17 * XW + 13) / 16 * 16 + 2, STF = (17 * XF + 13) / 16 * 16 + 2;
+  static_assert(STW >= 17 * XW && STF >= 17 * XF, "scratch rows");
+  static constexpr uint32_t BK = (uint32_t)S * 512;      // a 16-wide K half of the element operand: S digits x 32 rows
+  static constexpr uint32_t BCH = 2 * BK;                // one 32-wide K chunk: rows q 32 + e for digit q of element e
+  static_assert((uint32_t)kOzTE * (STW + STF + 4) * 8 <= CT * BCH, "the scratch fits the operand");
   static constexpr uint32_t NODE_B = (uint32_t)kOzTE * NP * 4;
   static constexpr uint32_t SLOT_B = 2 * NODE_B + kOzTE * kMixedGeoWords * 4 + round16(kOzTE * kMixedConnWords * 4);
   // shared memory (bytes)
   static constexpr uint32_t OFF_B = 0;
-  static constexpr uint32_t OFF_RING = OFF_B + S * BSLICE;
+  static constexpr uint32_t OFF_RING = OFF_B + CT * BCH;
   static constexpr uint32_t OFF_SLOT = OFF_RING + kOzRing * kOzChunk;
   static constexpr uint32_t OFF_BARY = OFF_SLOT + kOzSlots * SLOT_B;
   static constexpr uint32_t OFF_L0 = OFF_BARY + NP * 3 * 8;               // double per element, 2 tile buffers
@@ -108,8 +115,10 @@ __device__ __forceinline__ double pow2(int e) {
 // Exponent E with |x| < 2^E for the largest |x| of a row (0 for an all-zero row): frexp's exponent.
 __device__ __forceinline__ int row_exp(double amax) {
   if (!(amax > 0.0)) return -1100;  // all zero: every digit is zero whatever the scale
+  const int b = (int)(__double_as_longlong(amax) >> 52);  // biased exponent of a positive value
+  if (b > 0) return b - 1022;
   int e;
-  frexp(amax, &e);
+  frexp(amax, &e);  // subnormal
   return e;
 }
 
@@ -123,7 +132,7 @@ __device__ __forceinline__ void tc_mma_i8(uint32_t tmem, uint64_t da, uint64_t d
 // Digits of 16 values of a row with exponent E: each value rounded once to the integer n = rint(x 2^(B-E)),
 // B = 7 + 8 (S - 1) (|n| <= 2^B; clamped to 2^B - 1 at the top), then cut by arithmetic shifts, which is exact:
 // digit 0 = n >> (B - 7) in [-128, 127] (s8), digit p > 0 = the byte (n >> 8 (S - 1 - p)) & 255 (u8).  `scale`
-// is 2^(B-E).  Digit p of value v goes to byte v of out[p].
+// is 2^(B-E).  Digit p of value v goes to byte v of out[p]; digit 0 goes as d + 128, so that every byte is unsigned.
 template <int S>
 __device__ __forceinline__ void digits16(const double (&x)[16], double scale, uint4 (&out)[S]) {
   constexpr int B = 7 + 8 * (S - 1);
@@ -142,6 +151,21 @@ __device__ __forceinline__ void digits16(const double (&x)[16], double scale, ui
   }
 #pragma unroll
   for (int p = 0; p < S; ++p) out[p] = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+  out[0].x ^= 0x80808080u;
+  out[0].y ^= 0x80808080u;
+  out[0].z ^= 0x80808080u;
+  out[0].w ^= 0x80808080u;
+}
+
+// max of ex over the warp's lanes of each element (consecutive lanes: one element or two) into rows[element]
+__device__ __forceinline__ void oz_row_max(int *rows, int e, int ex, int lane) {
+  const int e0 = __shfl_sync(0xffffffffu, e, 0), e1 = __shfl_sync(0xffffffffu, e, 31);
+  const int m0 = __reduce_max_sync(0xffffffffu, e == e0 ? ex : -1100);
+  if (lane == 0 && m0 > -1100) atomicMax(&rows[e0], m0);
+  if (e1 != e0) {
+    const int m1 = __reduce_max_sync(0xffffffffu, e == e1 ? ex : -1100);
+    if (lane == 0 && m1 > -1100) atomicMax(&rows[e1], m1);
+  }
 }
 
 // 8 consecutive TMEM columns (int32) of this warp's 32 lanes starting at taddr; waits for the load.
@@ -185,7 +209,7 @@ template <int N, int S, bool CONS>
 __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const OzArgs A) {
   using C = OzCfg<N, S>;
   constexpr int NP = C::NP, NFP = C::NFP, NF = C::NF, KD = C::KD, KV = C::KV, CV = C::CV, CT = C::CT;
-  constexpr int XV = C::XV, NX = C::NX, GPT = C::GPT;
+  constexpr int XW = C::XW, XF = C::XF, NY = C::NY, STW = C::STW, STF = C::STF;
   constexpr int TE = kOzTE, NTH = 32 * kOzCW;
   extern __shared__ __align__(1024) unsigned char sm[];
   unsigned char *sB = sm + C::OFF_B, *ring = sm + C::OFF_RING, *slots = sm + C::OFF_SLOT;
@@ -326,9 +350,9 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
   bool failed = false;
   if (warp == kOzCW) {
     // MMA warp: tile k's element digits ready (bful) and tile k-1's accumulators read (tfree) -> for every
-    // matrix chunk (p, c) from the ring, lane 0 issues the MMAs with element digits q <= S-1-p into level p + q
-    constexpr uint32_t M = 128, NN = TE;
-    const uint32_t idesc_base = (2u << 4) | ((NN >> 3) << 17) | ((M >> 4) << 24);  // S32 accumulate, K-major
+    // matrix chunk (p, c) from the ring, lane 0 issues one MMA with the element digits q <= S-1-p into levels p + q
+    constexpr uint32_t M = 128;
+    const uint32_t idesc_base = (2u << 4) | ((M >> 4) << 24);  // S32 accumulate, K-major, unsigned digits
     int64_t g = 0;
     int k = 0, kc = -1;
     for (;; ++k) {
@@ -351,15 +375,11 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
           if (lane == 0) {
             const uint64_t da = smem_desc(saddr(ring + (size_t)rs * kOzChunk), 2048, 128);
             const int acc = c < CV ? 0 : 1;
-#pragma unroll
-            for (int q = 0; q < S; ++q) {
-              if (p + q < S) {
-                const uint64_t db = smem_desc(saddr(sB + (size_t)q * C::BSLICE + (size_t)c * C::BCH), 512, 128);
-                const uint32_t idesc = idesc_base | ((p == 0 ? 1u : 0u) << 7) | ((q == 0 ? 1u : 0u) << 10);
-                const uint32_t col = (uint32_t)(((p + q) * 2 + acc) * TE);
-                tc_mma_i8(tmem + col, da, db, idesc, (p == 0 && (c == 0 || c == CV)) ? 0u : 1u);
-              }
-            }
+            const uint64_t db = smem_desc(saddr(sB + (size_t)c * C::BCH), C::BK, 128);
+            // digits q = 0 .. S-1-p side by side: columns of levels p .. S-1, which lie side by side too
+            const uint32_t idesc = idesc_base | ((p == 0 ? 1u : 0u) << 7) | ((uint32_t)((S - p) * TE >> 3) << 17);
+            const uint32_t col = (uint32_t)((acc * S + p) * TE);
+            tc_mma_i8(tmem + col, da, db, idesc, (p == 0 && (c == 0 || c == CV)) ? 0u : 1u);
             tc_commit(&aemp[rs]);  // the ring slot is free once these MMAs have read it
           }
           __syncwarp();
@@ -419,126 +439,137 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
       const float *sLo = sHi + TE * NP;
       const float *sGeo = sLo + TE * NP;
       const int *sCon = reinterpret_cast<const int *>(sGeo + TE * kMixedGeoWords);
-      const int64_t slot0 = tl.node_base, slotn = (int64_t)ne * NP;
+      const int64_t slot0 = tl.node_base;
 
-      // ---- element digits: values of this thread's groups, row maxima, digits ----
-      const bool valid = eb < ne;
-      const int ee = valid ? eb : 0;
-      const float *hi = sHi + ee * NP;
-      const float *lo = sLo + ee * NP;
-      const float4 g0 = *reinterpret_cast<const float4 *>(sGeo + ee * kMixedGeoWords);
-      const float4 g1 = *reinterpret_cast<const float4 *>(sGeo + ee * kMixedGeoWords + 4);
-      const double cd[3] = {(double)g0.x, (double)g0.y, (double)g0.z};
+      // ---- values, in FP64, into the scratch ----
       // element arithmetic in FP64 without contraction (dmul/dadd): every rounding is the restatement's, so the
       // digits, which feed an ill-conditioned product at high order, match it exactly
-      const double uA = (double)hi[vA] + (double)lo[vA], uB = (double)hi[vB] + (double)lo[vB];
-      const double uC = (double)hi[vC] + (double)lo[vC], uD = (double)hi[vD] + (double)lo[vD];
-      const double wA = CONS ? __dmul_rn(0.5 * uA, uA) : uA;
-      const double dB = (CONS ? __dmul_rn(0.5 * uB, uB) : uB) - wA;
-      const double dC = (CONS ? __dmul_rn(0.5 * uC, uC) : uC) - wA;
-      const double dD = (CONS ? __dmul_rn(0.5 * uD, uD) : uD) - wA;
-      if (valid && xg == 0)
-        sL0[eb] = 0.5 * __dadd_rn(__dadd_rn(__dmul_rn(cd[0], dB), __dmul_rn(cd[1], dC)), __dmul_rn(cd[2], dD));
-      double val[GPT][16];
-      double mv = 0.0, ml = 0.0;
-      bool badg = false;
-      const uint32_t codes = (uint32_t)sCon[ee * kMixedConnWords + 4];
+      double *sW = reinterpret_cast<double *>(sB), *sF = sW + TE * STW, *sVx = sF + TE * STF;
+      // the Lax-Friedrichs flux: consecutive threads take consecutive points of an element, so that a warp's gathers
+      // fall into a few elements' rows; all gathers first, then the math
+      {
+        float pH[XF], pL[XF];
+        bool badg = false;
 #pragma unroll
-      for (int gi = 0; gi < GPT; ++gi) {
-        const int x = xg + 16 * gi;
-#pragma unroll
-        for (int v = 0; v < 16; ++v) val[gi][v] = 0.0;
-        if (!valid || x >= NX) continue;
-        if (x < XV) {  // dw at nodes 16 x .. 16 x + 15
-#pragma unroll
-          for (int v = 0; v < 16; ++v) {
-            const int j = 16 * x + v;
-            if (j < NP) {
-              const double uj = (double)hi[j] + (double)lo[j];
-              const double wj = CONS ? __dmul_rn(0.5 * uj, uj) : uj;
-              const double lin = __dadd_rn(__dadd_rn(__dmul_rn(sBary[3 * j], dB), __dmul_rn(sBary[3 * j + 1], dC)),
-                                           __dmul_rn(sBary[3 * j + 2], dD));
-              const double dw = (wj - wA) - lin;
-              val[gi][v] = dw;
-              mv = fmax(mv, fabs(dw));
-            }
-          }
-        } else {  // the Lax-Friedrichs flux at face points 16 (x - XV) ..: all gathers first, then the math
-          float pH[16], pL[16];
-#pragma unroll
-          for (int v = 0; v < 16; ++v) {
-            const int m = 16 * (x - XV) + v;
-            pH[v] = 0.f;
-            pL[v] = 0.f;
-            if (m < NF) {
-              const int f = sPt[NF + m], pp = m - f * NFP;
-              const uint32_t nbs = (uint32_t)sCon[ee * kMixedConnWords + f];
-              const int cdx = min((int)((codes >> (8 * f)) & 0xffu), ncodes - 1);
-              const uint32_t idx = nbs + sFt[cdx * 64 + pp];
-              if (idx < n_u32) {
-                pH[v] = __ldg(A.uhi_in + idx);
-                pL[v] = __ldg(A.ulo_in + idx);
-              } else {  // out of range: reported, and the point takes its own trace (zero jump)
-                badg = true;
-                pH[v] = hi[sPt[m]];
-                pL[v] = lo[sPt[m]];
-              }
-            }
-          }
-#pragma unroll
-          for (int v = 0; v < 16; ++v) {
-            const int m = 16 * (x - XV) + v;
-            if (m < NF) {
-              const int f = sPt[NF + m], own = sPt[m];
-              const double uM = (double)hi[own] + (double)lo[own];
-              const double uP = (double)pH[v] + (double)pL[v];
-              const float gf = f == 0 ? g0.w : f == 1 ? g1.x : f == 2 ? g1.y : g1.z;
-              const double gg = (double)gf, d = uM - uP;
-              const double fl = __dmul_rn(0.5 * d, __dsub_rn(__dmul_rn(0.5 * (uM + uP), gg),
-                                                            __dmul_rn(fmax(fabs(uM), fabs(uP)), fabs(gg))));
-              val[gi][v] = fl;
-              ml = fmax(ml, fabs(fl));
+        for (int i = 0; i < XF; ++i) {
+          const int x = tid + i * NTH, e = x / (16 * XF), m = x - e * (16 * XF);
+          pH[i] = 0.f;
+          pL[i] = 0.f;
+          if (e < ne && m < NF) {
+            const int f = sPt[NF + m], pp = m - f * NFP;
+            const uint32_t nbs = (uint32_t)sCon[e * kMixedConnWords + f];
+            const uint32_t codes = (uint32_t)sCon[e * kMixedConnWords + 4];
+            const int cdx = min((int)((codes >> (8 * f)) & 0xffu), ncodes - 1);
+            const uint32_t idx = nbs + sFt[cdx * 64 + pp];
+            if (idx < n_u32) {
+              pH[i] = __ldg(A.uhi_in + idx);
+              pL[i] = __ldg(A.ulo_in + idx);
+            } else {  // out of range: reported, and the point takes its own trace (zero jump)
+              badg = true;
+              pH[i] = sHi[e * NP + sPt[m]];
+              pL[i] = sLo[e * NP + sPt[m]];
             }
           }
         }
-      }
-      if (badg) atomicExch(A.status, kStatusBadGather);
-      if (valid) {
-        const double cmax = fmax(fabs(cd[0]), fmax(fabs(cd[1]), fabs(cd[2])));
-        if (mv > 0.0) atomicMax(&sEv[eb], row_exp(cmax * mv));
-        if (ml > 0.0) atomicMax(&sEl[eb], row_exp(ml));
+        if (badg) atomicExch(A.status, kStatusBadGather);
+        if (tid < ne) {  // an element's vertex values and the derivative of its linear part
+          const float *hi = sHi + tid * NP, *lo = sLo + tid * NP, *ge = sGeo + tid * kMixedGeoWords;
+          const double uA = (double)hi[vA] + (double)lo[vA], uB = (double)hi[vB] + (double)lo[vB];
+          const double uC = (double)hi[vC] + (double)lo[vC], uD = (double)hi[vD] + (double)lo[vD];
+          const double wA = CONS ? __dmul_rn(0.5 * uA, uA) : uA;
+          const double dB = (CONS ? __dmul_rn(0.5 * uB, uB) : uB) - wA;
+          const double dC = (CONS ? __dmul_rn(0.5 * uC, uC) : uC) - wA;
+          const double dD = (CONS ? __dmul_rn(0.5 * uD, uD) : uD) - wA;
+          sVx[4 * tid] = wA;
+          sVx[4 * tid + 1] = dB;
+          sVx[4 * tid + 2] = dC;
+          sVx[4 * tid + 3] = dD;
+          sL0[tid] = 0.5 * __dadd_rn(__dadd_rn(__dmul_rn((double)ge[0], dB), __dmul_rn((double)ge[1], dC)),
+                                     __dmul_rn((double)ge[2], dD));
+        }
+#pragma unroll
+        for (int i = 0; i < XF; ++i) {
+          const int x = tid + i * NTH, e = x / (16 * XF), m = x - e * (16 * XF);
+          double fl = 0.0;
+          if (e < ne && m < NF) {
+            const int f = sPt[NF + m], own = sPt[m];
+            const double uM = (double)sHi[e * NP + own] + (double)sLo[e * NP + own];
+            const double uP = (double)pH[i] + (double)pL[i];
+            const double gg = (double)sGeo[e * kMixedGeoWords + 3 + f], d = uM - uP;
+            fl = __dmul_rn(0.5 * d, __dsub_rn(__dmul_rn(0.5 * (uM + uP), gg),
+                                              __dmul_rn(fmax(fabs(uM), fabs(uP)), fabs(gg))));
+          }
+          sF[e * STF + 17 * (m >> 4) + (m & 15)] = fl;
+          oz_row_max(sEl, e, row_exp(fabs(fl)), lane);
+        }
       }
       asm volatile("bar.sync 1, %0;" ::"n"(NTH) : "memory");
+#pragma unroll
+      for (int i = 0; i < XW; ++i) {  // dw = w minus its linear vertex interpolant
+        const int x = tid + i * NTH, e = x / (16 * XW), j = x - e * (16 * XW);
+        double dw = 0.0, cmax = 0.0;
+        if (e < ne && j < NP) {
+          const double uj = (double)sHi[e * NP + j] + (double)sLo[e * NP + j];
+          const double wj = CONS ? __dmul_rn(0.5 * uj, uj) : uj;
+          const double lin = __dadd_rn(__dadd_rn(__dmul_rn(sBary[3 * j], sVx[4 * e + 1]),
+                                                 __dmul_rn(sBary[3 * j + 1], sVx[4 * e + 2])),
+                                       __dmul_rn(sBary[3 * j + 2], sVx[4 * e + 3]));
+          dw = (wj - sVx[4 * e]) - lin;
+          const float *ge = sGeo + e * kMixedGeoWords;
+          cmax = (double)fmaxf(fabsf(ge[0]), fmaxf(fabsf(ge[1]), fabsf(ge[2])));
+        }
+        sW[e * STW + 17 * (j >> 4) + (j & 15)] = dw;
+        oz_row_max(sEv, e, row_exp(cmax * fabs(dw)), lane);
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(NTH) : "memory");
+      // ---- digits: thread group xg of element eb takes digit groups xg, xg + 16 (and 32) of the element: direction
+      // d, values 16 x .. of dw, scaled by c_d; or values 16 x .. of the flux ----
+      const bool valid = eb < ne;
+      const int ee = valid ? eb : 0;
+      double cd[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) cd[d] = (double)sGeo[ee * kMixedGeoWords + d];
+      constexpr int BITS = 7 + 8 * (S - 1);
+      const double sv = pow2(BITS - sEv[ee]), sl = pow2(BITS - sEl[ee]);
+      constexpr int GPT = NY < 32 ? (NY + 15) / 16 : 2;
+      // digit group y: kind d (0..2 volume directions, 3 the flux) and its group x; K index d KD + 16 x
+      auto kind = [](int y) { return (y >= XW) + (y >= 2 * XW) + (y >= 3 * XW); };
+      auto src = [&](int y) {
+        const int d = kind(y), x = y - d * XW;
+        return (d < 3 ? sW + ee * STW : sF + ee * STF) + 17 * x;
+      };
+      auto emit = [&](const double (&v)[16], int y) {
+        double z[16];
+        const int d = kind(y), kk = d * KD + 16 * (y - d * XW);
+        const double c = d == 0 ? cd[0] : d == 1 ? cd[1] : d == 2 ? cd[2] : 1.0;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) z[q] = c * v[q];
+        uint4 dg[S];
+        digits16<S>(z, d < 3 ? sv : sl, dg);
+        unsigned char *o = sB + (size_t)(kk >> 5) * C::BCH + (size_t)((kk >> 4) & 1) * C::BK + (eb >> 3) * 128 +
+                           (eb & 7) * 16;
+#pragma unroll
+        for (int p = 0; p < S; ++p) *reinterpret_cast<uint4 *>(o + p * 512) = dg[p];
+      };
+      double val[GPT][16];
+#pragma unroll
+      for (int gi = 0; gi < GPT; ++gi)
+#pragma unroll
+        for (int v = 0; v < 16; ++v) val[gi][v] = xg + 16 * gi < NY ? src(xg + 16 * gi)[v] : 0.0;
+      double *over = reinterpret_cast<double *>(slots + (size_t)s * C::SLOT_B) + eb * 17;  // the state is read by now
+      if (NY > 32 && xg == 0)
+#pragma unroll
+        for (int v = 0; v < 16; ++v) over[v] = src(32)[v];
+      asm volatile("bar.sync 1, %0;" ::"n"(NTH) : "memory");  // the scratch is read: the digits take its place
       if (valid) {
-        constexpr int BITS = 7 + 8 * (S - 1);
-        const double sv = pow2(BITS - sEv[eb]), sl = pow2(BITS - sEl[eb]);
 #pragma unroll
-        for (int gi = 0; gi < GPT; ++gi) {
-          const int x = xg + 16 * gi;
-          if (x >= NX) continue;
-          if (x < XV) {
+        for (int gi = 0; gi < GPT; ++gi)
+          if (xg + 16 * gi < NY) emit(val[gi], xg + 16 * gi);
+        if (NY > 32 && xg == 0) {
+          double v[16];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-              double y[16];
-#pragma unroll
-              for (int v = 0; v < 16; ++v) y[v] = cd[d] * val[gi][v];
-              uint4 dg[S];
-              digits16<S>(y, sv, dg);
-              const int kk = d * KD + 16 * x;  // K index of the group's first value
-              const uint32_t off = (uint32_t)(kk >> 5) * C::BCH + (uint32_t)(((kk >> 4) & 1) * 4 + (eb >> 3)) * 128 +
-                                   (uint32_t)(eb & 7) * 16;
-#pragma unroll
-              for (int p = 0; p < S; ++p) *reinterpret_cast<uint4 *>(sB + (size_t)p * C::BSLICE + off) = dg[p];
-            }
-          } else {
-            uint4 dg[S];
-            digits16<S>(val[gi], sl, dg);
-            const int kk = KV + 16 * (x - XV);
-            const uint32_t off = (uint32_t)(kk >> 5) * C::BCH + (uint32_t)(((kk >> 4) & 1) * 4 + (eb >> 3)) * 128 +
-                                 (uint32_t)(eb & 7) * 16;
-#pragma unroll
-            for (int p = 0; p < S; ++p) *reinterpret_cast<uint4 *>(sB + (size_t)p * C::BSLICE + off) = dg[p];
-          }
+          for (int q = 0; q < 16; ++q) v[q] = over[q];
+          emit(v, 32);
         }
       }
       fence_async_smem();  // the digits are read by the tensor cores (async proxy)
@@ -547,13 +578,7 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
       mbar_arrive(&sdone[s]);  // the state slot may be refilled (the epilogue reads the state from global)
 
       // ---- epilogue: join the levels, the stage update ----
-      const bool done = mbar_wait_bounded(accf, (uint32_t)k & 1u, kSpinLimit);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (!done) {
-        pend = true;  // no TMEM reads; the others learn of it at the next barrier
-        continue;
-      }
-      // this thread's state and residual first (coalesced over the lanes' nodes), then the accumulators
+      // this thread's state and residual (coalesced over the lanes' nodes) while the MMAs run
       float rs[8], hs[8], ls[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
@@ -566,6 +591,12 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
           ls[q] = __ldg(A.ulo_in + gi);
         }
       }
+      const bool done = mbar_wait_bounded(accf, (uint32_t)k & 1u, kSpinLimit);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (!done) {
+        pend = true;  // no TMEM reads; the others learn of it at the next barrier
+        continue;
+      }
       // Horner over the levels, highest first, loading TMEM in batches of up to three levels per wait
       double hv[8], hl[8];
 #pragma unroll
@@ -577,15 +608,17 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
           int av[3][8];
 #pragma unroll
           for (int j = 0; j < 3; ++j)
-            if (L0b - j >= 0) tmem_ld8_nowait(lane_tmem + (uint32_t)(((L0b - j) * 2 + acc) * TE + e0), av[j]);
+            if (L0b - j >= 0) tmem_ld8_nowait(lane_tmem + (uint32_t)((acc * S + L0b - j) * TE + e0), av[j]);
           tmem_wait_ld();
 #pragma unroll
           for (int j = 0; j < 3; ++j)
             if (L0b - j >= 0) {
+              // the elements' first digits went in as d + 128: level L holds 128 times its row of digit-L sums too much
+              const int corr = __ldg(A.rexp + 256 + (acc * S + L0b - j) * 128 + node);
 #pragma unroll
               for (int q = 0; q < 8; ++q) {
                 double &h = acc ? hl[q] : hv[q];
-                h = fma(h, 0.00390625, (double)av[j][q]);
+                h = fma(h, 0.00390625, (double)(av[j][q] - corr));
               }
             }
         }
@@ -674,7 +707,8 @@ void oz_pack_n(const double *Dr, const double *Ds, const double *Dt, const doubl
   using C = OzCfg<N, S>;
   constexpr int NP = C::NP, NF = C::NF, KD = C::KD, KV = C::KV, KL = C::KL, CT = C::CT;
   out.assign((size_t)S * CT * kOzChunk, 0);
-  rexp.assign(256, -1100);
+  rexp.assign(256 + 2 * S * 128, -1100);
+  std::fill(rexp.begin() + 256, rexp.end(), 0);
   const double *D[3] = {Dr, Ds, Dt};
   std::vector<double> rv((size_t)KV), rl((size_t)KL);
   std::vector<std::vector<int>> dv, dl;
@@ -703,6 +737,7 @@ void oz_pack_n(const double *Dr, const double *Ds, const double *Dt, const doubl
         const size_t off = (size_t)(p * CT + c) * kOzChunk + (size_t)(((kk >> 4) * 16 + (r >> 3)) * 128) +
                            (size_t)((r & 7) * 16 + (kk & 15));
         out[off] = (uint8_t)(v & 0xff);
+        rexp[(size_t)(256 + ((k < KV ? 0 : S) + p) * 128 + r)] += 128 * v;
       }
   }
 }
