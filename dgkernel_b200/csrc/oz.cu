@@ -35,10 +35,18 @@
 //
 // The matrix digits (S x 128 rows x (3 KD + KL) bytes, a few hundred KB) do not fit shared memory: they are
 // packed on the host in 4 KB chunks (one 32-wide K step of one digit) and streamed from L2 through a ring by a
-// producer warp; every chunk of digit p feeds the S - p MMAs with element digits q <= S - 1 - p, which stay in
-// shared memory for the tile.  CTA: 16 consumer warps (element digits, epilogue), one producer warp (state
-// slots and matrix chunks, 1-D bulk copies), one MMA warp.  Every wait is bounded; a failed wait sets the
-// status word, the CTA drains its copies and MMAs and frees TMEM.
+// producer warp, kOzGroup chunks per copy.  The element digits of a chunk lie side by side (row q 32 + e for digit q of
+// element e), so a chunk of matrix digit p feeds one MMA of N = 32 (S - p) columns, whose accumulators, levels p .. S-1,
+// lie side by side too.  One MMA has one signedness per operand: the elements' first digits go in as d + 128, and the
+// epilogue takes 128 times the matrices' digit sums from the levels they reach (integers: exact).  CTA: 16 consumer
+// warps (element digits, epilogue), one producer warp (state slots and matrix chunks, 1-D bulk copies), one MMA warp.
+// Every wait is bounded; a failed wait sets the status word, the CTA drains its copies and MMAs and frees TMEM.
+//
+// A tile runs through its phases one after the other (the digits' operand fills the shared memory), so their latency is
+// what bounds the kernel.  Order 7, 16^3 x 6, two steps: 2593 us with an MMA per pair of digits (357 a tile, 56 of its
+// 97 thousand clocks) and the values formed by the threads that cut them into digits (gathers 32 sectors wide); 1803
+// with one MMA per chunk and the values formed by consecutive threads in a scratch; 1331 with three chunks per copy and
+// commit (a chunk at a time, the producer's issue loop took 380 clocks a chunk).
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -56,7 +64,8 @@ namespace {
 
 constexpr int kOzTE = 32;         // elements per tile (the MMA's N; one compact-geometry slot)
 constexpr int kOzCW = 16;         // consumer warps
-constexpr int kOzRing = 16;       // matrix-chunk ring slots (64 KB in flight: covers the L2 latency)
+constexpr int kOzGroup = 3;       // matrix chunks per ring slot and copy (S CT chunks of a tile: a multiple of 6)
+constexpr int kOzRing = 5;        // ring slots (60 KB in flight: covers the L2 latency)
 constexpr int kOzSlots = 1;       // state slots: released after the digits are built, refilled during the MMAs
 constexpr int kOzChunk = 4096;    // bytes of one matrix chunk: 128 rows x 32 K
 constexpr int kOzTmemCols = 512;
@@ -87,7 +96,9 @@ struct OzCfg {
   // shared memory (bytes)
   static constexpr uint32_t OFF_B = 0;
   static constexpr uint32_t OFF_RING = OFF_B + CT * BCH;
-  static constexpr uint32_t OFF_SLOT = OFF_RING + kOzRing * kOzChunk;
+  static constexpr uint32_t OFF_SLOT = OFF_RING + kOzRing * kOzGroup * kOzChunk;
+  static constexpr int NG = S * CT / kOzGroup;            // ring slots filled per tile
+  static_assert(S * CT % kOzGroup == 0, "whole groups");
   static constexpr uint32_t OFF_BARY = OFF_SLOT + kOzSlots * SLOT_B;
   static constexpr uint32_t OFF_L0 = OFF_BARY + NP * 3 * 8;               // double per element, 2 tile buffers
   static constexpr uint32_t OFF_EXP = OFF_L0 + 2 * kOzTE * 8;             // int: Ev[2][32], El[2][32], Fv[128], Fl[128]
@@ -270,7 +281,9 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
     if (lane == 0) {
       bool bad = false;
       int nfill = 0;  // state fills issued (tiles 0 .. nfill - 1)
-      int64_t g = 0;  // matrix chunks issued
+      int64_t g = 0;  // ring slots filled
+      int rs = 0;     // the next one, and the parity of its fill
+      uint32_t par = 0;
       auto issue_fill = [&]() {
         const int k = nfill, s = k % kOzSlots;
         const MTile tl = A.tiles[blockIdx.x + k * G];
@@ -299,12 +312,10 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
         const int t = blockIdx.x + k * G;
         if (t >= A.ntiles) break;
         if (t + G >= A.ntiles) pdl_trigger();
-        for (int j = 0; j < S * CT; ++j, ++g) {
-          const int rs = (int)(g % kOzRing);
+        for (int j = 0; j < C::NG; ++j, ++g) {
           if (g >= kOzRing) {
-            const uint32_t par = (uint32_t)((g / kOzRing) - 1) & 1u;
             uint32_t it = 0;
-            while (!mbar_test_wait(&aemp[rs], par)) {
+            while (!mbar_test_wait(&aemp[rs], par ^ 1u)) {
               try_fill();
               if (++it >= kSpinLimit) {
                 bad = true;
@@ -316,8 +327,13 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
             bad = true;
             break;
           }
-          mbar_expect_tx(&aful[rs], kOzChunk);
-          bulk_g2s(ring + (size_t)rs * kOzChunk, A.amat + (size_t)j * kOzChunk, kOzChunk, &aful[rs]);
+          mbar_expect_tx(&aful[rs], kOzGroup * kOzChunk);
+          bulk_g2s(ring + (size_t)rs * kOzGroup * kOzChunk, A.amat + (size_t)j * kOzGroup * kOzChunk,
+                   kOzGroup * kOzChunk, &aful[rs]);
+          if (++rs == kOzRing) {
+            rs = 0;
+            par ^= 1u;
+          }
           try_fill();
         }
         // the fill of tile k + 1 must be out before the chunks of tile k + 1 can be used (bounded wait)
@@ -354,7 +370,8 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
     constexpr uint32_t M = 128;
     const uint32_t idesc_base = (2u << 4) | ((M >> 4) << 24);  // S32 accumulate, K-major, unsigned digits
     int64_t g = 0;
-    int k = 0, kc = -1;
+    int k = 0, kc = -1, rs = 0;
+    uint32_t par = 0;
     for (;; ++k) {
       const int t = blockIdx.x + k * G;
       if (t >= A.ntiles) break;
@@ -364,26 +381,35 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (int p = 0; p < S && !failed; ++p) {
-        for (int c = 0; c < CT; ++c, ++g) {
-          const int rs = (int)(g % kOzRing);
-          if (!mbar_wait_bounded(&aful[rs], (uint32_t)(g / kOzRing) & 1u, kSpinLimit)) {
-            failed = true;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          if (lane == 0) {
-            const uint64_t da = smem_desc(saddr(ring + (size_t)rs * kOzChunk), 2048, 128);
-            const int acc = c < CV ? 0 : 1;
+      int p = 0, c = 0;  // digit and K chunk of the next matrix chunk
+      for (int j = 0; j < C::NG; ++j, ++g) {
+        if (!mbar_wait_bounded(&aful[rs], par, kSpinLimit)) {
+          failed = true;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (lane == 0) {
+          const uint32_t sa = saddr(ring + (size_t)rs * kOzGroup * kOzChunk);
+#pragma unroll
+          for (int u = 0; u < kOzGroup; ++u) {
+            const uint64_t da = smem_desc(sa + u * kOzChunk, 2048, 128);
             const uint64_t db = smem_desc(saddr(sB + (size_t)c * C::BCH), C::BK, 128);
             // digits q = 0 .. S-1-p side by side: columns of levels p .. S-1, which lie side by side too
             const uint32_t idesc = idesc_base | ((p == 0 ? 1u : 0u) << 7) | ((uint32_t)((S - p) * TE >> 3) << 17);
-            const uint32_t col = (uint32_t)((acc * S + p) * TE);
+            const uint32_t col = (uint32_t)(((c < CV ? 0 : S) + p) * TE);
             tc_mma_i8(tmem + col, da, db, idesc, (p == 0 && (c == 0 || c == CV)) ? 0u : 1u);
-            tc_commit(&aemp[rs]);  // the ring slot is free once these MMAs have read it
+            if (++c == CT) {
+              c = 0;
+              ++p;
+            }
           }
-          __syncwarp();
+          tc_commit(&aemp[rs]);  // the ring slot is free once these MMAs have read it
         }
+        if (++rs == kOzRing) {
+          rs = 0;
+          par ^= 1u;
+        }
+        __syncwarp();
       }
       if (failed) break;
       if (lane == 0) tc_commit(accf);
