@@ -168,6 +168,7 @@ struct CompactGeoArgs {
 struct SplitJoinArgs {
   int npart, join;  // join = 0: u -> (hi, lo);  join = 1: (hi, lo) -> u
   const int64_t *count, *u_off, *hi_off, *lo_off;  // device, npart each (values)
+  int64_t most;     // the largest count
   double *u;
   float *hi, *lo;
 };

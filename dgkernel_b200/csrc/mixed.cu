@@ -37,6 +37,12 @@ struct MixedCfg {
   static constexpr int NP = O::NP, NFP = O::NFP, NF = O::NF;
   static constexpr int TE = kMixedSlotElems;
   static constexpr int NPJ = (NP + 3) & ~3;  // derivative rows padded to whole float4 groups
+  // Values per access to a lane's own rows.  With an even Np the lanes' scalars lie 4 (Np = 20) or more to a bank, as
+  // vectors they do not; the traces, whose nodes follow a mask, are read from a copy of uhi at an odd stride (order 5's
+  // copies would take half of the ring).  Order 3, 24 instances of 6^3 to 24^3: 2447 -> 2340
+  // us per two steps (shared-memory conflicts 147 -> 22 thousand clocks an SM; the matrix broadcasts remain).
+  static constexpr int VW = NP % 4 == 0 ? 4 : NP % 2 == 0 ? 2 : 1;
+  static constexpr uint32_t COPY_FLOATS = VW > 1 && N <= 3 ? (uint32_t)TE * (NP + 1) : 0;  // per consumer warp
   static constexpr uint32_t NODE_B = TE * NP * 4;
   static constexpr uint32_t GEO_B = TE * kMixedGeoWords * 4;
   static constexpr uint32_t CONN_B = TE * kMixedConnWords * 4;
@@ -49,15 +55,16 @@ struct MixedCfg {
 
 // Shared-memory layout of the kernel (host and device agree through this function).
 struct MixedSmem {
-  uint32_t ring, dm, lift, bary, bars, tags, ftab, fmask, misc, total;
+  uint32_t ring, dm, lift, copy, bary, bars, tags, ftab, fmask, misc, total;
 };
-__host__ __device__ inline MixedSmem mixed_smem(uint32_t slot_b, uint32_t dm_floats, uint32_t l_floats, int np,
-                                               int nfp, int ns, int ncodes) {
+__host__ __device__ inline MixedSmem mixed_smem(uint32_t slot_b, uint32_t dm_floats, uint32_t l_floats,
+                                               uint32_t copy_floats, int np, int nfp, int ns, int ncodes) {
   MixedSmem m{};
   m.ring = 0;
   m.dm = m.ring + (uint32_t)ns * slot_b;
   m.lift = m.dm + dm_floats * 4;
-  m.bary = m.lift + l_floats * 4;
+  m.copy = m.lift + l_floats * 4;
+  m.bary = m.copy + ((copy_floats + 1) & ~1u) * 4;
   m.bars = m.bary + (uint32_t)np * 3 * 8;
   m.tags = m.bars + 2u * (uint32_t)ns * 8;
   m.ftab = m.tags + round16(4u * (uint32_t)ns);
@@ -85,15 +92,37 @@ __device__ __forceinline__ void issue_slot(const MixedArgs &A, const MTile &tl, 
 
 __device__ __forceinline__ int vload(const int *p) { return *reinterpret_cast<const volatile int *>(p); }
 
+template <int V>
+__device__ __forceinline__ void ld_vec(const float *p, float (&v)[V]) {
+  if constexpr (V == 4) {
+    const float4 x = *reinterpret_cast<const float4 *>(p);
+    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+  } else if constexpr (V == 2) {
+    const float2 x = *reinterpret_cast<const float2 *>(p);
+    v[0] = x.x, v[1] = x.y;
+  } else {
+    v[0] = *p;
+  }
+}
+template <int V>
+__device__ __forceinline__ void st_vec(float *p, const float (&v)[V]) {
+  if constexpr (V == 4)
+    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  else if constexpr (V == 2)
+    *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+  else
+    *p = v[0];
+}
+
 }  // namespace
 
 template <int N, int CW>
 __global__ void __launch_bounds__(32 * (CW + 1), 1) rhs_stage_mixed_kernel(const MixedArgs A) {
   using C = MixedCfg<N>;
-  constexpr int NP = C::NP, NFP = C::NFP, NF = C::NF, NPJ = C::NPJ, TE = C::TE;
+  constexpr int NP = C::NP, NFP = C::NFP, NF = C::NF, NPJ = C::NPJ, TE = C::TE, VW = C::VW;
   extern __shared__ __align__(128) unsigned char sm[];
   const int NS = A.ns;
-  const MixedSmem L = mixed_smem(C::SLOT_B, C::DM_FLOATS, C::L_FLOATS, NP, NFP, NS, A.ncodes);
+  const MixedSmem L = mixed_smem(C::SLOT_B, C::DM_FLOATS, C::L_FLOATS, CW * C::COPY_FLOATS, NP, NFP, NS, A.ncodes);
   unsigned char *ring = sm + L.ring;
   float *sDm = reinterpret_cast<float *>(sm + L.dm);
   float *sL = reinterpret_cast<float *>(sm + L.lift);
@@ -211,46 +240,65 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1) rhs_stage_mixed_kernel(const
     const double dC = (cons ? 0.5 * uC * uC : uC) - wA;
     const double dD = (cons ? 0.5 * uD * uD : uD) - wA;
     float2 du[NPJ / 2];
+    // the traces' source: the element's own hi, or its copy at an odd stride
+    float *tr = reinterpret_cast<float *>(sm + L.copy) + (size_t)warp * C::COPY_FLOATS + lane * (NP + 1);
 #pragma unroll
-    for (int j = 0; j < NPJ; ++j) {
-      float v = 0.f;
-      if (j < NP) {
-        const double uj = (double)hi[j] + (double)lo[j];
-        const double wj = cons ? 0.5 * uj * uj : uj;
-        v = (float)((wj - wA) - (sBary[3 * j] * dB + sBary[3 * j + 1] * dC + sBary[3 * j + 2] * dD));
+    for (int j0 = 0; j0 < NPJ; j0 += VW) {
+      float h[VW], l[VW], v[VW];
+      if (j0 < NP) {
+        ld_vec<VW>(hi + j0, h);
+        ld_vec<VW>(lo + j0, l);
       }
-      if (j & 1)
-        du[j / 2].y = v;
-      else
-        du[j / 2].x = v;
+#pragma unroll
+      for (int q = 0; q < VW; ++q) {
+        const int j = j0 + q;
+        v[q] = 0.f;
+        if (j < NP) {
+          const double uj = (double)h[q] + (double)l[q];
+          const double wj = cons ? 0.5 * uj * uj : uj;
+          v[q] = (float)((wj - wA) - (sBary[3 * j] * dB + sBary[3 * j + 1] * dC + sBary[3 * j + 2] * dD));
+          if (C::COPY_FLOATS) tr[j] = h[q];
+        }
+        if (j & 1)
+          du[j / 2].y = v[q];
+        else
+          du[j / 2].x = v[q];
+      }
     }
+    const float *trace = C::COPY_FLOATS ? tr : hi;
     // derivative of the linear part along (1,1,1): d/dr = (wB-wA)/2 and likewise for s, t
     const float L0 = (float)(0.5 * ((double)cr * dB + (double)cs * dC + (double)ct * dD));
 
     // Volume pass: dd_i = cr (Dr dw)_i + cs (Ds dw)_i + ct (Dt dw)_i + L0 with paired FMAs; the residual slot
     // receives a*resu + dt*vol (the surface term is added in the next pass).
 #pragma unroll 1
-    for (int i = 0; i < NP; ++i) {
-      const float4 *Dq = reinterpret_cast<const float4 *>(sDm + i * 3 * NPJ);
-      float2 ar = make_float2(0.f, 0.f), as = ar, at = ar, br = ar, bs = ar, bt = ar;
+    for (int i0 = 0; i0 < NP; i0 += VW) {
+      const int o = e * NP + i0;
+      float re[VW], h[VW];
+      ld_vec<VW>(sRe + o, re);
+      ld_vec<VW>(hi + i0, h);
 #pragma unroll
-      for (int g = 0; g < NPJ / 4; ++g) {
-        const float4 q0 = Dq[3 * g], q1 = Dq[3 * g + 1], q2 = Dq[3 * g + 2];
-        ar = __ffma2_rn(make_float2(q0.x, q0.y), du[2 * g], ar);
-        as = __ffma2_rn(make_float2(q0.z, q0.w), du[2 * g], as);
-        at = __ffma2_rn(make_float2(q1.x, q1.y), du[2 * g], at);
-        br = __ffma2_rn(make_float2(q1.z, q1.w), du[2 * g + 1], br);
-        bs = __ffma2_rn(make_float2(q2.x, q2.y), du[2 * g + 1], bs);
-        bt = __ffma2_rn(make_float2(q2.z, q2.w), du[2 * g + 1], bt);
+      for (int q = 0; q < VW; ++q) {
+        const float4 *Dq = reinterpret_cast<const float4 *>(sDm + (i0 + q) * 3 * NPJ);
+        float2 ar = make_float2(0.f, 0.f), as = ar, at = ar, br = ar, bs = ar, bt = ar;
+#pragma unroll
+        for (int g = 0; g < NPJ / 4; ++g) {
+          const float4 q0 = Dq[3 * g], q1 = Dq[3 * g + 1], q2 = Dq[3 * g + 2];
+          ar = __ffma2_rn(make_float2(q0.x, q0.y), du[2 * g], ar);
+          as = __ffma2_rn(make_float2(q0.z, q0.w), du[2 * g], as);
+          at = __ffma2_rn(make_float2(q1.x, q1.y), du[2 * g], at);
+          br = __ffma2_rn(make_float2(q1.z, q1.w), du[2 * g + 1], br);
+          bs = __ffma2_rn(make_float2(q2.x, q2.y), du[2 * g + 1], bs);
+          bt = __ffma2_rn(make_float2(q2.z, q2.w), du[2 * g + 1], bt);
+        }
+        const float ur = (ar.x + ar.y) + (br.x + br.y);
+        const float us = (as.x + as.y) + (bs.x + bs.y);
+        const float ut = (at.x + at.y) + (bt.x + bt.y);
+        const float dd = fmaf(cr, ur, fmaf(cs, us, fmaf(ct, ut, L0)));
+        const float vol = cons ? -dd : -h[q] * dd;
+        re[q] = fmaf(a, re[q], dt * vol);
       }
-      const float ur = (ar.x + ar.y) + (br.x + br.y);
-      const float us = (as.x + as.y) + (bs.x + bs.y);
-      const float ut = (at.x + at.y) + (bt.x + bt.y);
-      const float dd = fmaf(cr, ur, fmaf(cs, us, fmaf(ct, ut, L0)));
-      const float vol = cons ? -dd : -hi[i] * dd;
-      const int o = e * NP + i;
-      const float t0 = fmaf(a, sRe[o], dt * vol);
-      if (valid) sRe[o] = t0;
+      if (valid) st_vec<VW>(sRe + o, re);
     }
 
     // Neighbour traces uP: inside the slot from shared memory, otherwise from the previous stage's state, read
@@ -280,7 +328,7 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1) rhs_stage_mixed_kernel(const
       const float g = gf[f], ga = fabsf(g);
 #pragma unroll
       for (int i = 0; i < NFP; ++i) {
-        const float uM = hi[sFm[f * NFP + i]];
+        const float uM = trace[sFm[f * NFP + i]];
         const float uP = fl[f * NFP + i];
         const float d = uM - uP;
         fl[f * NFP + i] = 0.5f * d * (0.5f * (uM + uP) * g - fmaxf(fabsf(uM), fabsf(uP)) * ga);
@@ -291,35 +339,45 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1) rhs_stage_mixed_kernel(const
     // Surface pass: LIFT row times the flux (paired FMAs), then the stage update in FP64, split into hi + lo.
     const uint32_t tail0 = ((uint32_t)(ne * NP * 4) & ~15u) / 4;  // nodes past the last full 16 B: plain stores
 #pragma unroll 1
-    for (int i = 0; i < NP; ++i) {
-      const float4 *Lq = reinterpret_cast<const float4 *>(sL + i * NF);
-      float2 l0 = make_float2(0.f, 0.f), l1 = l0, l2 = l0, l3 = l0;
+    for (int i0 = 0; i0 < NP; i0 += VW) {
+      const int o = e * NP + i0;
+      float re[VW], h[VW], l[VW];
+      ld_vec<VW>(sRe + o, re);
+      ld_vec<VW>(hi + i0, h);
+      ld_vec<VW>(lo + i0, l);
 #pragma unroll
-      for (int g = 0; g < NF / 4; ++g) {
-        const float4 m = Lq[g];
-        if (g & 1) {
-          l2 = __ffma2_rn(make_float2(m.x, m.y), make_float2(fl[4 * g], fl[4 * g + 1]), l2);
-          l3 = __ffma2_rn(make_float2(m.z, m.w), make_float2(fl[4 * g + 2], fl[4 * g + 3]), l3);
-        } else {
-          l0 = __ffma2_rn(make_float2(m.x, m.y), make_float2(fl[4 * g], fl[4 * g + 1]), l0);
-          l1 = __ffma2_rn(make_float2(m.z, m.w), make_float2(fl[4 * g + 2], fl[4 * g + 3]), l1);
+      for (int q = 0; q < VW; ++q) {
+        const float4 *Lq = reinterpret_cast<const float4 *>(sL + (i0 + q) * NF);
+        float2 l0 = make_float2(0.f, 0.f), l1 = l0, l2 = l0, l3 = l0;
+#pragma unroll
+        for (int g = 0; g < NF / 4; ++g) {
+          const float4 m = Lq[g];
+          if (g & 1) {
+            l2 = __ffma2_rn(make_float2(m.x, m.y), make_float2(fl[4 * g], fl[4 * g + 1]), l2);
+            l3 = __ffma2_rn(make_float2(m.z, m.w), make_float2(fl[4 * g + 2], fl[4 * g + 3]), l3);
+          } else {
+            l0 = __ffma2_rn(make_float2(m.x, m.y), make_float2(fl[4 * g], fl[4 * g + 1]), l0);
+            l1 = __ffma2_rn(make_float2(m.z, m.w), make_float2(fl[4 * g + 2], fl[4 * g + 3]), l1);
+          }
         }
+        const float lift = ((l0.x + l0.y) + (l1.x + l1.y)) + ((l2.x + l2.y) + (l3.x + l3.y));
+        const float rn = fmaf(dt, lift, re[q]);
+        const double un = ((double)h[q] + (double)l[q]) + b * (double)rn;
+        h[q] = __double2float_rn(un);
+        l[q] = __double2float_rn(un - (double)h[q]);
+        re[q] = rn;
       }
-      const float lift = ((l0.x + l0.y) + (l1.x + l1.y)) + ((l2.x + l2.y) + (l3.x + l3.y));
-      const int o = e * NP + i;
-      const float rn = fmaf(dt, lift, sRe[o]);
-      const double un = ((double)hi[i] + (double)lo[i]) + b * (double)rn;
-      const float hn = __double2float_rn(un);
-      const float ln = __double2float_rn(un - (double)hn);
       if (valid) {
-        sHi[o] = hn;
-        sLo[o] = ln;
-        sRe[o] = rn;
-        if ((uint32_t)o >= tail0) {
-          A.uhi_out[slot0 + o] = hn;
-          A.ulo_out[slot0 + o] = ln;
-          A.resu[slot0 + o] = rn;
-        }
+        st_vec<VW>(sHi + o, h);
+        st_vec<VW>(sLo + o, l);
+        st_vec<VW>(sRe + o, re);
+#pragma unroll
+        for (int q = 0; q < VW; ++q)
+          if ((uint32_t)(o + q) >= tail0) {
+            A.uhi_out[slot0 + o + q] = h[q];
+            A.ulo_out[slot0 + o + q] = l[q];
+            A.resu[slot0 + o + q] = re[q];
+          }
       }
     }
     fence_async_smem();  // this lane's slot writes become visible to the bulk stores
@@ -363,12 +421,12 @@ bool launch_mixed_n(const MixedArgs &A0, int ring_max, int num_sms, cudaStream_t
   MixedArgs A = A0;
   int ns = 0;
   const int cap = ring_max > 0 ? std::min(ring_max, 24) : 24;
-  while (ns < cap && mixed_smem(C::SLOT_B, C::DM_FLOATS, C::L_FLOATS, C::NP, C::NFP, ns + 1, A.ncodes).total <=
+  while (ns < cap && mixed_smem(C::SLOT_B, C::DM_FLOATS, C::L_FLOATS, CW * C::COPY_FLOATS, C::NP, C::NFP, ns + 1, A.ncodes).total <=
                          kSmemBudget)
     ++ns;
   if (ns < 2) return false;
   A.ns = ns;
-  const uint32_t smem = mixed_smem(C::SLOT_B, C::DM_FLOATS, C::L_FLOATS, C::NP, C::NFP, ns, A.ncodes).total;
+  const uint32_t smem = mixed_smem(C::SLOT_B, C::DM_FLOATS, C::L_FLOATS, CW * C::COPY_FLOATS, C::NP, C::NFP, ns, A.ncodes).total;
   auto kern = rhs_stage_mixed_kernel<N, CW>;
   mixed_attr<N, CW>();
   const int grid = std::max(1, std::min(num_sms, A.ntiles));
@@ -445,21 +503,47 @@ __global__ void compact_geometry_kernel(CompactGeoArgs<T> g) {
   }
 }
 
-// State split u -> (hi, lo) and join (hi, lo) -> u over partitions with their own value offsets.
-__global__ void split_join_kernel(SplitJoinArgs a) {
-  for (int p = 0; p < a.npart; ++p) {
+// State split u -> (hi, lo) and join (hi, lo) -> u over partitions with their own value offsets: a block per run of
+// kSplitRun values of a partition, loads of four values in flight.  24 uneven partitions, 16.4 M values: the two
+// steps that end in a join went from 2340 to 2326 us (a grid over one partition after another before).
+constexpr int kSplitRun = 4096, kSplitThreads = 256;
+
+__global__ void __launch_bounds__(kSplitThreads) split_join_kernel(SplitJoinArgs a) {
+  pdl_wait();
+  constexpr int CH = 4;
+  for (int p = blockIdx.y; p < a.npart; p += gridDim.y) {
     const int64_t n = a.count[p];
-    double *u = a.u + a.u_off[p];
-    float *hi = a.hi + a.hi_off[p];
-    float *lo = a.lo + a.lo_off[p];
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-      if (a.join) {
-        u[i] = (double)hi[i] + (double)lo[i];
-      } else {
-        const double v = u[i];
-        const float h = __double2float_rn(v);
-        hi[i] = h;
-        lo[i] = __double2float_rn(v - (double)h);
+    for (int64_t first = (int64_t)blockIdx.x * kSplitRun; first < n; first += (int64_t)gridDim.x * kSplitRun) {
+      const int m = (int)min((int64_t)kSplitRun, n - first);
+      double *u = a.u + a.u_off[p] + first;
+      float *hi = a.hi + a.hi_off[p] + first;
+      float *lo = a.lo + a.lo_off[p] + first;
+      for (int i0 = threadIdx.x; i0 < m; i0 += CH * kSplitThreads) {
+        if (a.join) {
+          float h[CH], l[CH];
+#pragma unroll
+          for (int j = 0; j < CH; ++j) {
+            const int i = i0 + j * kSplitThreads;
+            h[j] = i < m ? hi[i] : 0.f;
+            l[j] = i < m ? __ldcs(lo + i) : 0.f;
+          }
+#pragma unroll
+          for (int j = 0; j < CH; ++j)
+            if (i0 + j * kSplitThreads < m) __stcs(u + i0 + j * kSplitThreads, (double)h[j] + (double)l[j]);
+        } else {
+          double v[CH];
+#pragma unroll
+          for (int j = 0; j < CH; ++j) v[j] = i0 + j * kSplitThreads < m ? __ldcs(u + i0 + j * kSplitThreads) : 0.0;
+#pragma unroll
+          for (int j = 0; j < CH; ++j) {
+            const int i = i0 + j * kSplitThreads;
+            if (i < m) {
+              const float h = __double2float_rn(v[j]);
+              hi[i] = h;
+              lo[i] = __double2float_rn(v[j] - (double)h);
+            }
+          }
+        }
       }
     }
   }
@@ -512,8 +596,10 @@ template void launch_compact_geometry<float>(const CompactGeoArgs<float> &, cuda
 template void launch_compact_geometry<double>(const CompactGeoArgs<double> &, cudaStream_t);
 
 void launch_split_join(const SplitJoinArgs &a, cudaStream_t st) {
-  split_join_kernel<<<1184, 256, 0, st>>>(a);
-  cuda_check(cudaGetLastError(), "split_join_kernel launch");
+  const int64_t runs = (a.most + kSplitRun - 1) / kSplitRun;
+  const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(runs, 1 << 20)),
+                  (unsigned)std::min(a.npart, 65535));
+  launch_pdl(split_join_kernel, grid, kSplitThreads, 0, st, a);
 }
 
 }  // namespace dgk

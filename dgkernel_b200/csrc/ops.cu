@@ -918,6 +918,7 @@ struct MixedOp : Op {
 // State split u (float64) -> uhi + ulo (float32 pair) and the join back, per partition.
 struct SplitJoinOp : Op {
   int join;
+  int64_t most = 0;
   Binding *u, *hi, *lo;
   DevBuf cnt, uo, ho, lo_off;
   SplitJoinOp(Runner &r, Roles &R, int j) : join(j) {
@@ -929,7 +930,10 @@ struct SplitJoinOp : Op {
     same_layout(*hi, *lo, R.kname);
     require(u->values_per_elem == hi->values_per_elem, R.kname + ": u and uhi must hold the same values per element");
     std::vector<int64_t> c((size_t)r.npart);
-    for (int p = 0; p < r.npart; ++p) c[(size_t)p] = r.K[p] * hi->values_per_elem;
+    for (int p = 0; p < r.npart; ++p) {
+      c[(size_t)p] = r.K[p] * hi->values_per_elem;
+      most = std::max(most, c[(size_t)p]);
+    }
     cnt.upload(c.data(), c.size() * sizeof(int64_t));
     uo.upload(u->offsets.data(), sizeof(int64_t) * r.npart);
     ho.upload(hi->offsets.data(), sizeof(int64_t) * r.npart);
@@ -940,6 +944,7 @@ struct SplitJoinOp : Op {
     a.npart = r.npart;
     a.join = join;
     a.count = cnt.get<int64_t>();
+    a.most = most;
     a.u_off = uo.get<int64_t>();
     a.hi_off = ho.get<int64_t>();
     a.lo_off = lo_off.get<int64_t>();
