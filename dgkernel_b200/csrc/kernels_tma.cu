@@ -55,7 +55,11 @@ struct DmmaCfg {
   static constexpr int KL = NF / 4;        // k-steps of LIFT (NF = 4 Nfp)
   static constexpr int NT = TE / 8;        // n-tiles (8 elements)
   static constexpr int CONS = 32 * MT * NT / NW;  // consumer threads: one warp per (m-tile, NW n-tiles)
-  static constexpr int THREADS = CONS + 32;  // + one producer warp gathering neighbour traces
+  // Producer warps gathering neighbour traces.  The compact form's producer resolves a connectivity word and a table
+  // entry per point, which at orders 1 and 2 takes longer than the tile's products: with two warps a stage takes 48 and
+  // 133 us for 94 and 191 (40^3 x 6).  From order 3 on the products are the longer part, and a second one is slower.
+  static constexpr int PW = CP && N <= 2 ? 2 : 1;
+  static constexpr int THREADS = CONS + 32 * PW;
   // a bulk copy starts on 16 bytes; a tile that does not is copied from the 16 bytes that hold its start
   static constexpr int AV = 16 / sizeof(T);  // values per 16 bytes
   static constexpr uint32_t NODE_B = TE * NP * sizeof(T) + 16;
@@ -71,8 +75,10 @@ struct DmmaCfg {
   static constexpr int FTR = (NF / 4 + 15) & ~15;        // face-order table row: Nfp bytes rounded up to 16
   static constexpr uint32_t FTAB_B = CP ? 256 * FTR : 0;
   static constexpr size_t SMEM = 2 * (size_t)STAGE_B + WORK_B + 10 * sizeof(uint64_t) + FTAB_B;
-  static constexpr int MINB = N < 5 && 2 * SMEM <= 227 * 1024 ? 2 : 1;  // co-resident CTAs the launch bounds plan for
-  static constexpr int GJ = (TE * NF + 31) / 32;                  // gathers per producer lane and tile
+  // Co-resident CTAs that the launch bounds plan for.  At order 5 the compact form holds two only with a few registers
+  // spilled, which is still the faster (24^3 x 6: 178 us a stage, one CTA 242); the FP32 form runs one.
+  static constexpr int MINB = (CP || N < 5) && 2 * SMEM <= 227 * 1024 ? 2 : 1;
+  static constexpr int GJ = (TE * NF + 32 * PW - 1) / (32 * PW);  // gathers per producer lane and tile
   static_assert(NODE_B % 16 == 0 && FACE_B % 16 == 0 && GBUF_B % 16 == 0 && GEOC_B % 16 == 0,
                 "smem slots must stay 16-byte aligned");
   static_assert(TE % 8 == 0 && NF % 4 == 0 && NT % NW == 0, "tile must be whole n-tiles");
@@ -151,7 +157,7 @@ __device__ __forceinline__ void dmma_gather_load(const RhsArgs<T> &A, const Tile
   const int nfc = tl.nelem * NF;
 #pragma unroll
   for (int j = 0; j < GJ; ++j) {
-    const int idx = lane + 32 * j;
+    const int idx = lane + 32 * C::PW * j;
     src[j] = 0;
     code[j] = 0;
     if (idx < nfc) {
@@ -178,7 +184,7 @@ __device__ __forceinline__ void dmma_gather_finish(const RhsArgs<T> &A, const Ti
   const int ncd = min(A.ncodes, 256);
 #pragma unroll
   for (int j = 0; j < GJ; ++j) {
-    const int idx = lane + 32 * j;
+    const int idx = lane + 32 * C::PW * j;
     if (idx < nfc) {  // the point's face-order code, then the point's node in the neighbour
       const int e = idx / NF, q = idx - e * NF, f = q / NFP, p = q - f * NFP;
       const int cd = min((int)((code[j] >> (8 * f)) & 0xffu), ncd - 1);
@@ -217,7 +223,7 @@ __global__ void __launch_bounds__(DmmaCfg<N, CP, T>::THREADS, DmmaCfg<N, CP, T>:
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = gridDim.x;
   if (tid == 0) {
-    for (int i = 0; i < 8; ++i) mbar_init(&bar[i], 1);
+    for (int i = 0; i < 8; ++i) mbar_init(&bar[i], i == 2 || i == 3 ? C::PW : 1);
     done[0] = done[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -232,6 +238,7 @@ __global__ void __launch_bounds__(DmmaCfg<N, CP, T>::THREADS, DmmaCfg<N, CP, T>:
   __syncthreads();
 
   if (tid >= CONS) {
+    const int plane = C::PW == 1 ? lane : tid - CONS;  // lane among the producer warps
     pdl_wait();
     // ---------------- producer warp: neighbour traces ----------------
     // Software-pipelined over the CTA's tiles: while the traces of tile t are gathered, the loads of tile t + G's
@@ -248,7 +255,7 @@ __global__ void __launch_bounds__(DmmaCfg<N, CP, T>::THREADS, DmmaCfg<N, CP, T>:
     // loads are issued after the wait for the tile's buffer (pipelined, the compact stage ran 5% slower).
     int32_t src[GJ];
     uint32_t code[GJ];
-    if (!CP) dmma_gather_load<N, CP, T>(A, tl, sl, lane, src, code);
+    if (!CP) dmma_gather_load<N, CP, T>(A, tl, sl, plane, src, code);
     int k = 0;
     for (int t = blockIdx.x; t < A.ntiles; t += G, ++k) {
       const int s = k & 1;
@@ -256,13 +263,13 @@ __global__ void __launch_bounds__(DmmaCfg<N, CP, T>::THREADS, DmmaCfg<N, CP, T>:
         if (lane == 0) atomicExch(A.status, kStatusTimeoutCode);
         return;  // consumers time out on gready and leave as well
       }
-      if (CP) dmma_gather_load<N, CP, T>(A, tl, sl, lane, src, code);
-      dmma_gather_finish<N, CP, T>(A, tl, sft, lane, src, code);
+      if (CP) dmma_gather_load<N, CP, T>(A, tl, sl, plane, src, code);
+      dmma_gather_finish<N, CP, T>(A, tl, sft, plane, src, code);
       const int nfc = tl.nelem * NF;
       T up[GJ];
 #pragma unroll
       for (int j = 0; j < GJ; ++j) {
-        const int idx = lane + 32 * j;
+        const int idx = plane + 32 * C::PW * j;
         up[j] = T(0);
         if (idx < nfc) {
           if (src[j] >= 0 && (int64_t)src[j] < A.n_u_values) {
@@ -281,11 +288,11 @@ __global__ void __launch_bounds__(DmmaCfg<N, CP, T>::THREADS, DmmaCfg<N, CP, T>:
         tnn = A.tiles[t + 2 * G];
         if (CP) snn = A.tile_slot[t + 2 * G];
       }
-      if (!CP && t + G < A.ntiles) dmma_gather_load<N, CP, T>(A, tn, sn, lane, src, code);
+      if (!CP && t + G < A.ntiles) dmma_gather_load<N, CP, T>(A, tn, sn, plane, src, code);
       T *g = gbuf + s * TE * NF;
 #pragma unroll
       for (int j = 0; j < GJ; ++j) {
-        const int idx = lane + 32 * j;
+        const int idx = plane + 32 * C::PW * j;
         if (idx < nfc) g[idx] = up[j];
       }
       __syncwarp();
