@@ -4,7 +4,7 @@
 // Per stage, before the tensor-core mixed stage (tcm.cu), which adds the result to its right-hand side:
 //   ls_sensor   every element: modal coefficients uhat = Vinv u (FP64, on the FP64 tensor path), the
 //               Persson-Peraire activation from log10(E_top / E), the 35 -> 32 -> 32 -> 1 network (tanh, tanh,
-//               sigmoid; FP16 weights, FP32 sums; its hidden layers as TF32 tensor products with two-part
+//               sigmoid; FP16 weights, FP32 sums; its hidden layers as FP16 tensor products with two-part
 //               inputs) on uhat / |uhat| with the PP fallback inside (lo, hi) and, in mode 3, outputs <= lo read
 //               as a smooth element; eps_e = eps0 sigma_e h_e / N; elements with eps_e > 0 form the active list.
 //               The pass marks the active elements and their face neighbours, and ls_compact lists them (touched).
@@ -62,18 +62,22 @@ __device__ __forceinline__ int64_t slot_of_value(const LsArgs &A, int64_t g, int
   return -1;
 }
 
-// TF32 helpers of the network's tensor products: x = hi + lo with both parts TF32 (round to nearest), and one m16n8k8 product accumulated into d.
-__device__ __forceinline__ void ls_tf32_split(float x, uint32_t &hi, uint32_t &lo) {
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
-  const float r = x - __uint_as_float(hi);
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(r));
+// The network's inputs as FP16 pairs: x 2^10 = hi + lo, both rounded to nearest (|x| <= 1: a unit-norm feature or a
+// tanh; the scale keeps the low part out of FP16's subnormals for all but the smallest inputs), and one m16n8k16
+// product accumulated into d.
+constexpr float kLsScale = 1024.f;
+__device__ __forceinline__ void ls_put(__half *row, int lo_off, float x) {
+  const float v = x * kLsScale;
+  const __half h = __float2half_rn(v);
+  row[0] = h;
+  row[lo_off] = __float2half_rn(v - __half2float(h));
 }
 
-__device__ __forceinline__ void ls_mma_tf32(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+__device__ __forceinline__ void ls_mma_f16(float (&d)[4], const uint4 &a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
                "{%0,%1,%2,%3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+               : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
 }
 
 __device__ __forceinline__ void ls_dmma(double &c0, double &c1, double a, double b) {
@@ -89,38 +93,33 @@ __device__ __forceinline__ void ls_dmma(double &c0, double &c1, double a, double
 // pipe was 85 % busy with the matrix and the weights read entry by entry and rows at conflicting strides), so Vinv and
 // the weights lie there in fragment order (one 8-byte load per lane and fragment) and the rows at strides that spread
 // the 8 rows of a fragment over the banks.  The logarithm and the sine of the ramp run only where the energy ratio can
-// reach it.  @LSENS@
+// reach it.  Order 4, 32^3 x 6: 75 us with entry-by-entry reads, 61 so, 57 with the network on FP16 pairs (half the
+// products of TF32 ones at the same 22 bits an input, and the weights need no conversion).
 template <int N>
 struct LsSensorSmem {
-  static constexpr int NP = Order<N>::NP, MT = (NP + 7) / 8, KT = (NP + 3) / 4, K1 = (NP + 7) / 8, K2 = kLsHid / 8;
+  static constexpr int NP = Order<N>::NP, MT = (NP + 7) / 8, KT = (NP + 3) / 4, K1 = (NP + 15) / 16, K2 = kLsHid / 16;
   static constexpr int SU = frag_stride(NP);           // nodal values of an element
-  static constexpr int SX = (NP + 3) / 8 * 8 + 4;      // features: 4 mod 8, rows 4 banks apart (in some order)
-  static constexpr int SH = kLsHid + 4;                // hidden units
-  static_assert(SX >= NP && SX % 8 == 4, "feature row stride");
+  static constexpr int SX = 8 * K1 + 4;  // words of a feature row: two FP16 each, 4 mod 8 (conflict-free)
+  static constexpr int SH = 8 * K2 + 4;                // words of a row of hidden units
   double vinv[MT * KT * 32];                           // [m-tile][k-step][lane]
   double u[kLsWarps][8 * SU];
-  float x[kLsWarps][8 * SX], h[kLsWarps][8 * SH];
-  uint2 w[(K1 + K2) * 2 * 32];                         // FP16 weights: [k-step][m-tile][lane], 4 per lane
+  uint4 w[(K1 + K2) * 2 * 32];                         // FP16 weights: [k-step][m-tile][lane], 8 per lane
+  uint32_t x[kLsWarps][2][8 * SX], h[kLsWarps][2][8 * SH];  // high and low parts; columns past the inputs stay zero
   float b1[kLsHid], b2[kLsHid], w3[kLsHid], b3;
 };
 
-// one hidden layer: o[m-tile] += W x over K k-steps; x(k) is this lane's element g, input k
-template <int K, typename X>
-__device__ __forceinline__ void ls_layer(const uint2 *w, int lane, X &&x, float (&o)[2][4]) {
+// one hidden layer: o[m-tile] += W x over K k-steps; x points at this lane's word of its element's row, the low
+// parts lie `lo` words behind
+template <int K>
+__device__ __forceinline__ void ls_layer(const uint4 *w, const uint32_t *x, int lo, float (&o)[2][4]) {
 #pragma unroll
   for (int kk = 0; kk < K; ++kk) {
-    const int j0 = 8 * kk + (lane & 3);
-    uint32_t bh[2], bl[2];
-    ls_tf32_split(x(j0), bh[0], bl[0]);
-    ls_tf32_split(x(j0 + 4), bh[1], bl[1]);
+    const uint32_t h0 = x[8 * kk], h1 = x[8 * kk + 4], l0 = x[lo + 8 * kk], l1 = x[lo + 8 * kk + 4];
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt) {
-      const uint2 q = w[(kk * 2 + mt) * 32 + lane];
-      const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&q.x));
-      const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&q.y));
-      const uint32_t a[4] = {__float_as_uint(lo.x), __float_as_uint(lo.y), __float_as_uint(hi.x), __float_as_uint(hi.y)};
-      ls_mma_tf32(o[mt], a, bh);
-      ls_mma_tf32(o[mt], a, bl);
+      const uint4 a = w[(kk * 2 + mt) * 32];
+      ls_mma_f16(o[mt], a, h0, h1);
+      ls_mma_f16(o[mt], a, l0, l1);
     }
   }
 }
@@ -149,14 +148,17 @@ __global__ void __launch_bounds__(32 * kLsWarps, 3) ls_sensor_kernel(const LsArg
       const int l = i & 31, mt = (i >> 5) & 1, kk = i >> 6;
       const bool first = kk < K1;
       const float *W = first ? W1 : W2;
-      const int nin = first ? NP : kLsHid, r = 16 * mt + (l >> 2), j = 8 * (first ? kk : kk - K1) + (l & 3);
-      auto at = [&](int rr, int jj) { return jj < nin ? W[rr * nin + jj] : 0.f; };
-      const __half2 lo = __floats2half2_rn(at(r, j), at(r + 8, j)), hi = __floats2half2_rn(at(r, j + 4), at(r + 8, j + 4));
-      m.w[i] = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+      const int nin = first ? NP : kLsHid, r = 16 * mt + (l >> 2), j = 16 * (first ? kk : kk - K1) + 2 * (l & 3);
+      auto pair = [&](int rr, int jj) {
+        const __half2 v = __floats2half2_rn(jj < nin ? W[rr * nin + jj] : 0.f, jj + 1 < nin ? W[rr * nin + jj + 1] : 0.f);
+        return *reinterpret_cast<const uint32_t *>(&v);
+      };
+      m.w[i] = make_uint4(pair(r, j), pair(r + 8, j), pair(r, j + 8), pair(r + 8, j + 8));
     }
+    for (int i = tid; i < kLsWarps * 2 * 8 * S::SX; i += blockDim.x) (&m.x[0][0][0])[i] = 0;
     if (tid < kLsHid) {
-      m.b1[tid] = h16(B1[tid]);
-      m.b2[tid] = h16(B2[tid]);
+      m.b1[tid] = h16(B1[tid]) * kLsScale;
+      m.b2[tid] = h16(B2[tid]) * kLsScale;
       m.w3[tid] = h16(W3[tid]);
     }
     if (tid == 0) m.b3 = h16(W3[kLsHid]);
@@ -164,7 +166,7 @@ __global__ void __launch_bounds__(32 * kLsWarps, 3) ls_sensor_kernel(const LsArg
   if (blockIdx.x == 0 && tid == 0) A.counts[1] = 0;  // the touched list of this stage is counted after this kernel
   __syncthreads();
   double *su = m.u[warp];
-  float *sx = m.x[warp], *sh = m.h[warp];
+  __half *sx = reinterpret_cast<__half *>(m.x[warp][0]), *sh = reinterpret_cast<__half *>(m.h[warp][0]);
   const int el = 2 * c + (g & 1);  // this lane's element
   const int ngroups = 16 * A.ntiles, gstep = gridDim.x * kLsWarps;
   constexpr int FILL = (8 * NP + 31) / 32;  // values per lane
@@ -242,36 +244,37 @@ __global__ void __launch_bounds__(32 * kLsWarps, 3) ls_sensor_kernel(const LsArg
       for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-          if (8 * mt + g < NP) sx[(2 * c + h) * SX + 8 * mt + g] = (float)(uh[mt][h] * iv[h]);
+          if (8 * mt + g < NP) ls_put(sx + (2 * c + h) * 2 * SX + 8 * mt + g, 16 * SX, (float)(uh[mt][h] * iv[h]));
       __syncwarp();
-      // the network on the 8 elements with tensor products (mma.sync m16n8k8, TF32 operands, FP32 sums): every FP16
-      // weight is exact in TF32 and each FP32 input is split into two TF32 parts (hi + lo), so the products keep
-      // FP32-level rounding.  Rows are hidden units (two 16-row m-tiles), columns the warp's elements.
+      // the network on the 8 elements with tensor products (mma.sync m16n8k16, FP16 operands, FP32 sums): the weights
+      // are FP16 and each input a pair of FP16 parts, so the products keep FP32-level rounding.  Rows are hidden units
+      // (two 16-row m-tiles), columns the warp's elements.
       float o[2][4];
 #pragma unroll
       for (int mt = 0; mt < 2; ++mt) {
         o[mt][0] = o[mt][1] = m.b1[16 * mt + g];
         o[mt][2] = o[mt][3] = m.b1[16 * mt + g + 8];
       }
-      ls_layer<K1>(m.w, lane, [&](int j) { return j < NP ? sx[g * SX + j] : 0.f; }, o);
+      ls_layer<K1>(m.w + lane, m.x[warp][0] + g * SX + c, 8 * SX, o);
 #pragma unroll
       for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-        for (int f = 0; f < 4; ++f) sh[(2 * c + (f & 1)) * SH + 16 * mt + g + 8 * (f >> 1)] = tanhf(o[mt][f]);
+        for (int f = 0; f < 4; ++f)
+          ls_put(sh + (2 * c + (f & 1)) * 2 * SH + 16 * mt + g + 8 * (f >> 1), 16 * SH, tanhf(o[mt][f] * (1.f / kLsScale)));
       __syncwarp();
 #pragma unroll
       for (int mt = 0; mt < 2; ++mt) {
         o[mt][0] = o[mt][1] = m.b2[16 * mt + g];
         o[mt][2] = o[mt][3] = m.b2[16 * mt + g + 8];
       }
-      ls_layer<K2>(m.w + K1 * 2 * 32, lane, [&](int j) { return sh[g * SH + j]; }, o);
+      ls_layer<K2>(m.w + K1 * 2 * 32 + lane, m.h[warp][0] + g * SH + c, 8 * SH, o);
       // output unit: this lane's four units of elements 2c and 2c + 1, summed over the lanes of the same c
       float za = 0.f, zb = 0.f;
 #pragma unroll
       for (int mt = 0; mt < 2; ++mt) {
         const float wlo = m.w3[16 * mt + g], whi = m.w3[16 * mt + g + 8];
-        za += wlo * tanhf(o[mt][0]) + whi * tanhf(o[mt][2]);
-        zb += wlo * tanhf(o[mt][1]) + whi * tanhf(o[mt][3]);
+        za += wlo * tanhf(o[mt][0] * (1.f / kLsScale)) + whi * tanhf(o[mt][2] * (1.f / kLsScale));
+        zb += wlo * tanhf(o[mt][1] * (1.f / kLsScale)) + whi * tanhf(o[mt][3] * (1.f / kLsScale));
       }
 #pragma unroll
       for (int x = 4; x <= 16; x <<= 1) {
