@@ -584,7 +584,7 @@ def volume_microbench(prob, stream, hbm, local, launches: int = 20, warmup: int 
     err = float(np.linalg.norm(got - ux) / np.linalg.norm(ux))
     return {"value": gbs, "unit": "GB/s", "ms_per_launch": ms, "launches": launches, "bytes_per_launch": nbytes,
             "formula": "13 * 8 B * Np * K / t (tet_nudg_mesh_physical_derivative_test.go:544-547)",
-            "hbm_frac": gbs / hbm, "dof_per_s": Np * K / (ms * 1e-3), "kernel": "diff_kernel",
+            "hbm_frac": gbs / hbm, "dof_per_s": Np * K / (ms * 1e-3), "kernel": "diff_dmma_kernel",
             "dudx_rel_err_vs_analytic": err, "clocks": clk.summary()}
 
 
@@ -604,7 +604,7 @@ def run_burgers(args, world, rank, local):
              ("mixed", MIXED, {})]
     if args.order <= 4:
         forms.append(("mixed_tc", MIXED, {"mma": True}))
-    kernels = {"f64": "rhs_stage_dmma_kernel", "f64c": "rhs_stage_dmma_kernel (compact)", "f32": "rhs_stage_kernel",
+    kernels = {"f64": "rhs_stage_dmma_kernel", "f64c": "rhs_stage_dmma_kernel (compact)", "f32": "rhs_stage_dmma_kernel (float)",
                "mixed": "rhs_stage_mixed_kernel", "mixed_tc": "rhs_stage_tcm_kernel"}
     micro = None
     for name, dt, kw in forms:
