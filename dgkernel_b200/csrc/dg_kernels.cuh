@@ -54,8 +54,6 @@ template <> struct Shape<2> { static constexpr int TE = 64, RG = 5; };
 template <> struct Shape<3> { static constexpr int TE = 64, RG = 5; };
 template <> struct Shape<4> { static constexpr int TE = 32, RG = 5; };
 template <> struct Shape<5> { static constexpr int TE = 32, RG = 7; };
-template <> struct Shape<6> { static constexpr int TE = 32, RG = 7; };
-template <> struct Shape<7> { static constexpr int TE = 32, RG = 8; };
 
 template <int N>
 struct Cfg {

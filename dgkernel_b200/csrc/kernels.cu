@@ -1,5 +1,5 @@
-// sm_100a kernels: type conversion for the copy engine, and the tet-DG hot path (volume derivative,
-// reference-form computeRHS / updateSolution, fused Lax-Friedrichs RHS + LSERK4 stage).
+// sm_100a kernels: type conversion for the copy engine, the update kernels (updateSolution, lserkUpdate), and the
+// register-staged form of the fused Lax-Friedrichs RHS + LSERK4 stage (orders 1..5, for DGK_DISABLE_TMA=1).
 #include <cstdint>
 #include <type_traits>
 
@@ -480,8 +480,6 @@ int tile_elems(int N) {
     case 3: return Cfg<3>::TE;
     case 4: return Cfg<4>::TE;
     case 5: return Cfg<5>::TE;
-    case 6: return Cfg<6>::TE;
-    case 7: return Cfg<7>::TE;
     default: throw Error(DGK_ERR_UNSUPPORTED, "order N must be 1..7");
   }
 }
