@@ -3,7 +3,7 @@
 // linear vertex interpolant, flux and residual in FP32, update in FP64).
 //
 // mixed.cu gives each lane an element, which amortises the work around the products but leaves a small problem as a
-// few long serial chains: 14 us for any order-3 problem of up to 10,000 elements.  Here a thread owns one output row:
+// few long serial chains: 12 us for any order-3 problem of up to 10,000 elements.  Here a thread owns one output row:
 // its rows of Dr, Ds, Dt and LIFT stay in registers for the whole persistent kernel (100 values at order 3), and the
 // element vectors are read from shared memory as 16-byte broadcasts, four columns of three matrices (six paired FMAs)
 // per load.  Thread (e, i) also owns node i of element e and the face points i, i + Np, ...: consecutive threads are
@@ -14,12 +14,12 @@
 // 330 per node at order 3 against mixed.cu's 150) once every SM is busy.  The lines of rows_faster follow from stages in
 // a captured graph, us, mixed.cu / here:
 //   elements    order 1      order 2      order 3      order 4
-//        384    6.0 / 2.5    8.9 / 3.5   13.4 / 4.4   21.0 / 7.7
-//       6000    6.8 / 2.7    9.5 / 4.8   14.0 / 7.8   22.0 / 11.9
-//      16464    8.0 / 3.1   10.7 / 6.8   15.3 / 11.4  23.2 / 21.7
-//      29478    9.7 / 3.7   12.8 / 8.5   18.3 / 16.3  29.2 / 34.9
-//      48000   11.9 / 4.8   15.1 / 10.9  22.8 / 23.8  36.6 / 52.5
-//     131712   22.0 / 8.6   26.5 / 23.7  47.0 / 59.1  87.9 / 130.7
+//        384    4.0 / 2.3    6.6 / 2.7    9.7 / 3.3   19.1 / 6.0
+//       6000    5.6 / 2.5    8.3 / 3.5   12.0 / 6.8   22.0 / 10.7
+//      16464    6.6 / 2.9    9.3 / 5.6   12.6 / 10.6  22.4 / 20.6
+//      29478    8.5 / 3.0   11.4 / 7.6   15.3 / 15.6  28.4 / 33.2
+//      48000   10.7 / 4.4   14.0 / 10.5  19.9 / 23.0  36.0 / 50.4
+//     131712   21.0 / 8.1   25.7 / 23.7  41.9 / 58.1  86.4 / 128.3
 #include <algorithm>
 #include <cstdint>
 
@@ -281,7 +281,7 @@ bool rows_faster(int N, int64_t nelems, int num_sms) {
   switch (N) {
     case 1: return true;
     case 2: return nelems <= 1300 * (int64_t)num_sms;
-    case 3: return nelems <= 240 * (int64_t)num_sms;
+    case 3: return nelems <= 190 * (int64_t)num_sms;
     case 4: return nelems <= 110 * (int64_t)num_sms;
     default: return false;
   }
