@@ -5,6 +5,9 @@
 // when the operator was built), then waits for that kernel to complete (pdl_wait) before it touches anything another
 // kernel may have written.  This hides the launch gap and the prologue, which is most of a small problem's stage.
 // The trigger comes with the last tile, not earlier: a waiting CTA holds registers and shared memory.
+// The kernel's lifetime overlaps its predecessor's, so what the predecessor writes (state, residual, lists) is not read-only
+// for the whole of it: such arrays are read with ordinary loads, __ldcg or __ldcs, never with __ldg / ld.global.nc, whose
+// contract asks for that and which need not stay behind the wait.  Those are for the operator's constants alone.
 // Alone on the GPU, two steps of small mixed problems (2 to 16 instances of 4^3 to 16^3): 112 -> 77 and 94 -> 65 us; order 2,
 // 8^3 x 6 FP64 step: 40 -> 31 us; 64^3-class stages are unchanged.
 #pragma once

@@ -488,8 +488,8 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
             const int cdx = min((int)((codes >> (8 * f)) & 0xffu), ncodes - 1);
             const uint32_t idx = nbs + sFt[cdx * 64 + pp];
             if (idx < n_u32) {
-              pH[i] = __ldg(A.uhi_in + idx);
-              pL[i] = __ldg(A.ulo_in + idx);
+              pH[i] = __ldcg(A.uhi_in + idx);
+              pL[i] = __ldcg(A.ulo_in + idx);
             } else {  // out of range: reported, and the point takes its own trace (zero jump)
               badg = true;
               pH[i] = sHi[e * NP + sPt[m]];
@@ -613,8 +613,8 @@ __global__ void __launch_bounds__(32 * (kOzCW + 2), 1) rhs_stage_oz_kernel(const
         if (node < NP && e < ne) {
           const int64_t gi = slot0 + e * NP + node;
           rs[q] = A.resu[gi];
-          hs[q] = __ldg(A.uhi_in + gi);
-          ls[q] = __ldg(A.ulo_in + gi);
+          hs[q] = __ldcg(A.uhi_in + gi);
+          ls[q] = __ldcg(A.ulo_in + gi);
         }
       }
       const bool done = mbar_wait_bounded(accf, (uint32_t)k & 1u, kSpinLimit);

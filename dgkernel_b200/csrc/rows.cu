@@ -108,9 +108,9 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS, RowCfg<N>::MINB) rhs_stage
       for (int j = 0; j < NJ; ++j) {
         const bool ok = (uint32_t)idx[g][j] < nvalues;
         if (!ok) bad |= 1u << (g * NJ + j);
-        up[g][j] = ok ? __ldg(A.uhi_in + (uint32_t)idx[g][j]) : 0.f;
+        up[g][j] = ok ? __ldcg(A.uhi_in + (uint32_t)idx[g][j]) : 0.f;
       }
-      nh[g] = in ? __ldg(hp + g * EP * NP) : 0.f;
+      nh[g] = in ? __ldcg(hp + g * EP * NP) : 0.f;
       nl[g] = in ? __ldcs(lp + g * EP * NP) : 0.f;
       nr[g] = in ? __ldcs(rp + g * EP * NP) : 0.f;
     }
