@@ -308,8 +308,9 @@ __global__ void __launch_bounds__(32 * kLsWarps, 3) ls_sensor_kernel(const LsArg
 // touched list and row of every slot (-1 elsewhere); the flags are cleared for the next stage
 __global__ void ls_compact_kernel(const LsArgs A) {
   pdl_wait();
-  pdl_trigger();
-  for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < A.nslots; s += (int64_t)gridDim.x * blockDim.x) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < A.nslots; s += step) {
+    if (threadIdx.x == 0 && s + step >= A.nslots) pdl_trigger();
     if (A.tflag[s]) {
       const int r = atomicAdd(&A.counts[1], 1);
       A.tlist[r] = (int32_t)s;
@@ -328,6 +329,11 @@ __global__ void ls_compact_kernel(const LsArgs A) {
 // the few tens of KB stay there); lane l's output row is 8 mt + l / 4, its elements 2 (l mod 4) and
 // 2 (l mod 4) + 1.  The mixed stage requires straight-sided elements, so the metrics are constant over an
 // element and are read once per element.
+//
+// The list pass and the gradient let the next kernel start with their last group, the divergence not before its end.
+// Started at once, the waiting CTAs cost more than the launch gap that they hide as soon as the lists are long (order 4,
+// every element active, 32^3 x 6: 1204 us a stage, 994 so; 48^3 x 6: 3550 and 3293); the stage kernel waiting under the
+// divergence's last groups costs 6 % at order 3 (32^3 x 6: 691 us a stage, 651 so).  With empty lists it is all the same.
 template <int N>
 struct LsCfg {
   using O = Order<N>;
@@ -382,10 +388,10 @@ __global__ void __launch_bounds__(LsCfg<N>::THREADS) ls_grad_kernel(const LsArgs
   const int tid = threadIdx.x, lane = tid & 31, mt = tid >> 5;
   const int ar = lane >> 2, ac = lane & 3, r = 8 * mt + ar;
   pdl_wait();
-  pdl_trigger();
   const int n = *reinterpret_cast<volatile const int *>(&A.counts[0]);
   const int ngroups = (n + 7) / 8;
   for (int gi = blockIdx.x; gi < ngroups; gi += gridDim.x) {
+    if (tid == 0 && gi + (int)gridDim.x >= ngroups) pdl_trigger();
     ls_stage_elems<N>(A, A.alist, n, gi, se, true);
     __syncthreads();
     for (int x = tid; x < 8 * NPU; x += C::THREADS) {
@@ -473,7 +479,6 @@ __global__ void __launch_bounds__(LsCfg<N>::THREADS) ls_div_kernel(const LsArgs 
   const int tid = threadIdx.x, lane = tid & 31, mt = tid >> 5;
   const int ar = lane >> 2, ac = lane & 3, r = 8 * mt + ar;
   pdl_wait();
-  pdl_trigger();
   const int n = *reinterpret_cast<volatile const int *>(&A.counts[1]);
   if (blockIdx.x == 0 && tid == 0) A.counts[0] = 0;  // the next stage's sensor pass counts from zero
   const int ngroups = (n + 7) / 8;
