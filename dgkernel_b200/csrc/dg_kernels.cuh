@@ -163,13 +163,19 @@ struct CompactGeoArgs {
   int *bad;                    // count of elements that are not affine within 1e-9
 };
 
+// A run of consecutive values of one partition: its value offsets in u, hi and lo.
+struct SplitRun {
+  int64_t u, hi, lo;
+  int32_t n;
+};
+
 struct SplitJoinArgs {
-  int npart, join;  // join = 0: u -> (hi, lo);  join = 1: (hi, lo) -> u
-  const int64_t *count, *u_off, *hi_off, *lo_off;  // device, npart each (values)
-  int64_t most;     // the largest count
+  const SplitRun *runs;  // device; at most kSplitRunValues values each
+  int nruns, join;       // join = 0: u -> (hi, lo);  join = 1: (hi, lo) -> u
   double *u;
   float *hi, *lo;
 };
+constexpr int kSplitRunValues = 4096;
 
 // ---- precision form with exact integer products on the tensor cores (oz.cu) ----
 struct OzArgs {

@@ -504,48 +504,50 @@ __global__ void compact_geometry_kernel(CompactGeoArgs<T> g) {
 }
 
 // State split u -> (hi, lo) and join (hi, lo) -> u over partitions with their own value offsets: a block per run of
-// kSplitRun values of a partition, loads of four values in flight.  24 uneven partitions, 16.4 M values: the two
-// steps that end in a join went from 2340 to 2326 us (a grid over one partition after another before).
-constexpr int kSplitRun = 4096, kSplitThreads = 256;
+// values of a partition (operator's list), loads of four values in flight.  Bound by HBM.  24 uneven partitions, 16.4 M
+// values: the two steps that end in a join went from 2340 to 2326 us against a grid that walked the partitions one after
+// another.  A list, because a grid of runs x partitions is empty blocks where one partition is much larger than the
+// rest (998,250 elements of order 2 beside 3000 of 162: 41 us a join, where that grid took 3804).
+constexpr int kSplitThreads = 256;
 
 __global__ void __launch_bounds__(kSplitThreads) split_join_kernel(SplitJoinArgs a) {
-  pdl_wait();
   constexpr int CH = 4;
-  for (int p = blockIdx.y; p < a.npart; p += gridDim.y) {
-    const int64_t n = a.count[p];
-    for (int64_t first = (int64_t)blockIdx.x * kSplitRun; first < n; first += (int64_t)gridDim.x * kSplitRun) {
-      const int m = (int)min((int64_t)kSplitRun, n - first);
-      double *u = a.u + a.u_off[p] + first;
-      float *hi = a.hi + a.hi_off[p] + first;
-      float *lo = a.lo + a.lo_off[p] + first;
-      for (int i0 = threadIdx.x; i0 < m; i0 += CH * kSplitThreads) {
-        if (a.join) {
-          float h[CH], l[CH];
+  SplitRun r = a.runs[blockIdx.x];
+  pdl_wait();
+  for (int k = blockIdx.x;;) {
+    const int m = r.n;
+    double *u = a.u + r.u;
+    float *hi = a.hi + r.hi;
+    float *lo = a.lo + r.lo;
+    for (int i0 = threadIdx.x; i0 < m; i0 += CH * kSplitThreads) {
+      if (a.join) {
+        float h[CH], l[CH];
 #pragma unroll
-          for (int j = 0; j < CH; ++j) {
-            const int i = i0 + j * kSplitThreads;
-            h[j] = i < m ? hi[i] : 0.f;
-            l[j] = i < m ? __ldcs(lo + i) : 0.f;
-          }
+        for (int j = 0; j < CH; ++j) {
+          const int i = i0 + j * kSplitThreads;
+          h[j] = i < m ? hi[i] : 0.f;
+          l[j] = i < m ? __ldcs(lo + i) : 0.f;
+        }
 #pragma unroll
-          for (int j = 0; j < CH; ++j)
-            if (i0 + j * kSplitThreads < m) __stcs(u + i0 + j * kSplitThreads, (double)h[j] + (double)l[j]);
-        } else {
-          double v[CH];
+        for (int j = 0; j < CH; ++j)
+          if (i0 + j * kSplitThreads < m) __stcs(u + i0 + j * kSplitThreads, (double)h[j] + (double)l[j]);
+      } else {
+        double v[CH];
 #pragma unroll
-          for (int j = 0; j < CH; ++j) v[j] = i0 + j * kSplitThreads < m ? __ldcs(u + i0 + j * kSplitThreads) : 0.0;
+        for (int j = 0; j < CH; ++j) v[j] = i0 + j * kSplitThreads < m ? __ldcs(u + i0 + j * kSplitThreads) : 0.0;
 #pragma unroll
-          for (int j = 0; j < CH; ++j) {
-            const int i = i0 + j * kSplitThreads;
-            if (i < m) {
-              const float h = __double2float_rn(v[j]);
-              hi[i] = h;
-              lo[i] = __double2float_rn(v[j] - (double)h);
-            }
+        for (int j = 0; j < CH; ++j) {
+          const int i = i0 + j * kSplitThreads;
+          if (i < m) {
+            const float h = __double2float_rn(v[j]);
+            hi[i] = h;
+            lo[i] = __double2float_rn(v[j] - (double)h);
           }
         }
       }
     }
+    if ((k += gridDim.x) >= a.nruns) break;
+    r = a.runs[k];
   }
 }
 
@@ -596,10 +598,7 @@ template void launch_compact_geometry<float>(const CompactGeoArgs<float> &, cuda
 template void launch_compact_geometry<double>(const CompactGeoArgs<double> &, cudaStream_t);
 
 void launch_split_join(const SplitJoinArgs &a, cudaStream_t st) {
-  const int64_t runs = (a.most + kSplitRun - 1) / kSplitRun;
-  const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(runs, 1 << 20)),
-                  (unsigned)std::min(a.npart, 65535));
-  launch_pdl(split_join_kernel, grid, kSplitThreads, 0, st, a);
+  if (a.nruns > 0) launch_pdl(split_join_kernel, std::min(a.nruns, 1 << 20), kSplitThreads, 0, st, a);
 }
 
 }  // namespace dgk

@@ -917,10 +917,9 @@ struct MixedOp : Op {
 
 // State split u (float64) -> uhi + ulo (float32 pair) and the join back, per partition.
 struct SplitJoinOp : Op {
-  int join;
-  int64_t most = 0;
+  int join, nruns = 0;
   Binding *u, *hi, *lo;
-  DevBuf cnt, uo, ho, lo_off;
+  DevBuf runs;
   SplitJoinOp(Runner &r, Roles &R, int j) : join(j) {
     u = R.array("u");
     hi = R.array("uhi");
@@ -929,25 +928,21 @@ struct SplitJoinOp : Op {
     require(hi->dev_dtype == DGK_FLOAT32, R.kname + ": uhi must be float32 on the device");
     same_layout(*hi, *lo, R.kname);
     require(u->values_per_elem == hi->values_per_elem, R.kname + ": u and uhi must hold the same values per element");
-    std::vector<int64_t> c((size_t)r.npart);
+    std::vector<SplitRun> l;
     for (int p = 0; p < r.npart; ++p) {
-      c[(size_t)p] = r.K[p] * hi->values_per_elem;
-      most = std::max(most, c[(size_t)p]);
+      const int64_t n = r.K[p] * hi->values_per_elem;
+      for (int64_t f = 0; f < n; f += kSplitRunValues)
+        l.push_back({u->offsets[p] + f, hi->offsets[p] + f, lo->offsets[p] + f,
+                     (int32_t)std::min<int64_t>(kSplitRunValues, n - f)});
     }
-    cnt.upload(c.data(), c.size() * sizeof(int64_t));
-    uo.upload(u->offsets.data(), sizeof(int64_t) * r.npart);
-    ho.upload(hi->offsets.data(), sizeof(int64_t) * r.npart);
-    lo_off.upload(lo->offsets.data(), sizeof(int64_t) * r.npart);
+    nruns = (int)l.size();
+    runs.upload(l.data(), l.size() * sizeof(SplitRun));
   }
   void launch(Runner &r, const std::vector<double> &) override {
     SplitJoinArgs a{};
-    a.npart = r.npart;
+    a.runs = runs.get<SplitRun>();
+    a.nruns = nruns;
     a.join = join;
-    a.count = cnt.get<int64_t>();
-    a.most = most;
-    a.u_off = uo.get<int64_t>();
-    a.hi_off = ho.get<int64_t>();
-    a.lo_off = lo_off.get<int64_t>();
     a.u = reinterpret_cast<double *>(u->dptr);
     a.hi = reinterpret_cast<float *>(hi->dptr);
     a.lo = reinterpret_cast<float *>(lo->dptr);
