@@ -9,10 +9,11 @@ Timing runs stage 0 of the LSERK4 scheme with dt = 0 from a step boundary: the r
 state is rewritten unchanged, so tuning leaves the solution where it was (the next real stage 0 ignores the
 residual).  Every candidate computes the same arithmetic per element, so the choice changes speed only.
 
-Candidates of the mixed stage: its FP32-FMA form with 4, 8 or 11 consumer warps per CTA and a ring of as many
+Candidates of the mixed stage: the operator's own choice (on small problems the form with a matrix row per thread,
+else 11 consumer warps and a full ring), its slot form with 4, 8 or 11 consumer warps per CTA and a ring of as many
 slots as shared memory holds, or 6; and, at orders 1..4, its tensor-core form with 2 or 4 threads per element
-(8 or 16 consumer warps).  The two forms round differently (both within the mixed stage's error bound); launch
-shapes of one form give the same bits.  The plain stages have one launch shape per order and are not tuned.
+(8 or 16 consumer warps).  The tensor-core form rounds differently (both within the mixed stage's error bound);
+the others give the same bits.  The plain stages have one launch shape per order and are not tuned.
 """
 from __future__ import annotations
 
@@ -23,7 +24,9 @@ from typing import Callable, Dict, List, Optional
 
 from .burgers import RK4B
 
-MIXED_CANDIDATES: List[Dict] = [{"warps": w, "ring": r, "mma": False} for w in (11, 8, 4) for r in (None, 6)]
+DEFAULT_SHAPE: Dict = {"warps": None, "ring": None, "mma": False}
+MIXED_CANDIDATES: List[Dict] = [DEFAULT_SHAPE] + [{"warps": w, "ring": r, "mma": False} for w in (11, 8, 4)
+                                                  for r in (None, 6) if (w, r) != (11, None)]
 TCM_CANDIDATES: List[Dict] = [{"warps": w, "ring": None, "mma": True} for w in (16, 8)]
 
 
@@ -77,6 +80,15 @@ def search(candidates: List[Dict], measure: Callable[[Dict], float]) -> tuple:
     return best, times
 
 
+def current(entry: dict) -> bool:
+    """Whether a cached choice still names what was timed: entries from before the operator's own choice was a
+    candidate may hold a number of warps that was timed as the row form, which an explicit number does not select."""
+    best = entry["best"]
+    if best.get("mma") or best.get("ring") or not best.get("warps"):
+        return True
+    return json.dumps(DEFAULT_SHAPE, sort_keys=True) in entry.get("ms_per_stage", {})
+
+
 def _device_name() -> str:
     try:
         import torch
@@ -96,7 +108,7 @@ def autotune(problem, cache_path: Optional[str] = None, stages: int = 8, candida
     path = cache_path or default_cache_path()
     cache = load_cache(path)
     key = problem_key(_device_name(), "rhsStageMixed", problem.N, problem.dofs, len(problem.Kpart))
-    if not force and key in cache:
+    if not force and key in cache and current(cache[key]):
         best = cache[key]["best"]
         problem.build_stage(**best)
         return best

@@ -491,7 +491,7 @@ struct MatmulOp : Op {
 // matrices Dr, Ds, Dt, LIFT, Fmask and Bary (Np x 4 barycentric coordinates of the nodes).
 struct MixedOp : Op {
   int N = 0, ntiles = 0, conservative = 0, ncodes = 0, warps = 11, ring = 0, tensor = 0, mma = 0;
-  bool rows = false;  // the form with a matrix row per thread (warps has no meaning there, a ring depth asks for the other)
+  bool rows = false;  // the form with a matrix row per thread; a launch shape (warps or ring) asks for the other
   Binding *uhi, *ulo, *uhin, *ulon, *resu;
   DevBuf gown, tiles, geoE, conn, dm, lift, bary, vtx, ftab, fmask, amat, rexp, bmat;
   DevBuf tconn, hoff, hlist;  // tensor-core form: tile-local connectivity and the tiles' halo lists
@@ -677,7 +677,7 @@ struct MixedOp : Op {
       tcm_pack_operands(N, Dr->mat.data(), Ds->mat.data(), Dt->mat.data(), L->mat.data(), packed);
       bmat.upload(packed.data(), packed.size() * sizeof(uint16_t));
     }
-    rows = !tensor && !mma && ring == 0 && rows_faster(N, r.ktotal, r.num_sms);
+    rows = !tensor && !mma && ring == 0 && !R.explicit_.count("warps") && rows_faster(N, r.ktotal, r.num_sms);
     if (rows) gown.upload(gm.data(), gm.size() * sizeof(int32_t));  // the map as it is now, like the compact form
     const int te = tensor ? oz_tile_elems() : rows ? rows_tile_elems(N) : kMixedSlotElems;
     std::vector<MTile> tl;
