@@ -62,17 +62,19 @@ __device__ __forceinline__ int64_t slot_of_value(const LsArgs &A, int64_t g, int
   return -1;
 }
 
-// The network's inputs as FP16 pairs: x 2^10 = hi + lo, both rounded to nearest (|x| <= 1: a unit-norm feature or a
-// tanh; the scale keeps the low part out of FP16's subnormals for all but the smallest inputs), and one m16n8k16
-// product accumulated into d.
-constexpr float kLsScale = 1024.f;
+// The network's inputs as FP16 pairs: x 2^15 = hi + lo 2^-11, both rounded to nearest (|x| <= 1: a unit-norm feature or a
+// tanh).  The largest error is 1.2e-7 of x down to x = 2e-9, what a pair of TF32 parts has, and 4.4e-16 below, where the
+// state's pair and the modal transform carry x no further: the scales keep both parts out of FP16's subnormals, which is
+// why the low products have sums of their own (both parts at 2^10: 2.9e-6 of x at 1e-5 and 2.9e-3 at 1e-8).
+constexpr float kLsScale = 32768.f, kLsLow = 2048.f;
 __device__ __forceinline__ void ls_put(__half *row, int lo_off, float x) {
   const float v = x * kLsScale;
   const __half h = __float2half_rn(v);
   row[0] = h;
-  row[lo_off] = __float2half_rn(v - __half2float(h));
+  row[lo_off] = __float2half_rn((v - __half2float(h)) * kLsLow);
 }
 
+// one m16n8k16 product accumulated into d
 __device__ __forceinline__ void ls_mma_f16(float (&d)[4], const uint4 &a, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
                "{%0,%1,%2,%3};"
@@ -112,6 +114,7 @@ struct LsSensorSmem {
 // parts lie `lo` words behind
 template <int K>
 __device__ __forceinline__ void ls_layer(const uint4 *w, const uint32_t *x, int lo, float (&o)[2][4]) {
+  float ol[2][4] = {};  // the low parts' sums, 2^11 times their share
 #pragma unroll
   for (int kk = 0; kk < K; ++kk) {
     const uint32_t h0 = x[8 * kk], h1 = x[8 * kk + 4], l0 = x[lo + 8 * kk], l1 = x[lo + 8 * kk + 4];
@@ -119,9 +122,13 @@ __device__ __forceinline__ void ls_layer(const uint4 *w, const uint32_t *x, int 
     for (int mt = 0; mt < 2; ++mt) {
       const uint4 a = w[(kk * 2 + mt) * 32];
       ls_mma_f16(o[mt], a, h0, h1);
-      ls_mma_f16(o[mt], a, l0, l1);
+      ls_mma_f16(ol[mt], a, l0, l1);
     }
   }
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int f = 0; f < 4; ++f) o[mt][f] = fmaf(ol[mt][f], 1.f / kLsLow, o[mt][f]);
 }
 
 template <int N>
