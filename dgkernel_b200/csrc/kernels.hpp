@@ -27,7 +27,7 @@ void launch_update(const Tile *tiles, int ntiles, int np, T *u, T *resu, const T
 int tile_elems(int N);
 // Form with TMA streaming and the element-local products on the FP64 tensor path (kernels_tma.cu), orders 1..5.
 template <typename T>
-bool launch_rhs_dmma(int N, const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info);
+void launch_rhs_dmma(int N, const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info);
 template <typename T>
 int dmma_tile_elems(int N);  // 0 when the order has no such form
 // Form of orders 6 and 7 with the matrices streamed in fragment order (kernels_wide.cu).  wide_pack lays out

@@ -502,15 +502,14 @@ __global__ void __launch_bounds__(DmmaCfg<N, CP, T>::THREADS, DmmaCfg<N, CP, T>:
 }
 
 template <int N, bool CP, typename T>
-static bool dmma_launch_n(const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info) {
+static void dmma_launch_n(const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info) {
   using C = DmmaCfg<N, CP, T>;
-  if (C::SMEM > 227 * 1024) return false;
+  static_assert(C::SMEM <= 227 * 1024, "every order has the form");
   auto k = rhs_stage_dmma_kernel<N, CP, T>;
   const int per = resident_ctas(k, C::THREADS, C::SMEM, info);
   const int grid = std::min(A.ntiles, per * num_sms);
   if (info) *info = {grid, C::THREADS, (int)C::SMEM, per};
   if (grid > 0) launch_pdl(k, grid, C::THREADS, C::SMEM, st, A, rhs_only);
-  return true;
 }
 
 // Compact FP64 geometry of the compact form: per element slot the node-0 metrics and, per face, the first face
@@ -555,46 +554,39 @@ void launch_compact_geo64(const CompactGeoArgs<double> &g, double *out, cudaStre
   cuda_check(cudaGetLastError(), "compact_geo64_kernel launch");
 }
 
-template <typename T>
-bool launch_rhs_dmma(int N, const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info) {
-  if constexpr (std::is_same<T, double>::value)
-    if (A.geoc) switch (N) {
-        case 1: return dmma_launch_n<1, true, T>(A, rhs_only, num_sms, st, info);
-        case 2: return dmma_launch_n<2, true, T>(A, rhs_only, num_sms, st, info);
-        case 3: return dmma_launch_n<3, true, T>(A, rhs_only, num_sms, st, info);
-        case 4: return dmma_launch_n<4, true, T>(A, rhs_only, num_sms, st, info);
-        case 5: return dmma_launch_n<5, true, T>(A, rhs_only, num_sms, st, info);
-        default: return false;
-      }
+template <bool CP, typename T>
+static void dmma_launch(int N, const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info) {
   switch (N) {
-    case 1: return dmma_launch_n<1, false, T>(A, rhs_only, num_sms, st, info);
-    case 2: return dmma_launch_n<2, false, T>(A, rhs_only, num_sms, st, info);
-    case 3: return dmma_launch_n<3, false, T>(A, rhs_only, num_sms, st, info);
-    case 4: return dmma_launch_n<4, false, T>(A, rhs_only, num_sms, st, info);
-    case 5: return dmma_launch_n<5, false, T>(A, rhs_only, num_sms, st, info);
-    default: return false;
+    case 1: dmma_launch_n<1, CP, T>(A, rhs_only, num_sms, st, info); break;
+    case 2: dmma_launch_n<2, CP, T>(A, rhs_only, num_sms, st, info); break;
+    case 3: dmma_launch_n<3, CP, T>(A, rhs_only, num_sms, st, info); break;
+    case 4: dmma_launch_n<4, CP, T>(A, rhs_only, num_sms, st, info); break;
+    case 5: dmma_launch_n<5, CP, T>(A, rhs_only, num_sms, st, info); break;
+    default: throw Error(DGK_ERR_UNSUPPORTED, "stage on the FP64 tensor path: orders 1..5");
   }
 }
 
-template <int N, typename T>
-static int dmma_te() {
-  return DmmaCfg<N, false, T>::SMEM <= 227 * 1024 ? DmmaCfg<N, false, T>::TE : 0;
+template <typename T>
+void launch_rhs_dmma(int N, const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info) {
+  if constexpr (std::is_same<T, double>::value)
+    if (A.geoc) return dmma_launch<true, T>(N, A, rhs_only, num_sms, st, info);
+  dmma_launch<false, T>(N, A, rhs_only, num_sms, st, info);
 }
 
 template <typename T>
 int dmma_tile_elems(int N) {
   switch (N) {
-    case 1: return dmma_te<1, T>();
-    case 2: return dmma_te<2, T>();
-    case 3: return dmma_te<3, T>();
-    case 4: return dmma_te<4, T>();
-    case 5: return dmma_te<5, T>();
+    case 1: return DmmaShape<1, T>::TE;
+    case 2: return DmmaShape<2, T>::TE;
+    case 3: return DmmaShape<3, T>::TE;
+    case 4: return DmmaShape<4, T>::TE;
+    case 5: return DmmaShape<5, T>::TE;
     default: return 0;
   }
 }
 
-template bool launch_rhs_dmma<double>(int, const RhsArgs<double> &, int, int, cudaStream_t, LaunchInfo *);
-template bool launch_rhs_dmma<float>(int, const RhsArgs<float> &, int, int, cudaStream_t, LaunchInfo *);
+template void launch_rhs_dmma<double>(int, const RhsArgs<double> &, int, int, cudaStream_t, LaunchInfo *);
+template void launch_rhs_dmma<float>(int, const RhsArgs<float> &, int, int, cudaStream_t, LaunchInfo *);
 template int dmma_tile_elems<double>(int);
 template int dmma_tile_elems<float>(int);
 
