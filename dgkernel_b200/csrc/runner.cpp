@@ -517,7 +517,13 @@ static std::vector<double> resolve_scalars(KernelConfig &cfg, int nscalars, cons
   }
   std::vector<double> vals(cfg.scalar_at.size());
   for (size_t k = 0; k < vals.size(); ++k) {
-    const int at = cfg.scalar_at[k];
+    int at = cfg.scalar_at[k];
+    // a scalar that is listed more than once takes the last of its places that has a value
+    while (at >= 0 && at >= nscalars && !cfg.scalars[(size_t)at]->scalar_bound) {
+      const Binding *b = cfg.scalars[(size_t)at];
+      do --at;
+      while (at >= 0 && cfg.scalars[(size_t)at] != b);
+    }
     if (at >= 0 && cfg.scalars[(size_t)at]->scalar_bound)
       vals[k] = cfg.scalars[(size_t)at]->scalar_value;
     else if (at >= 0 && at < nscalars)
