@@ -166,23 +166,23 @@ __device__ __forceinline__ void prefetch_tile(const RhsArgs<T> &A, const Tile &t
 }
 
 // Shared-memory carve-up of the fused kernels.
-template <typename T, int N, bool MSMEM>
+template <typename T, int N>
 struct Smem {
   using O = Order<N>;
   using C = Cfg<N>;
-  static constexpr int DM = MSMEM ? 3 * O::NP * Pad<O::NP>::V : 0;
-  static constexpr int LM = MSMEM ? O::NP * Pad<O::NF>::V : 0;
+  static constexpr int DM = 3 * O::NP * Pad<O::NP>::V;
+  static constexpr int LM = O::NP * Pad<O::NF>::V;
   static constexpr int U = C::TE * O::NPS;
   static constexpr int D3 = 3 * C::TE * O::NPS;
   static constexpr int F = C::TE * O::NFS;
   static constexpr size_t bytes = sizeof(T) * (size_t)(DM + LM + U + D3 + F) + sizeof(int) * O::NF;
 };
 
-template <typename T, int N, bool MSMEM>
+template <typename T, int N>
 __global__ void __launch_bounds__(Cfg<N>::THREADS, 2) rhs_stage_kernel(RhsArgs<T> A, int rhs_only) {
   using O = Order<N>;
   using C = Cfg<N>;
-  using S = Smem<T, N, MSMEM>;
+  using S = Smem<T, N>;
   constexpr int NP = O::NP, NF = O::NF, NPS = O::NPS, NFS = O::NFS, TE = C::TE, RG = C::RG;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *sD = reinterpret_cast<T *>(smem_raw);
@@ -193,13 +193,11 @@ __global__ void __launch_bounds__(Cfg<N>::THREADS, 2) rhs_stage_kernel(RhsArgs<T
   int *sfm = reinterpret_cast<int *>(sf + S::F);
   const int tid = threadIdx.x, nth = C::THREADS;  // launched with exactly Cfg<N>::THREADS threads
   if (tid == 0 && blockIdx.x < A.ntiles) prefetch_tile(A, A.tiles[blockIdx.x], NP, NF);
-  if (MSMEM) {  // the operator stores both matrices with the padded row strides used here
-    for (int i = tid; i < S::DM; i += nth) sD[i] = A.Dmat[i];
-    for (int i = tid; i < S::LM; i += nth) sL[i] = A.LIFT[i];
-  }
+  // the operator stores both matrices with the padded row strides used here
+  for (int i = tid; i < S::DM; i += nth) sD[i] = A.Dmat[i];
+  for (int i = tid; i < S::LM; i += nth) sL[i] = A.LIFT[i];
   for (int i = tid; i < NF; i += nth) sfm[i] = A.fmask[i];
-  const T *Dm = MSMEM ? sD : A.Dmat;
-  const T *Lm = MSMEM ? sL : A.LIFT;
+  const T *Dm = sD, *Lm = sL;
   const int e_own = tid % TE, g_own = tid / TE;
   const T a = A.a, b = A.b, dt = A.dt;
   __syncthreads();
@@ -414,11 +412,6 @@ __global__ void update_kernel(const Tile *tiles, int ntiles, int np, T *u, T *re
 // ------------------------------------------------------------------------------------------------
 // host launchers
 // ------------------------------------------------------------------------------------------------
-template <typename T, int N>
-static bool mats_fit() {
-  return Smem<T, N, true>::bytes <= 200 * 1024;
-}
-
 template <typename K>
 static int resident(K kernel, int threads, size_t smem) {
   cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
@@ -430,21 +423,13 @@ static int resident(K kernel, int threads, size_t smem) {
 template <typename T, int N>
 static void rhs_launch_n(const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStream_t st, LaunchInfo *info) {
   const int threads = Cfg<N>::THREADS;
-  if (mats_fit<T, N>()) {
-    auto k = rhs_stage_kernel<T, N, true>;
-    const size_t sm = Smem<T, N, true>::bytes;
-    const int per = std::max(1, resident(k, threads, sm));
-    const int grid = std::min(A.ntiles, per * num_sms);
-    if (info) *info = {grid, threads, (int)sm, per};
-    if (grid > 0) k<<<grid, threads, sm, st>>>(A, rhs_only);
-  } else {
-    auto k = rhs_stage_kernel<T, N, false>;
-    const size_t sm = Smem<T, N, false>::bytes;
-    const int per = std::max(1, resident(k, threads, sm));
-    const int grid = std::min(A.ntiles, per * num_sms);
-    if (info) *info = {grid, threads, (int)sm, per};
-    if (grid > 0) k<<<grid, threads, sm, st>>>(A, rhs_only);
-  }
+  auto k = rhs_stage_kernel<T, N>;
+  constexpr size_t sm = Smem<T, N>::bytes;
+  static_assert(sm <= 227 * 1024, "the matrices fit shared memory at every order");
+  const int per = std::max(1, resident(k, threads, sm));
+  const int grid = std::min(A.ntiles, per * num_sms);
+  if (info) *info = {grid, threads, (int)sm, per};
+  if (grid > 0) k<<<grid, threads, sm, st>>>(A, rhs_only);
 }
 
 template <typename T>
@@ -480,7 +465,7 @@ int tile_elems(int N) {
     case 3: return Cfg<3>::TE;
     case 4: return Cfg<4>::TE;
     case 5: return Cfg<5>::TE;
-    default: throw Error(DGK_ERR_UNSUPPORTED, "order N must be 1..7");
+    default: throw Error(DGK_ERR_UNSUPPORTED, "order N must be 1..5");
   }
 }
 

@@ -31,10 +31,6 @@ namespace {
 constexpr int kLsHid = 32;
 constexpr int kLsWarps = 8;  // sensor pass: warps per block, 8 elements each at a time
 
-__host__ __device__ constexpr int ls_mlp_params(int nin) {
-  return kLsHid * nin + kLsHid + kLsHid * kLsHid + kLsHid + kLsHid + 1;
-}
-
 __device__ __forceinline__ double ls_pp_sigma(double S, double s0, double kappa) {
   if (!(S >= s0 - kappa)) return 0.0;
   if (S > s0 + kappa) return 1.0;
