@@ -14,12 +14,14 @@
 // 330 per node at order 3 against mixed.cu's 150) once every SM is busy.  The lines of rows_faster follow from stages in
 // a captured graph, us, mixed.cu / here:
 //   elements    order 1      order 2      order 3      order 4
-//        384    4.0 / 2.3    6.6 / 2.7    9.7 / 3.3   19.1 / 6.0
-//       6000    5.6 / 2.5    8.3 / 3.5   12.0 / 6.8   22.0 / 10.7
-//      16464    6.6 / 2.9    9.3 / 5.6   12.6 / 10.6  22.4 / 20.6
-//      29478    8.5 / 3.0   11.4 / 7.6   15.3 / 15.6  28.4 / 33.2
-//      48000   10.7 / 4.4   14.0 / 10.5  19.9 / 23.0  36.0 / 50.4
-//     131712   21.0 / 8.1   25.7 / 23.7  41.9 / 58.1  86.4 / 128.3
+//        384    4.0 / 2.1    6.4 / 2.7    9.7 / 3.1   19.1 / 5.9
+//       6000    5.5 / 2.3    8.3 / 3.8   12.0 / 6.6   21.9 / 10.7
+//      16464    6.6 / 2.9    9.3 / 6.2   12.6 / 10.5  22.4 / 20.6
+//      29478    8.3 / 2.9   11.3 / 8.0   15.2 / 15.4  28.2 / 33.0
+//      48000   10.7 / 4.3   14.0 / 10.7  19.9 / 22.8  36.0 / 50.2
+//     131712   21.0 / 8.2   25.7 / 23.8  41.8 / 57.5  86.5 / 127.3
+//     196608                35.5 / 34.7
+//     384000   55.2 / 19.6  82.1 / 68.0
 #include <algorithm>
 #include <cstdint>
 
@@ -276,7 +278,9 @@ int rows_tile_elems(int N) {
   }
 }
 
-// Elements per SM up to which this form is the faster one (see the table above; order 2 by the slopes of its columns).
+// Elements per SM up to which this form is taken (148 SMs; the table above).  Orders 3 and 4 lie near their crossings (order
+// 3: 28,950 elements 15.2 / 15.3; order 4: 16,464 22.4 / 20.6, 29,478 28.2 / 33.0).  At order 2 it is ahead on either
+// side of the line (189,114 elements 34.3 / 33.3, 196,608 35.5 / 34.7), which could lie higher.
 bool rows_faster(int N, int64_t nelems, int num_sms) {
   switch (N) {
     case 1: return true;
