@@ -375,35 +375,36 @@ __global__ void __launch_bounds__(Cfg<N>::THREADS, 2) rhs_stage_kernel(RhsArgs<T
   }
 }
 
-// Elementwise updates over tiles: mode 0 = the reference's updateSolution
+// Elementwise updates over runs of kUpdateValues values: mode 0 = the reference's updateSolution
 // (resu = rka*resu + rkb*rhsu; u += resu), mode 1 = standard LSERK4 (resu = a*resu + dt*rhs; u += b*resu).
-// Bound by HBM; a thread's loads are issued four values at a time.
+// Bound by HBM: a run is four loads of each array per thread, all in flight, and a block of its own, so that every block
+// has a full run whatever the values per element (16 M values: FP64 96.5 us, 6.6 TB/s; FP32 51.3).  Tiles of 64 elements
+// held a quarter of those loads at 4 values per element (FP64 154 us, FP32 136) and ragged tails at others (35: 111 and
+// 68); runs walked by a grid of eight blocks an SM take 106 and 54.
 template <typename T>
-__global__ void update_kernel(const Tile *tiles, int ntiles, int np, T *u, T *resu, const T *rhs, T c0, T c1, T c2,
-                              int mode) {
-  constexpr int CH = 4;
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const Tile tl = tiles[t];
-    const int n = tl.nelem * np;
-    for (int x0 = threadIdx.x; x0 < n; x0 += CH * blockDim.x) {
-      T r[CH], v[CH], w[CH];
+__global__ void __launch_bounds__(kUpdateThreads) update_kernel(const Tile *runs, int nruns, T *u, T *resu, const T *rhs,
+                                                                T c0, T c1, T c2, int mode) {
+  constexpr int CH = kUpdateValues / kUpdateThreads;
+  for (int t = blockIdx.x; t < nruns; t += gridDim.x) {
+    const Tile run = runs[t];
+    const int n = run.nelem;
+    T *pr = resu + run.node_base, *pu = u + run.node_base;
+    const T *pw = rhs + run.node_base;
+    T r[CH], v[CH], w[CH];
 #pragma unroll
-      for (int j = 0; j < CH; ++j) {
-        const int x = x0 + j * blockDim.x;
-        const int64_t gi = tl.node_base + x;
-        r[j] = x < n ? resu[gi] : T(0);
-        v[j] = x < n ? u[gi] : T(0);
-        w[j] = x < n ? rhs[gi] : T(0);
-      }
+    for (int j = 0; j < CH; ++j) {
+      const int x = threadIdx.x + j * kUpdateThreads;
+      r[j] = x < n ? pr[x] : T(0);
+      v[j] = x < n ? pu[x] : T(0);
+      w[j] = x < n ? pw[x] : T(0);
+    }
 #pragma unroll
-      for (int j = 0; j < CH; ++j) {
-        const int x = x0 + j * blockDim.x;
-        const int64_t gi = tl.node_base + x;
-        if (x < n) {
-          const T res = mode == 0 ? c0 * r[j] + c1 * w[j] : c0 * r[j] + c2 * w[j];
-          resu[gi] = res;
-          u[gi] = mode == 0 ? v[j] + res : v[j] + c1 * res;
-        }
+    for (int j = 0; j < CH; ++j) {
+      const int x = threadIdx.x + j * kUpdateThreads;
+      if (x < n) {
+        const T res = mode == 0 ? c0 * r[j] + c1 * w[j] : c0 * r[j] + c2 * w[j];
+        pr[x] = res;
+        pu[x] = mode == 0 ? v[j] + res : v[j] + c1 * res;
       }
     }
   }
@@ -445,18 +446,18 @@ void launch_rhs(int N, const RhsArgs<T> &A, int rhs_only, int num_sms, cudaStrea
 }
 
 template <typename T>
-void launch_update(const Tile *tiles, int ntiles, int np, T *u, T *resu, const T *rhs, double c0, double c1, double c2,
-                   int mode, int num_sms, cudaStream_t st) {
-  const int grid = std::min(ntiles, num_sms * 8);
-  if (grid > 0) update_kernel<T><<<grid, 256, 0, st>>>(tiles, ntiles, np, u, resu, rhs, (T)c0, (T)c1, (T)c2, mode);
+void launch_update(const Tile *runs, int nruns, T *u, T *resu, const T *rhs, double c0, double c1, double c2, int mode,
+                   cudaStream_t st) {
+  const int grid = std::min(nruns, 1 << 20);
+  if (grid > 0) update_kernel<T><<<grid, kUpdateThreads, 0, st>>>(runs, nruns, u, resu, rhs, (T)c0, (T)c1, (T)c2, mode);
 }
 
 template void launch_rhs<double>(int, const RhsArgs<double> &, int, int, cudaStream_t, LaunchInfo *);
 template void launch_rhs<float>(int, const RhsArgs<float> &, int, int, cudaStream_t, LaunchInfo *);
-template void launch_update<double>(const Tile *, int, int, double *, double *, const double *, double, double, double,
-                                    int, int, cudaStream_t);
-template void launch_update<float>(const Tile *, int, int, float *, float *, const float *, double, double, double, int,
-                                   int, cudaStream_t);
+template void launch_update<double>(const Tile *, int, double *, double *, const double *, double, double, double, int,
+                                    cudaStream_t);
+template void launch_update<float>(const Tile *, int, float *, float *, const float *, double, double, double, int,
+                                    cudaStream_t);
 
 int tile_elems(int N) {
   switch (N) {

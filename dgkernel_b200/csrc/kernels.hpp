@@ -21,9 +21,11 @@ void launch_diff(int N, const DiffArgs<T> &A, int num_sms, cudaStream_t st, Laun
 int diff_tile_elems(int N);
 template <typename T>
 void launch_diff_wide(int N, int tile_elems, const DiffArgs<T> &A, int num_sms, cudaStream_t st, LaunchInfo *info);
+// runs: a run's first value (node_base) and count (nelem, at most kUpdateValues)
+constexpr int kUpdateThreads = 256, kUpdateValues = 4 * kUpdateThreads;
 template <typename T>
-void launch_update(const Tile *tiles, int ntiles, int np, T *u, T *resu, const T *rhs, double c0, double c1, double c2,
-                   int mode, int num_sms, cudaStream_t st);
+void launch_update(const Tile *runs, int nruns, T *u, T *resu, const T *rhs, double c0, double c1, double c2, int mode,
+                   cudaStream_t st);
 int tile_elems(int N);
 // Form with TMA streaming and the element-local products on the FP64 tensor path (kernels_tma.cu), orders 1..5.
 template <typename T>

@@ -428,29 +428,36 @@ struct RhsOp : Op {
 // Elementwise updates: the reference's updateSolution (mode 0) and the LSERK4 recurrence (mode 1).
 template <typename T>
 struct UpdateOp : Op {
-  int mode, ntiles;
-  int64_t np;
+  int mode, nruns;
   Binding *u, *resu, *rhs;
-  DevBuf tiles;
+  DevBuf runs;
   UpdateOp(Runner &r, Roles &R, int m) : mode(m) {
     u = R.array("u");
     resu = R.array("resu");
     rhs = R.array(mode == 0 ? "rhsu" : "rhs");
     same_layout(*u, *resu, R.kname);
     same_layout(*u, *rhs, R.kname);
-    np = std::max<int64_t>(1, u->values_per_elem);
-    auto tl = make_tiles(r, *u, nullptr, 64, (int)np, 0);
-    ntiles = (int)tl.size();
-    tiles.upload(tl.data(), tl.size() * sizeof(Tile));
+    const int64_t np = std::max<int64_t>(1, u->values_per_elem);
+    std::vector<Tile> l;  // runs of values: a block's four loads per thread each, whatever the values per element
+    for (int p = 0; p < r.npart; ++p) {
+      const int64_t n = r.K[p] * np;
+      for (int64_t f = 0; f < n; f += kUpdateValues) {
+        Tile x{};
+        x.node_base = u->offsets[p] + f;
+        x.nelem = (int32_t)std::min<int64_t>(kUpdateValues, n - f);
+        l.push_back(x);
+      }
+    }
+    nruns = (int)l.size();
+    runs.upload(l.data(), l.size() * sizeof(Tile));
   }
   std::vector<std::string> scalar_names() const override {
     if (mode == 0) return {"rka", "rkb"};
     return {"a", "b", "dt"};
   }
   void launch(Runner &r, const std::vector<double> &s) override {
-    launch_update<T>(tiles.get<Tile>(), ntiles, (int)np, reinterpret_cast<T *>(u->dptr),
-                     reinterpret_cast<T *>(resu->dptr), reinterpret_cast<const T *>(rhs->dptr), s[0], s[1],
-                     mode == 0 ? 0.0 : s[2], mode, r.num_sms, r.stream());
+    launch_update<T>(runs.get<Tile>(), nruns, reinterpret_cast<T *>(u->dptr), reinterpret_cast<T *>(resu->dptr),
+                     reinterpret_cast<const T *>(rhs->dptr), s[0], s[1], mode == 0 ? 0.0 : s[2], mode, r.stream());
   }
 };
 
