@@ -56,6 +56,13 @@ struct RowSmem {
   float hi[2][C::TE * C::NP];
 };
 
+// The field whose derivative is taken: u or u^2/2, rounded by itself (a product that the compiler may merge with the
+// subtraction after it would leave mixed.cu's bits, whose form is chosen at run time).
+template <bool CONS>
+__device__ __forceinline__ double row_w(double u) {
+  return CONS ? __dmul_rn(0.5 * u, u) : u;
+}
+
 template <int N, bool CONS>
 __global__ void __launch_bounds__(RowCfg<N>::THREADS, RowCfg<N>::MINB) rhs_stage_rows_kernel(const MixedArgs A) {
   using C = RowCfg<N>;
@@ -169,11 +176,8 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS, RowCfg<N>::MINB) rhs_stage
       const double *ue = m.u[p] + e * NP;
       const float *ge = m.geo[p] + e * kMixedGeoWords, *he = m.hi[p] + e * NP;
       const double uA = ue[vA], uB = ue[vB], uC = ue[vC], uD = ue[vD];
-      const double wA = CONS ? 0.5 * uA * uA : uA;
-      const double dB = (CONS ? 0.5 * uB * uB : uB) - wA;
-      const double dC = (CONS ? 0.5 * uC * uC : uC) - wA;
-      const double dD = (CONS ? 0.5 * uD * uD : uD) - wA;
-      const double w = CONS ? 0.5 * u[g] * u[g] : u[g];
+      const double wA = row_w<CONS>(uA), w = row_w<CONS>(u[g]);
+      const double dB = row_w<CONS>(uB) - wA, dC = row_w<CONS>(uC) - wA, dD = row_w<CONS>(uD) - wA;
       if (lives) m.dw[p][e * NPJ + i] = (float)((w - wA) - (b1 * dB + b2 * dC + b3 * dD));
 #pragma unroll
       for (int j = 0; j < NJ; ++j) {
@@ -188,10 +192,8 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS, RowCfg<N>::MINB) rhs_stage
       // derivative of the linear part along (1,1,1), one thread per element: d/dr = (wB-wA)/2 and likewise for s, t
       const double *ue = m.u[p] + tid * NP;
       float *ge = m.geo[p] + tid * kMixedGeoWords;
-      const double wA = CONS ? 0.5 * ue[vA] * ue[vA] : ue[vA];
-      const double dB = (CONS ? 0.5 * ue[vB] * ue[vB] : ue[vB]) - wA;
-      const double dC = (CONS ? 0.5 * ue[vC] * ue[vC] : ue[vC]) - wA;
-      const double dD = (CONS ? 0.5 * ue[vD] * ue[vD] : ue[vD]) - wA;
+      const double wA = row_w<CONS>(ue[vA]);
+      const double dB = row_w<CONS>(ue[vB]) - wA, dC = row_w<CONS>(ue[vC]) - wA, dD = row_w<CONS>(ue[vD]) - wA;
       ge[7] = (float)(0.5 * ((double)ge[0] * dB + (double)ge[1] * dC + (double)ge[2] * dD));
     }
     __syncthreads();
