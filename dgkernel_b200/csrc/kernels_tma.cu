@@ -26,7 +26,7 @@ namespace dgk {
 // FP64's): 1.1 G FMAs a stage at order 4 and 32^3 x 6 are 62 us at the FP64 rate, under the 91 us of its bytes, where
 // the FP32 cores need a shared-memory matrix entry per FMA.  Flux, metrics and update stay in FP32.  Their tiles hold two
 // n-tiles per warp from order 3 on: the barriers and waits of a tile then serve 16 elements.
-// Order 4, 32^3 x 6: 187 us a stage from 247 with the register-staged form on the FP32 cores.
+// Order 4, 32^3 x 6: 182 us a stage from 247 with the register-staged form on the FP32 cores.
 //
 // The products OUT = M * U of a tile are small GEMMs: M is NP x NP (Dr, Ds, Dt) or NP x NF (LIFT), U holds
 // the TE element vectors of the tile as columns.  Warp w owns rows 8w..8w+7 (one m-tile) of every matrix
@@ -696,7 +696,7 @@ __global__ void __launch_bounds__(DiffCfg<N, T>::THREADS, DiffCfg<N, T>::MINB) d
             __stcs(A.out[1] + gi, uy);
             __stcs(A.out[2] + gi, uz);
           } else {
-            __stcs(A.out[0] + gi, -su[o] * (ux + uy + uz));
+            A.out[0][gi] = -su[o] * (ux + uy + uz);  // not streamed: an update reads it next
           }
         }
       }

@@ -1,5 +1,5 @@
-// Fused strong-form Lax-Friedrichs RHS + LSERK4 stage at orders 6 and 7, arrays in FP64 or FP32 (ST), where the reference matrices (237 and
-// 483 KB) fit neither registers nor shared memory.
+// Fused strong-form Lax-Friedrichs RHS + LSERK4 stage at orders 6 and 7, arrays in FP64 or FP32 (T), where the reference
+// matrices (237 and 483 KB) fit neither registers nor shared memory.
 //
 // The products run on the FP64 tensor path (mma.sync m8n8k4) with the matrices streamed from L2: the operator stores
 // them in fragment order, so a warp's A fragment is 256 consecutive bytes, loaded two k-steps ahead and used for NT
@@ -8,9 +8,9 @@
 // of bank conflicts.  The nine metrics and four face arrays are read once, straight from global memory, 64 consecutive
 // bytes per element.  They are brought into L2 by bulk prefetches shortly before their phase: prefetched a whole tile
 // ahead, the CTAs' tiles together outgrow L2, and prefetched ahead of a phase that loads itself, they delay it (order 7,
-// 16^3 x 6: 1012 us per LSERK4 step a tile ahead, 860 as here, with NT = 4).  Several small CTAs share an SM and drift
-// apart, so one's memory phases run under another's products: three CTAs of 16 elements take
-// 775 us, two of 16 take 840 and two of 32 take 860.  Each warp owns one or two 8-row m-tiles.
+// 16^3 x 6, measured on tiles of 32 elements, a shape since removed: 1012 us per LSERK4 step a tile ahead, 860 as here).
+// Several small CTAs share an SM and drift apart, so one's memory phases run under another's products: three CTAs of 16
+// elements take 775 us, two of 16 take 840 and two of 32 take 860.  Each warp owns one or two 8-row m-tiles.
 //
 // Bound by the FP64 rate (60,480 FMAs per element at order 7, 82 us of the 155 us per stage) and by the latency of
 // the memory phases.  The form before it read a matrix entry per FMA through L1: 655 us per stage.
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(WideCfg<N, NT>::THREADS, WideCfg<N, NT>::MINB)
               __stcs(A.out[1] + gi, uy);
               __stcs(A.out[2] + gi, uz);
             } else {
-              __stcs(A.out[0] + gi, -(T)su[e * SU + row] * (ux + uy + uz));
+              A.out[0][gi] = -(T)su[e * SU + row] * (ux + uy + uz);  // not streamed: an update reads it next
             }
           }
         }
