@@ -1,4 +1,4 @@
-// Mixed-precision stage with a matrix row per thread: orders 1 and 2, and 3 and 4 while a problem is small (operator
+// Mixed-precision stage with a matrix row per thread: order 1, and orders 2..4 while a problem is small (operator
 // "rhsStageMixed"; the arithmetic is mixed.cu's, bit for bit: compensated pair state, products on the field minus its
 // linear vertex interpolant, flux and residual in FP32, update in FP64).
 //
@@ -13,18 +13,15 @@
 // tile's state is stored; its operands (field minus linear part, face terms) are.  Bound by its instruction count (about
 // 330 per node at order 3 against mixed.cu's 150) once every SM is busy.  The lines of rows_faster follow from stages in
 // a captured graph, us, mixed.cu / here:
-//   elements    order 1       order 2        order 3      order 4
-//        384    3.9 / 2.1     6.4 / 2.8      9.7 / 3.3   19.1 / 6.0
-//       6000    5.6 / 2.3     8.3 / 3.9     12.1 / 6.8   22.0 / 10.7
-//      16464    6.7 / 2.9     9.3 / 6.2     12.6 / 10.8  22.4 / 20.6
-//      24576    7.8 / 3.1    10.7 / 7.0     14.6 / 13.6  27.7 / 28.3
-//      29478    8.3 / 3.0    11.4 / 8.1     15.2 / 15.4  28.4 / 33.3
-//      48000   10.8 / 4.2    13.9 / 10.7    19.5 / 22.8  36.1 / 50.5
-//     131712   21.2 / 7.9    25.3 / 24.1    41.0 / 57.8  86.9 / 127.5
-//     196608   30.1 / 11.1   34.7 / 35.0
-//     384000   55.3 / 19.5   81.6 / 68.9
-//     663552    119 / 32.0    141 / 119.5
-//    1572864    303 / 77.2    325 / 280.1
+//   elements    order 1      order 2      order 3      order 4
+//        384    4.0 / 2.1    6.4 / 2.7    9.7 / 3.1   19.1 / 5.9
+//       6000    5.5 / 2.3    8.3 / 3.8   12.0 / 6.6   21.9 / 10.7
+//      16464    6.6 / 2.9    9.3 / 6.2   12.6 / 10.5  22.4 / 20.6
+//      29478    8.3 / 2.9   11.3 / 8.0   15.2 / 15.4  28.2 / 33.0
+//      48000   10.7 / 4.3   14.0 / 10.7  19.9 / 22.8  36.0 / 50.2
+//     131712   21.0 / 8.2   25.7 / 23.8  41.8 / 57.5  86.5 / 127.3
+//     196608                35.5 / 34.7
+//     384000   55.2 / 19.6  82.1 / 68.0
 #include <algorithm>
 #include <cstdint>
 
@@ -283,13 +280,13 @@ int rows_tile_elems(int N) {
   }
 }
 
-// Whether this form is taken: at orders 1 and 2 always (order 2: level with the other form around 200,000 elements, where
-// the state leaves L2, and ahead on either side), at orders 3 and 4 up to a number of elements per SM near the crossing
-// (148 SMs, the table above; order 3: 28,950 elements 15.2 / 15.3; order 4: 16,464 22.4 / 20.6, 20,250 25.8 / 24.1).
+// Elements per SM up to which this form is taken (148 SMs; the table above).  Orders 3 and 4 lie near their crossings (order
+// 3: 28,950 elements 15.2 / 15.3; order 4: 16,464 22.4 / 20.6, 29,478 28.2 / 33.0).  At order 2 it is ahead on either
+// side of the line (189,114 elements 34.3 / 33.3, 196,608 35.5 / 34.7), which could lie higher.
 bool rows_faster(int N, int64_t nelems, int num_sms) {
   switch (N) {
-    case 1:
-    case 2: return true;
+    case 1: return true;
+    case 2: return nelems <= 1300 * (int64_t)num_sms;
     case 3: return nelems <= 190 * (int64_t)num_sms;
     case 4: return nelems <= 110 * (int64_t)num_sms;
     default: return false;
