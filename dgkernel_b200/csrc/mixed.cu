@@ -38,11 +38,19 @@ struct MixedCfg {
   static constexpr int TE = kMixedSlotElems;
   static constexpr int NPJ = (NP + 3) & ~3;  // derivative rows padded to whole float4 groups
   // Values per access to a lane's own rows.  With an even Np the lanes' scalars lie 4 (Np = 20) or more to a bank, as
-  // vectors they do not; the traces, whose nodes follow a mask, are read from a copy of uhi at an odd stride (order 5's
-  // copies would take half of the ring).  Order 3, 24 instances of 6^3 to 24^3: 2447 -> 2340
-  // us per two steps (shared-memory conflicts 147 -> 22 thousand clocks an SM; the matrix broadcasts remain).
+  // vectors they do not; the traces, whose nodes follow a mask, are read from a copy of uhi at an odd stride at order 3
+  // (order 5's copies would take half of the ring, order 2's cost what they save).  The products of a vector's rows come
+  // first and the rows they update are loaded after them, which leaves the products more registers.  Order 3, 24
+  // instances of 6^3 to 24^3: 2447 -> 2340 us per two steps with the vectors (shared-memory conflicts 147 -> 22 thousand
+  // clocks an SM; the matrix broadcasts remain).  Rows loaded before and after: order 3, 48^3 x 6 191 -> 186 us a stage;
+  // order 5, 32^3 x 6 350 -> 332; order 2, 64^3 x 6, with no copy 325 -> 319.
   static constexpr int VW = NP % 4 == 0 ? 4 : NP % 2 == 0 ? 2 : 1;
-  static constexpr uint32_t COPY_FLOATS = VW > 1 && N <= 3 ? (uint32_t)TE * (NP + 1) : 0;  // per consumer warp
+  static constexpr uint32_t COPY_FLOATS = VW > 1 && N == 3 ? (uint32_t)TE * (NP + 1) : 0;  // per consumer warp
+  // Tile descriptors loaded ahead: a fill ahead by the producer, before the wait for the slot by a consumer.  A descriptor
+  // comes from HBM on a large mesh, and at low order a CTA takes a tile a microsecond, which that load alone held up: slot
+  // form, us a stage, order 1, 64^3 x 6 298 -> 143; order 2, 48^3 x 6 139 -> 86; order 3 186 -> 172; order 4, 64^3 x 6
+  // 911 -> 893.  Order 5 has fewer slots than warps, and there it costs (48^3 x 6: 1096 -> 1158).
+  static constexpr bool AHEAD = N <= 4;
   static constexpr uint32_t NODE_B = TE * NP * 4;
   static constexpr uint32_t GEO_B = TE * kMixedGeoWords * 4;
   static constexpr uint32_t CONN_B = TE * kMixedConnWords * 4;
@@ -158,9 +166,13 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1) rhs_stage_mixed_kernel(const
     if (lane == 0) {
       int k = 0;
       bool bad = false;
+      MTile next{};
+      if (C::AHEAD && (int)blockIdx.x < A.ntiles) next = A.tiles[blockIdx.x];
       for (;; ++k) {
         const int t = blockIdx.x + k * G;
         if (t >= A.ntiles) break;
+        MTile tl = next;
+        if (C::AHEAD && t + G < A.ntiles) next = A.tiles[t + G];
         const int s = k % NS;
         if (k >= NS && !mbar_wait_bounded(&empty[s], (uint32_t)((k / NS) - 1) & 1u, kSpinLimit)) {
           bad = true;
@@ -172,7 +184,8 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1) rhs_stage_mixed_kernel(const
         }
         if (t + G >= A.ntiles) pdl_trigger();
         *reinterpret_cast<volatile int *>(&sTag[s]) = k;  // fill k/NS of slot s is issued (k-NS was consumed)
-        issue_slot<N>(A, A.tiles[t], ring + (size_t)s * C::SLOT_B, &full[s]);
+        if (!C::AHEAD) tl = A.tiles[t];
+        issue_slot<N>(A, tl, ring + (size_t)s * C::SLOT_B, &full[s]);
       }
       if (bad) {
         atomicExch(A.status, kStatusTimeoutCode);
@@ -195,6 +208,8 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1) rhs_stage_mixed_kernel(const
   for (int k = warp;; k += CW) {
     const int t = blockIdx.x + k * G;
     if (t >= A.ntiles) break;
+    MTile tl;
+    if (C::AHEAD) tl = A.tiles[t];
     const int s = k % NS;
     // Warps own fixed tiles but share the ring, so a warp can reach tile k while the slot still waits for an
     // earlier occupant; its parity wait is unambiguous only once the fill before k's has completed, which the
@@ -214,7 +229,7 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1) rhs_stage_mixed_kernel(const
       }
       break;
     }
-    const MTile tl = A.tiles[t];
+    if (!C::AHEAD) tl = A.tiles[t];
     const int ne = tl.nelem;
     const bool valid = lane < ne;
     const int e = valid ? lane : 0;  // idle lanes mirror element 0 and store nothing
@@ -274,9 +289,7 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1) rhs_stage_mixed_kernel(const
 #pragma unroll 1
     for (int i0 = 0; i0 < NP; i0 += VW) {
       const int o = e * NP + i0;
-      float re[VW], h[VW];
-      ld_vec<VW>(sRe + o, re);
-      ld_vec<VW>(hi + i0, h);
+      float dd[VW], re[VW], h[VW];
 #pragma unroll
       for (int q = 0; q < VW; ++q) {
         const float4 *Dq = reinterpret_cast<const float4 *>(sDm + (i0 + q) * 3 * NPJ);
@@ -294,8 +307,13 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1) rhs_stage_mixed_kernel(const
         const float ur = (ar.x + ar.y) + (br.x + br.y);
         const float us = (as.x + as.y) + (bs.x + bs.y);
         const float ut = (at.x + at.y) + (bt.x + bt.y);
-        const float dd = fmaf(cr, ur, fmaf(cs, us, fmaf(ct, ut, L0)));
-        const float vol = cons ? -dd : -h[q] * dd;
+        dd[q] = fmaf(cr, ur, fmaf(cs, us, fmaf(ct, ut, L0)));
+      }
+      ld_vec<VW>(sRe + o, re);
+      ld_vec<VW>(hi + i0, h);
+#pragma unroll
+      for (int q = 0; q < VW; ++q) {
+        const float vol = cons ? -dd[q] : -h[q] * dd[q];
         re[q] = fmaf(a, re[q], dt * vol);
       }
       if (valid) st_vec<VW>(sRe + o, re);
@@ -341,10 +359,7 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1) rhs_stage_mixed_kernel(const
 #pragma unroll 1
     for (int i0 = 0; i0 < NP; i0 += VW) {
       const int o = e * NP + i0;
-      float re[VW], h[VW], l[VW];
-      ld_vec<VW>(sRe + o, re);
-      ld_vec<VW>(hi + i0, h);
-      ld_vec<VW>(lo + i0, l);
+      float lift[VW], re[VW], h[VW], l[VW];
 #pragma unroll
       for (int q = 0; q < VW; ++q) {
         const float4 *Lq = reinterpret_cast<const float4 *>(sL + (i0 + q) * NF);
@@ -360,8 +375,14 @@ __global__ void __launch_bounds__(32 * (CW + 1), 1) rhs_stage_mixed_kernel(const
             l1 = __ffma2_rn(make_float2(m.z, m.w), make_float2(fl[4 * g + 2], fl[4 * g + 3]), l1);
           }
         }
-        const float lift = ((l0.x + l0.y) + (l1.x + l1.y)) + ((l2.x + l2.y) + (l3.x + l3.y));
-        const float rn = fmaf(dt, lift, re[q]);
+        lift[q] = ((l0.x + l0.y) + (l1.x + l1.y)) + ((l2.x + l2.y) + (l3.x + l3.y));
+      }
+      ld_vec<VW>(sRe + o, re);
+      ld_vec<VW>(hi + i0, h);
+      ld_vec<VW>(lo + i0, l);
+#pragma unroll
+      for (int q = 0; q < VW; ++q) {
+        const float rn = fmaf(dt, lift[q], re[q]);
         const double un = ((double)h[q] + (double)l[q]) + b * (double)rn;
         h[q] = __double2float_rn(un);
         l[q] = __double2float_rn(un - (double)h[q]);

@@ -13,15 +13,19 @@
 // tile's state is stored; its operands (field minus linear part, face terms) are.  Bound by its instruction count (about
 // 330 per node at order 3 against mixed.cu's 150) once every SM is busy.  The lines of rows_faster follow from stages in
 // a captured graph, us, mixed.cu / here:
-//   elements    order 1      order 2      order 3      order 4
-//        384    4.0 / 2.1    6.4 / 2.7    9.7 / 3.1   19.1 / 5.9
-//       6000    5.5 / 2.3    8.3 / 3.8   12.0 / 6.6   21.9 / 10.7
-//      16464    6.6 / 2.9    9.3 / 6.2   12.6 / 10.5  22.4 / 20.6
-//      29478    8.3 / 2.9   11.3 / 8.0   15.2 / 15.4  28.2 / 33.0
-//      48000   10.7 / 4.3   14.0 / 10.7  19.9 / 22.8  36.0 / 50.2
-//     131712   21.0 / 8.2   25.7 / 23.8  41.8 / 57.5  86.5 / 127.3
-//     196608                35.5 / 34.7
-//     384000   55.2 / 19.6  82.1 / 68.0
+//   elements    order 1       order 2        order 3      order 4
+//        384    3.8 / 1.9     6.2 / 2.7      9.5 / 3.3   18.9 / 6.0
+//       6000    5.4 / 2.3     8.1 / 3.9     11.9 / 6.8   21.7 / 10.7
+//      16464    6.0 / 2.9     8.7 / 6.2     12.1 / 10.5  22.3 / 20.6
+//      20250                  8.9 / 6.6     12.8 / 11.5  25.2 / 24.2
+//      24576                  9.6 / 7.0     14.2 / 13.6  27.1 / 28.3
+//      29478    7.2 / 2.9     9.9 / 8.1     14.4 / 15.4  27.6 / 33.3
+//      48000    8.7 / 4.2    11.9 / 10.7
+//      82944                 16.2 / 15.8
+//      93750                 17.2 / 17.7
+//     131712   15.4 / 8.0    22.0 / 24.1    39.1 / 58.0  87.0 / 127.6
+//     384000   37.7 / 19.5   52.5 / 68.8
+//     663552   62.7 / 32.1   87.6 / 119.6
 #include <algorithm>
 #include <cstdint>
 
@@ -280,14 +284,13 @@ int rows_tile_elems(int N) {
   }
 }
 
-// Elements per SM up to which this form is taken (148 SMs; the table above).  Orders 3 and 4 lie near their crossings (order
-// 3: 28,950 elements 15.2 / 15.3; order 4: 16,464 22.4 / 20.6, 29,478 28.2 / 33.0).  At order 2 it is ahead on either
-// side of the line (189,114 elements 34.3 / 33.3, 196,608 35.5 / 34.7), which could lie higher.
+// Elements per SM up to which this form is taken (148 SMs; the table above): order 1 always, orders 2 and 3 up to their
+// crossings, order 4 somewhat below it.
 bool rows_faster(int N, int64_t nelems, int num_sms) {
   switch (N) {
     case 1: return true;
-    case 2: return nelems <= 1300 * (int64_t)num_sms;
-    case 3: return nelems <= 190 * (int64_t)num_sms;
+    case 2: return nelems <= 590 * (int64_t)num_sms;
+    case 3: return nelems <= 175 * (int64_t)num_sms;
     case 4: return nelems <= 110 * (int64_t)num_sms;
     default: return false;
   }
