@@ -9,8 +9,8 @@ Timing runs stage 0 of the LSERK4 scheme with dt = 0 from a step boundary: the r
 state is rewritten unchanged, so tuning leaves the solution where it was (the next real stage 0 ignores the
 residual).  Every candidate computes the same arithmetic per element, so the choice changes speed only.
 
-Candidates of the mixed stage: the operator's own choice (at orders 1 and 2, and on small problems of orders 3 and 4,
-the form with a matrix row per thread, else 11 consumer warps and a full ring), its slot form with 4, 8 or 11 consumer warps per CTA and a ring of as many
+Candidates of the mixed stage: the operator's own choice (at order 1 and on small problems the form with a matrix row
+per thread, else 11 consumer warps and a full ring), its slot form with 4, 8 or 11 consumer warps per CTA and a ring of as many
 slots as shared memory holds, or 6; and, at orders 1..4, its tensor-core form with 2 or 4 threads per element
 (8 or 16 consumer warps).  The tensor-core form rounds differently (both within the mixed stage's error bound);
 the others give the same bits.  The plain stages have one launch shape per order and are not tuned.
